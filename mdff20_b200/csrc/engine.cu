@@ -198,11 +198,14 @@ Engine::~Engine() {
                     d_nhc};
     for (auto &x : dd) cudaFree(x);
     int *di[] = {d_typ, d_polar, d_nb, d_nbn, d_co, d_con, d_cell_of, d_cell_cnt, d_cell_start, d_cell_cur,
-                 d_cell_ions, d_rebuild, d_tile_row, d_tile_k};
+                 d_cell_ions, d_rebuild};
     for (auto &x : di) cudaFree(x);
     cudaFree(d_pair);
     cudaFree(d_damp);
-    cudaFree(d_seg);
+    cudaFree(d_tab64);
+    cudaFree(d_rowxy);
+    cudaFree(d_w64);
+    cudaFree(d_btick);
     cudaFree(d_row);
     cudaFree(d_rho_part);
     cudaFree(d_rho);
@@ -471,7 +474,6 @@ void Engine::setup_kspace() {
     std::vector<double3> kv(nk);
     std::vector<double> Ak(nk), kcoe(nk);
     std::vector<KRow> rows;
-    std::vector<KSeg> segs;
     double alpha2 = p.alphaES * p.alphaES;
     const Cell &c = cell;
     int ik = 0;
@@ -488,16 +490,6 @@ void Engine::setup_kspace() {
             R.pad0 = R.pad1 = R.pad2 = 0;
             if (R.cnt <= 0) continue;
             rows.push_back(R);
-            for (int z0 = nzmin; z0 <= K2; z0 += KSEG) {
-                KSeg S;
-                S.nx = nx;
-                S.ny = ny;
-                S.z0 = z0;
-                S.cnt = std::min(KSEG, K2 - z0 + 1);
-                S.koff = ik + (z0 - nzmin);
-                S.pad0 = S.pad1 = S.pad2 = 0;
-                segs.push_back(S);
-            }
             for (int nz = nzmin; nz < K2 + 1; nz++) {
                 double kx = TPI_D * ((double)nx * c.B[0][0] + (double)ny * c.B[0][1] + (double)nz * c.B[0][2]);
                 double ky = TPI_D * ((double)nx * c.B[1][0] + (double)ny * c.B[1][1] + (double)nz * c.B[1][2]);
@@ -511,59 +503,19 @@ void Engine::setup_kspace() {
         }
     }
     nrow = (int)rows.size();
-    nseg = (int)segs.size();
-    // ion-pass k slices: whole rows, at most 512 k per slice (8 KB of shared memory);
-    // the slices are the second grid dimension of the ion pass
-    const int TILEK = 512;
-    h_tile_row.clear();
-    h_tile_k.clear();
-    int r = 0;
-    tile_kmax = 0;
-    while (r < nrow) {
-        int k0 = rows[r].koff, cnt = 0, r1 = r;
-        while (r1 < nrow && cnt + rows[r1].cnt <= TILEK) {
-            cnt += rows[r1].cnt;
-            r1++;
-        }
-        if (r1 == r) throw Error(MDFFGPU_ERR_ARG, "k row longer than a tile");
-        h_tile_row.push_back(r);
-        h_tile_k.push_back(k0);
-        tile_kmax = std::max(tile_kmax, cnt);
-        r = r1;
-    }
-    h_tile_row.push_back(nrow);
-    h_tile_k.push_back(nk);
-    ntile = (int)h_tile_row.size() - 1;
     d_kvec = dalloc<double3>(nk);
     d_Ak = dalloc<double>(nk);
     d_kcoe = dalloc<double>(nk);
     d_row = dalloc<KRow>(nrow);
-    d_seg = dalloc<KSeg>(nseg);
-    d_tile_row = dalloc<int>(ntile + 1);
-    d_tile_k = dalloc<int>(ntile + 1);
     MDFF_CK(cudaMemcpy(d_kvec, kv.data(), sizeof(double3) * nk, cudaMemcpyHostToDevice));
     MDFF_CK(cudaMemcpy(d_Ak, Ak.data(), sizeof(double) * nk, cudaMemcpyHostToDevice));
     MDFF_CK(cudaMemcpy(d_kcoe, kcoe.data(), sizeof(double) * nk, cudaMemcpyHostToDevice));
     MDFF_CK(cudaMemcpy(d_row, rows.data(), sizeof(KRow) * nrow, cudaMemcpyHostToDevice));
-    MDFF_CK(cudaMemcpy(d_seg, segs.data(), sizeof(KSeg) * nseg, cudaMemcpyHostToDevice));
-    MDFF_CK(cudaMemcpy(d_tile_row, h_tile_row.data(), sizeof(int) * (ntile + 1), cudaMemcpyHostToDevice));
-    MDFF_CK(cudaMemcpy(d_tile_k, h_tile_k.data(), sizeof(int) * (ntile + 1), cudaMemcpyHostToDevice));
-    // rho pass grid: segment blocks x ion chunks filling `waves` full waves of
-    // RHO_MIN_BLOCKS resident blocks per SM (MDFFGPU_RHO_WAVES overrides, default 1)
-    int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-    int segblocks = ceil_div(nseg, 128);
-    double waves = 1.0;
-    if (const char *w = getenv("MDFFGPU_RHO_WAVES")) waves = std::max(0.1, atof(w));
-    int chunks = std::max(1, (int)(waves * RHO_MIN_BLOCKS * nsm) / segblocks);
-    chunks = std::min(chunks, std::max(1, ceil_div(n, 32)));
-    rho_chunk = ceil_div(n, chunks);
-    rho_chunks = ceil_div(n, rho_chunk);
-    d_rho_part = dalloc<double2>((size_t)rho_chunks * nk);
     d_rho = dalloc<double2>(nk);
     d_rho_acc = dalloc<double2>(nk);
     d_rho_it = dalloc<double2>(nk);
-    d_ion_part = dalloc<double>((size_t)ntile * n * 12);
+    setup_kspace64(*this, rows);
     setup_kspace32(*this, rows);
 }
 
@@ -794,6 +746,7 @@ void Engine::field_of(const double *d_qv, const double3 *d_muv, bool lq, bool ld
     o.self2 = self2_of(p.alphaES);
     o.self_mu = d_muv;
     o.rho_raw = rho_raw;
+    o.energy = false;
     launch_rec(*this, d_qv, d_muv, lq, ld, o);
 }
 
@@ -804,9 +757,8 @@ void Engine::field_pol(const double3 *d_p, double3 *d_out, double2 *rho_raw, boo
         if (use32 && real32) launch_pol_field32(*this, d_p, d_tmp3);
         else launch_dir_field_cached(*this, d_p, d_tmp3);
     };
-    // beside the k-space passes when launch_combine32 reads d_tmp3 (mixed k space)
-    if (use32 && rec32) on_side(stream == body_stream ? SIDE_BODY : SIDE_FIELD, real);
-    else real();
+    // beside the k-space passes (the ion pass or its combine joins it before reading d_tmp3)
+    on_side(stream == body_stream ? SIDE_BODY : SIDE_FIELD, real);
     RecOut o;
     o.ef = d_out;
     o.ef_dir = d_tmp3;
@@ -1049,39 +1001,41 @@ void Engine::pim_cg(bool fused) {
     if (ord < 0 || ord > 5) throw Error(MDFFGPU_ERR_ARG, "extrapolate_order must be 0..5");
     int e = (istep >= ord + 1) ? ord : (!istep ? 0 : istep - 1);
     int es = (e != ord) ? e + 1 : e;
-    if (fused) {
+    // one evaluation for the residual: in the fused CG, and in the plain one without static
+    // dipoles (with them it keeps E_stat and T mu0 apart: a dipole acts on an ion only where
+    // that ion's own dipole is non-zero, src/ewald.c:737)
+    if (fused || !ldip) {
         MDFF_LAUNCH(*this, k_aspc_predict, nb, 256, 0, n, aspc_coef(e, cg_poly), es, d_hist, d_mu_ind);
         MDFF_LAUNCH(*this, k_add3, nb, 256, 0, n, d_mu_static, d_mu_ind, d_mu_tot);
         // the residual reads the field at the polarisable ions only (FP64 real space
         // evaluates every ion; the k-space ion pass and FP32 real space only those)
         bool sub = subset32 && npol > 0;
-        if (use32 && real32) {
-            // on the branch of the in-cutoff lists, beside the k-space passes below (the
-            // FP32 k-space combine joins it)
-            auto dir = [&] {
+        // on the branch of the in-cutoff lists or cached pair factors, beside the k-space
+        // passes below (the ion pass or its combine joins it)
+        on_side(SIDE_PREP, [&] {
+            if (use32 && real32)
                 launch_dir32(*this, d_q, d_mu_tot, p.alphaES, lqch != 0, true, ldmp != 0, false, true, d_tmp3,
                              nullptr, sub ? d_pidx : nullptr, npol);
-            };
-            if (rec32) on_side(SIDE_PREP, dir);
-            else dir();
-        } else {
-            launch_dir(*this, d_q, d_mu_tot, p.alphaES, lqch != 0, true, ldmp != 0, false, true, false, false,
-                       d_tmp3, nullptr, nullptr);
-        }
+            else
+                launch_dir(*this, d_q, d_mu_tot, p.alphaES, lqch != 0, true, ldmp != 0, false, true, false, false,
+                           d_tmp3, nullptr, nullptr);
+        });
         RecOut o;
         o.ef = d_ef_ind;
         o.ef_dir = d_tmp3;
         o.self2 = self2_of(p.alphaES);
         o.self_mu = d_mu_tot;
-        o.rho_raw = d_rho_acc;
+        o.rho_raw = fused ? d_rho_acc : nullptr;
+        o.energy = false;
         if (sub) {
             o.out_idx = d_pidx;
             o.out_cnt = npol;
         }
         launch_rec(*this, d_q, d_mu_tot, lqch != 0, true, o);
-        join_side(SIDE_PREP);   // (joined by the combine already; the loop below reads the records)
+        join_side(SIDE_PREP);   // (joined by the ion pass already; the loop below reads the records)
         MDFF_LAUNCH(*this, k_cg_residual, nb, 256, 0, n, d_polar, d_invpol, d_muzero, d_ef_ind, d_mu_ind, d_cg_r);
     } else {
+        join_side(SIDE_PREP);
         field_of(d_q, d_mu_static, lqch != 0, ldip != 0, ldmp != 0, d_ef_stat);
         MDFF_LAUNCH(*this, k_aspc_predict, nb, 256, 0, n, aspc_coef(e, cg_poly), es, d_hist, d_mu_ind);
         field_of(d_qzero, d_mu_ind, false, true, false, d_ef_ind);
@@ -1102,14 +1056,9 @@ void Engine::pim_cg(bool fused) {
     test.status = d_status;
     test.guard = d_ticket + 4;
     auto iteration = [&](CgTest t) {
-        if (fused && subset32 && npol > 0) {
-            // T p over the polarisable ions; Ap and p.Ap in the FP32 k-space combine, or
-            // by k_cg_ap after the FP64 one
-            bool ap_in_combine = use32 && rec32;
-            field_pol(d_cg_p, d_ef_ind, d_rho_it, ap_in_combine);
-            if (!ap_in_combine)
-                MDFF_LAUNCH(*this, k_cg_ap, nb, 256, 0, n, d_polar, d_invpol, d_cg_p, d_ef_ind, d_cg_ap, d_part,
-                            part_stride, d_scal, d_ticket);
+        if (subset32 && npol > 0) {
+            // T p over the polarisable ions; Ap and p.Ap formed by the ion pass
+            field_pol(d_cg_p, d_ef_ind, fused ? d_rho_it : nullptr, true);
         } else {
             field_of(d_qzero, d_cg_p, false, true, false, d_ef_ind, fused ? d_rho_it : nullptr);
             MDFF_LAUNCH(*this, k_cg_ap, nb, 256, 0, n, d_polar, d_invpol, d_cg_p, d_ef_ind, d_cg_ap, d_part,
@@ -1237,12 +1186,13 @@ void Engine::pim_ko() {
 
 // get_dipoles (src/coulombic.c:67-130): mu = static + induced
 void Engine::get_dipoles() {
+    // the CG's first field pass continues the branch of the pair preparation with its
+    // real-space part and the k space beside it joins it; the other solvers join it here
+    const bool cont =
+        lpol && (pim_solver == MDFFGPU_PIM_CG || pim_solver == MDFFGPU_PIM_CG_FUSED);
     // mixed precision: in-cutoff list and dipole-field records of these positions (the
-    // real-space kernels of this force evaluation read them)
+    // real-space kernels of this force evaluation read them), issued beside the k-space tables
     if (use32 && real32) {
-        // issued beside the k-space tables; the fused CG's first field pass continues that
-        // branch with its real-space part and its k-space combine joins it
-        const bool cont = lpol && pim_solver == MDFFGPU_PIM_CG_FUSED && rec32;
         if (!prep_issued) launch_pair_prep32(*this);
         else if (!cont) join_side(SIDE_PREP);
         prep_issued = false;
@@ -1253,7 +1203,10 @@ void Engine::get_dipoles() {
             bool &flag;
             ~CoefScope() { flag = false; }
         } scope{coef_ready};
-        if (!(use32 && real32)) launch_dir_prep(*this, p.alphaES);
+        if (!(use32 && real32)) {
+            on_side(SIDE_PREP, [&] { launch_dir_prep(*this, p.alphaES); });
+            if (!cont) join_side(SIDE_PREP);
+        }
         coef_ready = true;
         if (pim_solver == MDFFGPU_PIM_CG || pim_solver == MDFFGPU_PIM_CG_FUSED)
             pim_cg(pim_solver == MDFFGPU_PIM_CG_FUSED);
@@ -1301,7 +1254,7 @@ void Engine::engforce(bool check_finite) {
         get_dipoles();
         bool ld = (ldip || lpol);
         // direct space: forces, energy, virial (do_forces, do_stress; src/field.c:381-383);
-        // beside the k-space force pass in mixed precision (launch_combine32 joins it)
+        // beside the k-space force pass (the ion pass or its combine joins it)
         auto direct = [&] {
             if (use32 && real32)
                 launch_dir32(*this, d_q, d_mu_tot, p.alphaES, lqch != 0, ld, ldmp != 0, true, false, nullptr, d_tmp3);
@@ -1310,9 +1263,7 @@ void Engine::engforce(bool check_finite) {
                            nullptr, nullptr, d_tmp3);
             reduce(S_DIR_U, 7, ceil_div(n, 8));
         };
-        if (use32 && rec32) on_side(SIDE_DIR, direct);
-        else direct();
-        if (!(use32 && rec32)) join_side(SIDE_SR);
+        on_side(SIDE_DIR, direct);
         RecOut o;
         o.f = d_f;
         o.f_dir = d_tmp3;

@@ -23,10 +23,8 @@ struct PairDamp {
     double b1, c1, b2, c2;
 };
 
-// one k-space row segment: up to KSEG consecutive nz values at fixed (nx, ny)
-constexpr int KSEG = 16;
-constexpr int RHO_MIN_BLOCKS = 4;   // resident k_rho blocks per SM (caps registers at 128)
 constexpr int RHOR_K = 32;          // k per k_rho_reduce block
+// one k-space row segment: consecutive nz values at fixed (nx, ny)
 struct KSeg {
     int nx, ny, z0, cnt;
     int koff, pad0, pad1, pad2;
@@ -150,6 +148,9 @@ struct RecOut {
     CgAp cg;                          // mixed precision, field only: the CG product at the output ions
 };
 void launch_rec(Engine &e, const double *q, const double3 *mu, bool lq, bool ld, const RecOut &o);
+// kspace64.cu: the FP64 passes
+void setup_kspace64(Engine &e, const std::vector<KRow> &rows);
+void launch_rec64(Engine &e, const double *q, const double3 *mu, bool lq, bool ld, const RecOut &o);
 // fit.cu: the status bits of a force-matching evaluation as an Error (none: returns)
 void fit_status(unsigned status);
 constexpr int FIT_NRES = 1 + MDFFGPU_FIT_NPARAM + 1;   // loss, gradient, status bits per evaluation
@@ -277,15 +278,10 @@ struct Engine {
     bool list_ready = false;
 
     // ---- k space
-    int nk = 0, nseg = 0, nrow = 0, kmax[3] = {0, 0, 0};
+    int nk = 0, nrow = 0, kmax[3] = {0, 0, 0};
     double *d_Ak = nullptr, *d_kcoe = nullptr;
     double3 *d_kvec = nullptr;
-    KSeg *d_seg = nullptr;
     KRow *d_row = nullptr;
-    std::vector<int> h_tile_row;   // first row of each ion-pass tile (+ end)
-    std::vector<int> h_tile_k;     // first k of each tile (+ end)
-    int *d_tile_row = nullptr, *d_tile_k = nullptr;
-    int ntile = 0, tile_kmax = 0;
     double2 *d_rho_part = nullptr, *d_rho = nullptr;   // partial per ion chunk, total (Ak-scaled)
     double2 *d_rho_acc = nullptr, *d_rho_it = nullptr; // rho(k) of (q, mu) along the fused CG; of its p
     // mixed precision k space (kspace32.cu)
@@ -314,8 +310,13 @@ struct Engine {
     double *d_ion_part32 = nullptr;                     // [slices][n][6]
     int *d_pidx = nullptr;                              // polarisable ions, ascending
     bool rho_acc_ready = false;                         // d_rho_acc holds rho(k) of (q, mu_tot)
-    double *d_ion_part = nullptr;                       // ion-pass partial sums [ntile][n][12]
-    int rho_chunks = 0, rho_chunk = 0;
+    // FP64 k space (kspace64.cu): phase table rows [n][tab64_w], ion-pass weights, (nx, ny) of
+    // the rows, slice partials [slice][n][9] and the arrival counter per block of ions
+    double2 *d_tab64 = nullptr, *d_rowxy = nullptr;
+    double *d_w64 = nullptr, *d_ion_part = nullptr;
+    unsigned *d_btick = nullptr;
+    int tab64_w = 0, rho64_chunks_max = 0, ion64_slices_max = 0;
+    bool phase64_ready = false;                         // d_tab64 holds the phases of the positions in d_s
 
     // ---- reductions
     double *d_part = nullptr;    // [NSLOT][part_stride]

@@ -511,8 +511,7 @@ void Engine::solve_pim(const double3 *d_b, double3 *d_x, double rtol, int maxit)
                 d_ticket + 1);
     MDFF_CK(cudaMemcpyAsync(d_cg_p, d_mu_save, sizeof(double3) * n, cudaMemcpyDeviceToDevice, stream));
     // A p: the search direction vanishes off the polarisable ions, so the field passes
-    // run over those ions only; A p and p.A p in the FP32 k-space combine (or k_cg_ap),
-    // then x, r, z and r.z, r.r in one launch, as the induced-dipole CG does
+    // run over those ions only; A p and p.A p in the ion pass (or k_cg_ap), then x, r, z and r.z, r.r in one launch, as the induced-dipole CG does
     CgTest test{};
     test.mode = 2;
     test.rr0 = d_fscal + F_ADJ_RR0;
@@ -522,10 +521,10 @@ void Engine::solve_pim(const double3 *d_b, double3 *d_x, double rtol, int maxit)
     test.status = d_status;
     test.guard = d_ticket + 4;
     auto iteration = [&](CgTest t) {
-        const bool sub = subset32 && npol > 0, ap_in_combine = sub && use32 && rec32;
-        if (sub) field_pol(d_cg_p, d_ef_ind, nullptr, ap_in_combine);
+        const bool sub = subset32 && npol > 0;
+        if (sub) field_pol(d_cg_p, d_ef_ind, nullptr, true);
         else field_of(d_qzero, d_cg_p, false, true, false, d_ef_ind);
-        if (!ap_in_combine)
+        if (!sub)
             MDFF_LAUNCH(*this, k_cg_ap, nb, 256, 0, n, d_polar, d_invpol, d_cg_p, d_ef_ind, d_cg_ap, d_part,
                         part_stride, d_scal, d_ticket);
         MDFF_LAUNCH(*this, k_cg_step, nb, 256, 0, n, 0, d_polar, d_pol, d_scal, d_cg_p, d_cg_ap, d_x, d_cg_r,
@@ -631,8 +630,6 @@ void Engine::fit_issue(const double3 *d_ft, double scale, int tSi, int tO, const
     engforce();
     MDFF_LAUNCH(*this, k_fm_seed, nb, 256, 0, n, d_f, d_ft, scale, d_w, d_fpart, part_stride);
     fit_reduce(F_LOSS, 1, nb);
-    // fixed geometry for the adjoint: fractional coordinates and lists as in engforce
-    launch_kardir(*this, d_r, d_s);
     AdjArgs a;
     a.n = n;
     a.nt = nt;

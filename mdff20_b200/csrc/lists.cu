@@ -23,6 +23,7 @@ __global__ void k_kardir(int n, Cell c, const double4 *__restrict__ r, double4 *
 
 void launch_kardir(Engine &e, const double4 *r, double4 *s) {
     MDFF_LAUNCH(e, k_kardir, ceil_div(e.n, 256), 256, 0, e.n, e.cell, r, s);
+    e.phase64_ready = false;   // the positions may have moved
 }
 
 // ---------------------------------------------------------------- check_verletlist
