@@ -224,7 +224,7 @@ int mdffgpu_md_steps_host(mdffgpu_ctx *ctx, int first, int nsteps, const double 
  * cut_nb/cut_co the two list radii (rc + skin); the FULL lists go to the caller's
  * device buffers d_nb[n][cap_nb], d_nbn[n], d_co[n][cap_co], d_con[n] (each ion's
  * neighbours, both directions of every pair).  Scratch is a static device array of
- * about 5 MB, shared by every call on a device and holding the last call's data:
+ * about 4 MB, shared by every call on a device and holding the last call's data:
  * limits n <= 65536 (more returns MDFFGPU_ERR_ARG), a cell grid of at most 32768 cells
  * (a finer grid is coarsened to fit), at most 4096 ions per cell (so n <= 4096 when the
  * cell is too small for a cell grid; more returns MDFFGPU_ERR_CELL).  Calls that overlap on the GPU (other streams, other threads) race

@@ -277,37 +277,10 @@ int mdffgpu_check_verletlist(mdffgpu_ctx *ctx, int *rebuilt) {
     });
 }
 
-// the reference's half list from the full lists: keep (i, j) when the parity rule
-// of src/verlet.c:82-83 holds, ascending j
+// the reference's half list from the full lists, formed on the device (lists.cu)
 int mdffgpu_get_verletlist(mdffgpu_ctx *ctx, int which, int *point, int *list, int cap, int *count) {
     if (!point || (which != 0 && which != 1)) return MDFFGPU_ERR_ARG;
-    return guarded(ctx, [&](Engine &e) {
-        if (!e.list_ready) throw Error(MDFFGPU_ERR_STATE, "no Verlet list built");
-        int c = which ? e.cap_co : e.cap_nb;
-        std::vector<int> L((size_t)e.n * c), m(e.n);
-        download(e, L.data(), which ? e.d_co : e.d_nb, sizeof(int) * L.size());
-        download(e, m.data(), which ? e.d_con : e.d_nbn, sizeof(int) * e.n);
-        MDFF_CK(cudaStreamSynchronize(e.stream));
-        int tot = 0;
-        std::vector<int> row;
-        for (int i = 0; i < e.n; i++) {
-            point[i] = tot;
-            row.clear();
-            int mi = m[i] < c ? m[i] : c;
-            for (int k = 0; k < mi; k++) {
-                int j = L[(size_t)i * c + k];
-                if (((i > j) && ((i + j) % 2 == 0)) || ((i < j) && ((i + j) % 2 != 0))) row.push_back(j);
-            }
-            std::sort(row.begin(), row.end());
-            for (int j : row) {
-                if (list && tot < cap) list[tot] = j;
-                tot++;
-            }
-        }
-        point[e.n] = tot;
-        if (count) *count = tot;
-        if (list && tot > cap) throw Error(MDFFGPU_ERR_ARG, "list buffer too small");
-    });
+    return guarded(ctx, [&](Engine &e) { e.half_list(which, point, list, cap, count); });
 }
 
 int mdffgpu_engforce(mdffgpu_ctx *ctx) {

@@ -66,8 +66,8 @@ struct NhcArgs {
 void launch_nhc_chain(Engine &e, const NhcArgs &a, double *nhc, const double *scal, DevScalars *out);
 __global__ void k_set_ekin(const double *scal, DevScalars *out);
 __global__ void k_check_finite(int n, const double4 *r, const double3 *f, unsigned *status);
-__global__ void k_sort_cells(int ncell, int cell_cap, const int *start, const int *cnt, int *ions,
-                             const int *rebuild);
+__global__ void k_sort_cells(int ncell, int cell_cap, const int *start, const int *cnt, int *ions, const double4 *s,
+                             float4 *pk, const int *rebuild);
 
 template <typename T>
 static void dfree(T *&p) {
@@ -198,10 +198,11 @@ Engine::~Engine() {
                     d_nhc};
     for (auto &x : dd) cudaFree(x);
     int *di[] = {d_typ, d_polar, d_nb, d_nbn, d_co, d_con, d_cell_of, d_cell_cnt, d_cell_start, d_cell_cur,
-                 d_cell_ions, d_rebuild};
+                 d_cell_ions, d_rebuild, d_csr_point, d_csr_list};
     for (auto &x : di) cudaFree(x);
     cudaFree(d_pair);
     cudaFree(d_damp);
+    cudaFree(d_cell_pk);
     cudaFree(d_tab64);
     cudaFree(d_rowxy);
     cudaFree(d_w64);
@@ -544,6 +545,7 @@ void Engine::setup_cells() {
     d_cell_start = dalloc<int>(ncell);
     d_cell_cur = dalloc<int>(ncell);
     d_cell_ions = dalloc<int>(n);
+    d_cell_pk = dalloc<float4>(n);
 }
 
 void Engine::alloc_lists(int cnb, int cco) {

@@ -274,8 +274,11 @@ struct Engine {
     int nc[3] = {1, 1, 1}, ncell = 1, cell_cap = 4096;
     int *d_cell_of = nullptr, *d_cell_cnt = nullptr, *d_cell_start = nullptr, *d_cell_cur = nullptr,
         *d_cell_ions = nullptr;
+    float4 *d_cell_pk = nullptr; // ions in cell order: wrapped fractional coordinates (FP32) and index
     int *d_rebuild = nullptr;    // 1 when the lists must be rebuilt this step
     bool list_ready = false;
+    int *d_csr_point = nullptr, *d_csr_list = nullptr;   // half list in CSR form (half_list)
+    size_t csr_room = 0;                                 // entries d_csr_list holds
 
     // ---- k space
     int nk = 0, nrow = 0, kmax[3] = {0, 0, 0};
@@ -452,6 +455,7 @@ struct Engine {
     void gen_verletlist();
     int check_verletlist(bool reset_status = true);
     void ensure_lists();
+    void half_list(int which, int *point, int *list, int cap, int *count);
     void engforce(bool check_finite = true);   // check_finite: ST_NONFINITE from r and f
     void sr_forces(bool lj, double *u, double *pvir, double *tau);
     void sr_finish(bool lj);   // reduce the short-range slot, u / virial / stress into d_out

@@ -15,29 +15,29 @@
 namespace mdffgpu {
 
 __global__ void k_kardir(int n, Cell c, const double4 *r, double4 *s);
-__global__ void k_bin(int n, int3 nc, const double4 *s, int *cell_of, int *cnt, const int *rebuild);
+__global__ void k_bin(int n, int3 nc, const double4 *s, int *cell_of, int *cnt, double4 *svl, const int *rebuild);
 __global__ void k_scan_cells(int ncell, const int *cnt, int *start, int *cur, int cell_cap, unsigned *status,
                              const int *rebuild);
 __global__ void k_fill_cells(int n, const int *cell_of, const int *start, int *cur, int *ions, const int *rebuild);
-__global__ void k_sort_cells(int ncell, int cell_cap, const int *start, const int *cnt, int *ions,
-                             const int *rebuild);
-__global__ void k_build(int n, Cell c, int3 nc, const double4 *s, const int *cell_of, const int *start,
-                        const int *cnt, const int *ions, double rsq_nb, double rsq_co, int cap_nb, int *nbl,
-                        int *nbn, int cap_co, int *col, int *con, double4 *svl, unsigned *status,
-                        const int *rebuild);
+__global__ void k_sort_cells(int ncell, int cell_cap, const int *start, const int *cnt, int *ions, const double4 *s,
+                             float4 *pk, const int *rebuild);
+void run_build(cudaStream_t st, bool pdl, int n, const Cell &c, const int nc[3], const double4 *s, const int *cell_of,
+               const int *start, const int *cnt, const float4 *pk, double cut_nb, double cut_co, int cap_nb, int *nbl,
+               int *nbn, int cap_co, int *col, int *con, unsigned *status, const int *rebuild);
 
 // limits of the static scratch
 constexpr int NA_MAX_IONS = 65536;
 constexpr int NA_MAX_CELLS = 32768;
 constexpr int NA_CELL_CAP = 4096;   // members of one cell (bitonic sort in shared memory)
 
-// scratch layout, in 8-byte words: s[N] double4, svl[N] double4, then ints
-constexpr size_t NA_WORDS = (size_t)NA_MAX_IONS * 4 * 2 +                       // s, svl
+// scratch layout, in 8-byte words: s[N] double4, pk[N] float4, then ints
+constexpr size_t NA_WORDS = (size_t)NA_MAX_IONS * (4 + 2) +                     // s, pk
                             ((size_t)NA_MAX_IONS * 2 + (size_t)NA_MAX_CELLS * 3 + 64) / 2;  // ints
 static __device__ __align__(256) double g_noalloc_scratch[NA_WORDS];
 
 struct NaPtrs {
-    double4 *s, *svl;
+    double4 *s;
+    float4 *pk;
     int *cell_of, *ions, *cnt, *start, *cur, *rebuild;
     unsigned *status;
 };
@@ -61,8 +61,8 @@ static int na_pointers(NaPtrs *p) {
     }
     char *b = (char *)base;
     p->s = (double4 *)b;
-    p->svl = p->s + NA_MAX_IONS;
-    int *ib = (int *)(p->svl + NA_MAX_IONS);
+    p->pk = (float4 *)(p->s + NA_MAX_IONS);
+    int *ib = (int *)(p->pk + NA_MAX_IONS);
     p->cell_of = ib;
     p->ions = ib + NA_MAX_IONS;
     p->cnt = p->ions + NA_MAX_IONS;
@@ -139,15 +139,17 @@ extern "C" int mdffgpu_build_lists_noalloc(const double *d_pos, int n, const dou
     int3 g = make_int3(nc[0], nc[1], nc[2]);
     int nb = (n + 255) / 256;
     k_kardir<<<nb, 256, 0, st>>>(n, c, (const double4 *)d_pos, P.s);
-    k_bin<<<nb, 256, 0, st>>>(n, g, P.s, P.cell_of, P.cnt, P.rebuild);
+    k_bin<<<nb, 256, 0, st>>>(n, g, P.s, P.cell_of, P.cnt, (double4 *)nullptr, P.rebuild);
     k_scan_cells<<<1, 1024, 0, st>>>(ncell, P.cnt, P.start, P.cur, NA_CELL_CAP, P.status, P.rebuild);
     k_fill_cells<<<nb, 256, 0, st>>>(n, P.cell_of, P.start, P.cur, P.ions, P.rebuild);
-    k_sort_cells<<<ncell, 256, sizeof(int) * NA_CELL_CAP, st>>>(ncell, NA_CELL_CAP, P.start, P.cnt, P.ions,
+    k_sort_cells<<<ncell, 256, sizeof(int) * NA_CELL_CAP, st>>>(ncell, NA_CELL_CAP, P.start, P.cnt, P.ions, P.s, P.pk,
                                                               P.rebuild);
-    k_build<<<(int)(((long long)n * 32 + 255) / 256), 256, 0, st>>>(n, c, g, P.s, P.cell_of, P.start, P.cnt,
-                                                                    P.ions, cut_nb * cut_nb, cut_co * cut_co,
-                                                                    cap_nb, d_nb, d_nbn, cap_co, d_co, d_con,
-                                                                    P.svl, P.status, P.rebuild);
+    try {
+        run_build(st, false, n, c, nc, P.s, P.cell_of, P.start, P.cnt, P.pk, cut_nb, cut_co, cap_nb, d_nb, d_nbn, cap_co,
+                  d_co, d_con, P.status, P.rebuild);
+    } catch (const Error &x) {
+        return x.code;
+    }
     if (cudaGetLastError() != cudaSuccess) return MDFFGPU_ERR_CUDA;
     unsigned s = 0;
     if (cudaMemcpyAsync(&s, P.status, sizeof(unsigned), cudaMemcpyDeviceToHost, st) != cudaSuccess)
