@@ -48,7 +48,6 @@ __global__ void k_cg_step(int n, int nk, const int *polar, const double *pol, do
                           const double3 *ap, double3 *x, double3 *r, double3 *z, const double2 *rho_p, double2 *acc,
                           double *part, int stride, unsigned *ticket, CgTest test);
 __global__ void k_cg_test(CgTest t, const double *scal);
-__global__ void k_upol_final(const double *scal, double coul, DevScalars *out);
 __global__ void k_vv1(int n, double dt, double dtsq2, const double *invm, double4 *r, const double3 *v,
                       const double3 *f, double3 *fs);
 __global__ void k_vv2(int n, double dt2, const double *invm, const double *mass, double3 *v, const double3 *f,
@@ -154,7 +153,7 @@ Engine::Engine(const mdffgpu_params &prm, int dev) : p(prm) {
     d_svl = dalloc<double4>(n);
     d_rebuild = dalloc<int>(1);
     d_status = dalloc<unsigned>(1);
-    d_ticket = dalloc<unsigned>(8);
+    d_ticket = dalloc<unsigned>(16);
     d_scal = dalloc<double>(NSLOT);
     d_out = dalloc<DevScalars>(1);
     d_nhc = dalloc<double>(48);
@@ -775,7 +774,7 @@ void Engine::field_pol(const double3 *d_p, double3 *d_out, double2 *rho_raw, boo
         o.cg.invpol = d_invpol;
         o.cg.p = d_p;
         o.cg.ap = d_cg_ap;
-        o.cg.part = d_part;
+        o.cg.part = cg_clustered(*this) ? nullptr : d_part;
         o.cg.stride = part_stride;
         o.cg.scal = d_scal;
         o.cg.ticket = d_ticket;
@@ -1006,9 +1005,10 @@ void Engine::pim_cg(bool fused) {
     // one evaluation for the residual: in the fused CG, and in the plain one without static
     // dipoles (with them it keeps E_stat and T mu0 apart: a dipole acts on an ion only where
     // that ion's own dipole is non-zero, src/ewald.c:737)
+    const bool clustered = cg_clustered(*this);
+    const double3 *efs = nullptr;   // E_stat where the field pass does not hold it
     if (fused || !ldip) {
-        MDFF_LAUNCH(*this, k_aspc_predict, nb, 256, 0, n, aspc_coef(e, cg_poly), es, d_hist, d_mu_ind);
-        MDFF_LAUNCH(*this, k_add3, nb, 256, 0, n, d_mu_static, d_mu_ind, d_mu_tot);
+        launch_pim_begin(*this, aspc_coef(e, cg_poly), es);
         // the residual reads the field at the polarisable ions only (FP64 real space
         // evaluates every ion; the k-space ion pass and FP32 real space only those)
         bool sub = subset32 && npol > 0;
@@ -1035,17 +1035,20 @@ void Engine::pim_cg(bool fused) {
         }
         launch_rec(*this, d_q, d_mu_tot, lqch != 0, true, o);
         join_side(SIDE_PREP);   // (joined by the ion pass already; the loop below reads the records)
-        MDFF_LAUNCH(*this, k_cg_residual, nb, 256, 0, n, d_polar, d_invpol, d_muzero, d_ef_ind, d_mu_ind, d_cg_r);
     } else {
         join_side(SIDE_PREP);
         field_of(d_q, d_mu_static, lqch != 0, ldip != 0, ldmp != 0, d_ef_stat);
-        MDFF_LAUNCH(*this, k_aspc_predict, nb, 256, 0, n, aspc_coef(e, cg_poly), es, d_hist, d_mu_ind);
+        launch_pim_begin(*this, aspc_coef(e, cg_poly), es);
         field_of(d_qzero, d_mu_ind, false, true, false, d_ef_ind);
-        MDFF_LAUNCH(*this, k_cg_residual, nb, 256, 0, n, d_polar, d_invpol, d_ef_stat, d_ef_ind, d_mu_ind, d_cg_r);
+        efs = d_ef_stat;
     }
-    MDFF_LAUNCH(*this, k_cg_rz, nb, 256, 0, n, d_polar, d_pol, d_cg_r, d_mu_save, d_part, part_stride, d_scal,
-                d_ticket + 1);
-    MDFF_CK(cudaMemcpyAsync(d_cg_p, d_mu_save, sizeof(double3) * n, cudaMemcpyDeviceToDevice, stream));
+    if (!clustered) {
+        MDFF_LAUNCH(*this, k_cg_residual, nb, 256, 0, n, d_polar, d_invpol, efs ? efs : d_muzero, d_ef_ind, d_mu_ind,
+                    d_cg_r);
+        MDFF_LAUNCH(*this, k_cg_rz, nb, 256, 0, n, d_polar, d_pol, d_cg_r, d_mu_save, d_part, part_stride, d_scal,
+                    d_ticket + 1);
+        MDFF_CK(cudaMemcpyAsync(d_cg_p, d_mu_save, sizeof(double3) * n, cudaMemcpyDeviceToDevice, stream));
+    }
     int maxit = std::max(p.max_scf_pim_iter, 1);
     // one CG iteration up to the new residual norm and, recorded, the loop test in the
     // same launch (p <- z + beta p follows the test)
@@ -1067,24 +1070,30 @@ void Engine::pim_cg(bool fused) {
                         part_stride, d_scal, d_ticket);
         }
         // x, r update, rho(k) of the iterate, z = alpha r and the new r.z, r.r: one launch
-        MDFF_LAUNCH(*this, k_cg_step, nb + (fused ? ceil_div(nk, 256) : 0), 256, 0, n, nk, d_polar, d_pol, d_scal,
-                    d_cg_p, d_cg_ap, d_mu_ind, d_cg_r, d_mu_save, d_rho_it, fused ? d_rho_acc : nullptr, d_part,
-                    part_stride, d_ticket + 1, t);
+        // (clustered: p too)
+        if (clustered)
+            launch_cg_update(*this, d_mu_ind, d_rho_it, fused ? d_rho_acc : nullptr, t);
+        else
+            MDFF_LAUNCH(*this, k_cg_step, nb + (fused ? ceil_div(nk, 256) : 0), 256, 0, n, nk, d_polar, d_pol, d_scal,
+                        d_cg_p, d_cg_ap, d_mu_ind, d_cg_r, d_mu_save, d_rho_it, fused ? d_rho_acc : nullptr, d_part,
+                        part_stride, d_ticket + 1, t);
     };
     if (capturing) {
         // graph: the loop is a while node whose condition the device test sets
         record_while(
             [&](cudaGraphConditionalHandle h) {
                 test.h = h;
-                MDFF_LAUNCH(*this, k_cg_test, 1, 32, 0, test, d_scal);
+                if (clustered) launch_cg_begin(*this, efs, d_ef_ind, nullptr, d_mu_ind, test);
+                else MDFF_LAUNCH(*this, k_cg_test, 1, 32, 0, test, d_scal);
             },
             [&](cudaGraphConditionalHandle h) {
                 test.h = h;
                 iteration(test);
-                MDFF_LAUNCH(*this, k_cg_dir, nb, 256, 0, n, d_scal, d_mu_save, d_cg_p, test);
+                if (!clustered) MDFF_LAUNCH(*this, k_cg_dir, nb, 256, 0, n, d_scal, d_mu_save, d_cg_p, test);
             });
     } else {
         double rr = 0.0;
+        if (clustered) launch_cg_begin(*this, efs, d_ef_ind, nullptr, d_mu_ind, CgTest{});
         MDFF_CK(cudaMemcpyAsync(&rr, d_scal + S_RR, sizeof(double), cudaMemcpyDeviceToHost, stream));
         MDFF_CK(cudaStreamSynchronize(stream));
         double rmsd = std::sqrt(rr / (double)std::max(npol, 1));
@@ -1098,16 +1107,12 @@ void Engine::pim_cg(bool fused) {
             if (!std::isfinite(rmsd)) throw Error(MDFFGPU_ERR_NONFINITE, "CG diverged");
             it++;
             if (rmsd <= p.conv_tol_ind) break;
-            MDFF_LAUNCH(*this, k_cg_dir, nb, 256, 0, n, d_scal, d_mu_save, d_cg_p, none);
+            if (!clustered) MDFF_LAUNCH(*this, k_cg_dir, nb, 256, 0, n, d_scal, d_mu_save, d_cg_p, none);
         }
         if (rmsd > p.conv_tol_ind) throw Error(MDFFGPU_ERR_SCF, "CG did not converge in max_scf_pim_iter");
         last_scf_iter = it;
         last_rmsd = rmsd;
     }
-    MDFF_LAUNCH(*this, k_pim_sums, nb, 256, 0, n, d_polar, d_pol, d_invpol, d_mu_ind, d_ef_stat, d_part, part_stride);
-    reduce(S_UPOL, 1, nb);
-    MDFF_LAUNCH(*this, k_upol_final, 1, 32, 0, d_scal, coul_unit, d_out);
-    MDFF_LAUNCH(*this, k_hist_store, nb, 256, 0, n, d_mu_ind, d_hist);
     rho_acc_ready = fused;
 }
 
@@ -1214,11 +1219,16 @@ void Engine::get_dipoles() {
             pim_cg(pim_solver == MDFFGPU_PIM_CG_FUSED);
         else if (p.algo_pim == 1) pim_ko();
         else pim_reference();
-        int nb = ceil_div(n, 256);
-        MDFF_LAUNCH(*this, k_add3, nb, 256, 0, n, d_mu_static, d_mu_ind, d_mu_tot);
-    } else {
-        MDFF_CK(cudaMemcpyAsync(d_mu_tot, d_mu_static, sizeof(double3) * n, cudaMemcpyDeviceToDevice, stream));
+        if (!cont) {
+            int nb = ceil_div(n, 256);
+            MDFF_LAUNCH(*this, k_add3, nb, 256, 0, n, d_mu_static, d_mu_ind, d_mu_tot);
+            MDFF_LAUNCH(*this, k_self_sums, nb, 256, 0, n, d_q, d_mu_tot, d_part, part_stride);
+            reduce(S_Q2, 2, nb);
+            return;
+        }
     }
+    // total dipoles, the self sums and, after a CG, u_pol and the history
+    launch_pim_finish(*this, cont);
 }
 
 void Engine::finalize_coul(bool stress) {
@@ -1274,9 +1284,6 @@ void Engine::engforce(bool check_finite) {
         rho_acc_ready = false;
         launch_rec(*this, d_q, d_mu_tot, lqch != 0, ld, o);
         join_side(SIDE_DIR);
-        int nb = ceil_div(n, 256);
-        MDFF_LAUNCH(*this, k_self_sums, nb, 256, 0, n, d_q, d_mu_tot, d_part, part_stride);
-        reduce(S_Q2, 2, nb);
         finalize_coul(true);
     }
     for (int k = 0; k < NSIDE; k++) join_side(k);

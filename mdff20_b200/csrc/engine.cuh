@@ -80,6 +80,36 @@ struct CgTest {
                            // whatever k_cg_step did (a backstop of the while node)
 };
 
+// the loop test of CgTest on the new |r|^2 (first: before the first iteration, count 0)
+__device__ __forceinline__ void cg_test(const CgTest &t, double rr, int first) {
+    unsigned go = 0;
+    if (t.mode == 1) {
+        const double rmsd = sqrt(rr / (double)(t.npol > 1 ? t.npol : 1));
+        const int it = first ? 0 : t.out->scf_iter + 1;
+        t.out->scf_iter = it;
+        t.out->scf_rmsd = rmsd;
+        if (!isfinite(rmsd)) atomicOr(t.status, (unsigned)ST_NONFINITE);
+        else if (rmsd > t.tol) {
+            if (it < t.maxit) go = 1;
+            else atomicOr(t.status, (unsigned)ST_SCF);
+        }
+    } else {
+        if (first) {
+            *t.rr0 = rr;
+            *t.itc = 0.0;
+        } else {
+            *t.itc += 1.0;
+        }
+        const int it = (int)*t.itc;
+        if (!isfinite(rr)) atomicOr(t.status, (unsigned)ST_NONFINITE);
+        else if (rr > t.rtol2 * *t.rr0 && rr > 0.0) {
+            if (it < t.maxit) go = 1;
+            else atomicOr(t.status, (unsigned)ST_SCF);
+        }
+    }
+    cudaGraphSetConditional(t.h, go);
+}
+
 struct Engine;
 
 // zero-initialised device allocation; MDFFGPU_ERR_NOMEM on failure.  The zeroing runs on
@@ -122,7 +152,7 @@ struct CgAp {
     const double *invpol = nullptr;
     const double3 *p = nullptr;
     double3 *ap = nullptr;            // null: not formed
-    double *part = nullptr;
+    double *part = nullptr;           // null: p.ap is formed by the update (cg.cu)
     int stride = 0;
     double *scal = nullptr;
     unsigned *ticket = nullptr;
@@ -207,6 +237,18 @@ bool launch_rho_tc(Engine &e, const double *q, const double3 *mu, bool lq, bool 
 void launch_rho_tc_tables(Engine &e);
 void setup_rho_tc(Engine &e, int lz);
 void launch_ion32(Engine &e, const double *q, const double3 *mu, bool ld, const RecOut &o, const int *idx, int cnt);
+
+// cg.cu: one CG iteration's vector work (p.Ap, x, r, rho(k) of the iterate, z, r.z, r.r, the
+// loop test, p) in one launch of a thread-block cluster, and the start of the solve; for up to
+// CG_CLUSTER_MAX polarisable ions (cg_clustered)
+bool cg_clustered(const Engine &e);
+// r = efs + tx - invpol x (efs may be null), or with rhs: r = rhs, x = 0; z = alpha r, p = z
+void launch_cg_begin(Engine &e, const double3 *efs, const double3 *tx, const double3 *rhs, double3 *x, const CgTest &t);
+void launch_cg_update(Engine &e, double3 *x, const double2 *rho_p, double2 *acc, const CgTest &t);
+// the predicted dipoles and history shift; the end of the solve: total dipoles, history, u_pol,
+// and the self sums of charges and dipoles (pim false: static dipoles only, no solve)
+void launch_pim_begin(Engine &e, const AspcCoef &cf, int es);
+void launch_pim_finish(Engine &e, bool pim);
 
 // ---------------------------------------------------------------- engine state
 struct Engine {
@@ -522,9 +564,13 @@ struct Engine {
 // fewer configurations per second with it).
 
 // launch bookkeeping: every kernel launch goes through this
-#define MDFF_LAUNCH(eng, kernel, grid, block, smem, ...)                               \
+#define MDFF_LAUNCH(eng, kernel, grid, block, smem, ...) \
+    MDFF_LAUNCH_C(eng, 1, kernel, grid, block, smem, __VA_ARGS__)
+// ... in thread-block clusters of `cs` blocks
+#define MDFF_LAUNCH_C(eng, cs, kernel, grid, block, smem, ...)                         \
     do {                                                                               \
-        cudaLaunchAttribute at_[2];                                                    \
+        const unsigned MDFF_CLUSTER = (cs);                                                                               \
+        cudaLaunchAttribute at_[3];                                                    \
         unsigned na_ = 0;                                                              \
         if ((eng).pdl) {                                                               \
             at_[na_].id = cudaLaunchAttributeProgrammaticStreamSerialization;          \
@@ -539,6 +585,12 @@ struct Engine {
         cfg_.blockDim = dim3(block);                                                   \
         cfg_.dynamicSmemBytes = (smem);                                                \
         cfg_.stream = (eng).stream;                                                    \
+        if (MDFF_CLUSTER > 1) {                                                        \
+            at_[na_].id = cudaLaunchAttributeClusterDimension;                         \
+            at_[na_].val.clusterDim.x = MDFF_CLUSTER;                                  \
+            at_[na_].val.clusterDim.y = 1;                                             \
+            at_[na_++].val.clusterDim.z = 1;                                           \
+        }                                                                              \
         cfg_.attrs = at_;                                                              \
         cfg_.numAttrs = na_;                                                           \
         MDFF_CK(cudaLaunchKernelEx(&cfg_, kernel, __VA_ARGS__));                       \

@@ -505,11 +505,14 @@ void Engine::fit_apply_theta(const double *d_th, int tSi, int tO) {
 // recording, the loop is a device-controlled while node (the test in k_cg_step)
 void Engine::solve_pim(const double3 *d_b, double3 *d_x, double rtol, int maxit) {
     int nb = ceil_div(n, 256);
-    MDFF_CK(cudaMemsetAsync(d_x, 0, sizeof(double3) * n, stream));
-    MDFF_CK(cudaMemcpyAsync(d_cg_r, d_b, sizeof(double3) * n, cudaMemcpyDeviceToDevice, stream));
-    MDFF_LAUNCH(*this, k_cg_rz, nb, 256, 0, n, d_polar, d_pol, d_cg_r, d_mu_save, d_part, part_stride, d_scal,
-                d_ticket + 1);
-    MDFF_CK(cudaMemcpyAsync(d_cg_p, d_mu_save, sizeof(double3) * n, cudaMemcpyDeviceToDevice, stream));
+    const bool clustered = cg_clustered(*this);
+    if (!clustered) {
+        MDFF_CK(cudaMemsetAsync(d_x, 0, sizeof(double3) * n, stream));
+        MDFF_CK(cudaMemcpyAsync(d_cg_r, d_b, sizeof(double3) * n, cudaMemcpyDeviceToDevice, stream));
+        MDFF_LAUNCH(*this, k_cg_rz, nb, 256, 0, n, d_polar, d_pol, d_cg_r, d_mu_save, d_part, part_stride, d_scal,
+                    d_ticket + 1);
+        MDFF_CK(cudaMemcpyAsync(d_cg_p, d_mu_save, sizeof(double3) * n, cudaMemcpyDeviceToDevice, stream));
+    }
     // A p: the search direction vanishes off the polarisable ions, so the field passes
     // run over those ions only; A p and p.A p in the ion pass (or k_cg_ap), then x, r, z and r.z, r.r in one launch, as the induced-dipole CG does
     CgTest test{};
@@ -527,23 +530,28 @@ void Engine::solve_pim(const double3 *d_b, double3 *d_x, double rtol, int maxit)
         if (!sub)
             MDFF_LAUNCH(*this, k_cg_ap, nb, 256, 0, n, d_polar, d_invpol, d_cg_p, d_ef_ind, d_cg_ap, d_part,
                         part_stride, d_scal, d_ticket);
-        MDFF_LAUNCH(*this, k_cg_step, nb, 256, 0, n, 0, d_polar, d_pol, d_scal, d_cg_p, d_cg_ap, d_x, d_cg_r,
-                    d_mu_save, nullptr, nullptr, d_part, part_stride, d_ticket + 1, t);
+        if (clustered)
+            launch_cg_update(*this, d_x, nullptr, nullptr, t);
+        else
+            MDFF_LAUNCH(*this, k_cg_step, nb, 256, 0, n, 0, d_polar, d_pol, d_scal, d_cg_p, d_cg_ap, d_x, d_cg_r,
+                        d_mu_save, nullptr, nullptr, d_part, part_stride, d_ticket + 1, t);
     };
     if (capturing) {
         record_while(
             [&](cudaGraphConditionalHandle h) {
                 test.h = h;
-                MDFF_LAUNCH(*this, k_cg_test, 1, 32, 0, test, d_scal);
+                if (clustered) launch_cg_begin(*this, nullptr, nullptr, d_b, d_x, test);
+                else MDFF_LAUNCH(*this, k_cg_test, 1, 32, 0, test, d_scal);
             },
             [&](cudaGraphConditionalHandle h) {
                 test.h = h;
                 iteration(test);
-                MDFF_LAUNCH(*this, k_cg_dir, nb, 256, 0, n, d_scal, d_mu_save, d_cg_p, test);
+                if (!clustered) MDFF_LAUNCH(*this, k_cg_dir, nb, 256, 0, n, d_scal, d_mu_save, d_cg_p, test);
             });
         return;
     }
     double rr0 = 0.0, rr = 0.0;
+    if (clustered) launch_cg_begin(*this, nullptr, nullptr, d_b, d_x, CgTest{});
     MDFF_CK(cudaMemcpyAsync(&rr0, d_scal + S_RR, sizeof(double), cudaMemcpyDeviceToHost, stream));
     MDFF_CK(cudaStreamSynchronize(stream));
     rr = rr0;
@@ -555,7 +563,7 @@ void Engine::solve_pim(const double3 *d_b, double3 *d_x, double rtol, int maxit)
         MDFF_CK(cudaStreamSynchronize(stream));
         if (!std::isfinite(rr)) throw Error(MDFFGPU_ERR_NONFINITE, "adjoint CG diverged");
         it++;
-        MDFF_LAUNCH(*this, k_cg_dir, nb, 256, 0, n, d_scal, d_mu_save, d_cg_p, none);
+        if (!clustered) MDFF_LAUNCH(*this, k_cg_dir, nb, 256, 0, n, d_scal, d_mu_save, d_cg_p, none);
     }
     if (rr > rtol * rtol * rr0 && rr > 0.0) throw Error(MDFFGPU_ERR_SCF, "adjoint CG did not converge");
     last_adj_iter = it;

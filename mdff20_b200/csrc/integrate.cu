@@ -340,43 +340,12 @@ __global__ void k_cg_rz(int n, const int *__restrict__ polar, const double *__re
     last_block_slots(part, stride, S_RZ, 2, scal, ticket);
 }
 
-// the loop test of CgTest (first: before the first iteration, iteration count 0)
-__device__ void cg_test(const CgTest &t, const double *scal, int first) {
-    const double rr = scal[S_RR];
-    unsigned go = 0;
-    if (t.mode == 1) {
-        const double rmsd = sqrt(rr / (double)(t.npol > 1 ? t.npol : 1));
-        const int it = first ? 0 : t.out->scf_iter + 1;
-        t.out->scf_iter = it;
-        t.out->scf_rmsd = rmsd;
-        if (!isfinite(rmsd)) atomicOr(t.status, (unsigned)ST_NONFINITE);
-        else if (rmsd > t.tol) {
-            if (it < t.maxit) go = 1;
-            else atomicOr(t.status, (unsigned)ST_SCF);
-        }
-    } else {
-        if (first) {
-            *t.rr0 = rr;
-            *t.itc = 0.0;
-        } else {
-            *t.itc += 1.0;
-        }
-        const int it = (int)*t.itc;
-        if (!isfinite(rr)) atomicOr(t.status, (unsigned)ST_NONFINITE);
-        else if (rr > t.rtol2 * *t.rr0 && rr > 0.0) {
-            if (it < t.maxit) go = 1;
-            else atomicOr(t.status, (unsigned)ST_SCF);
-        }
-    }
-    cudaGraphSetConditional(t.h, go);
-}
-
 // the test of a recorded loop before its first iteration
 __global__ void k_cg_test(CgTest t, const double *scal) {
     grid_dep();
     if (threadIdx.x || blockIdx.x) return;
     *t.guard = 0u;
-    cg_test(t, scal, 1);
+    cg_test(t, scal[S_RR], 1);
 }
 
 // One CG update in a single launch: x += a p, r -= a Ap (a = rz / pAp, rz kept as rz_old),
@@ -420,7 +389,7 @@ __global__ void k_cg_step(int n, int nk, const int *__restrict__ polar, const do
     }
     block_sum_to_part<2>(v, part, S_RZ, stride);  // r.z, r.r
     const bool last = last_block_slots(part, stride, S_RZ, 2, scal, ticket);
-    if (last && threadIdx.x == 0 && test.mode) cg_test(test, scal, 0);
+    if (last && threadIdx.x == 0 && test.mode) cg_test(test, scal[S_RR], 0);
 }
 
 // p = z + beta p, beta = rz_new / rz_old; in a recorded loop (t.mode set) also the
@@ -437,13 +406,6 @@ __global__ void k_cg_dir(int n, const double *__restrict__ scal, const double3 *
     double beta = scal[S_RZ] / scal[S_RZOLD];
     double3 zz = z[i], pp = p[i];
     p[i] = make_double3(zz.x + beta * pp.x, zz.y + beta * pp.y, zz.z + beta * pp.z);
-}
-
-// u_pol = 1/2 sum mu.alpha^-1.mu in energy units
-__global__ void k_upol_final(const double *scal, double coul, DevScalars *out) {
-    grid_dep();
-    if (threadIdx.x || blockIdx.x) return;
-    out->u_pol = 0.5 * scal[S_UPOL] * coul;
 }
 
 // ---------------------------------------------------------------- integrators

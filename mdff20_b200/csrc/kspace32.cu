@@ -593,7 +593,7 @@ __global__ void k_combine32(Comb32Args a) {
             a.f[i] = make_double3(fo.x + fr[0] * a.coul, fo.y + fr[1] * a.coul, fo.z + fr[2] * a.coul);
         }
     }
-    if (!WF && a.cg.ap) {
+    if (!WF && a.cg.ap && a.cg.part) {
         block_sum_to_part<1>(pap, a.cg.part, S_PAP, a.cg.stride);
         last_block_slots(a.cg.part, a.cg.stride, S_PAP, 1, a.cg.scal, a.cg.ticket);
     }

@@ -22,9 +22,9 @@
 // (row, z), so rho(+-z) is formed in the lane.  A lane of the ion pass holds G, H, K of one
 // (ion, row).
 //
-// Measured (B200, 4000 dipoles of 6000 ions, nk 12194, kmax 14): rho pass 89 -> 26.7 us (15
-// TFLOP/s of the 8-flop count), ion pass and combine 68 -> 29 us; at 128 of 192 ions (kmax 10)
-// the rho pass 32 -> 3.9 us.  The thread-per-segment passes these replaced were slower at
+// Measured (B200, 4000 dipoles of 6000 ions, nk 12194, kmax 14): rho pass 89 -> 24.7 us (16
+// TFLOP/s of the 8-flop count), ion pass and combine 68 -> 25.9 us, with forces 104 -> 48.6 us;
+// at 128 of 192 ions (kmax 10) the rho pass 32 -> 3.6 us, the ion pass and combine 25 -> 7.6 us.  The thread-per-segment passes these replaced were slower at
 // every size, so no other FP64 path is kept.
 //
 // |nz| beyond 15 is split in groups of 16 (rho: a grid dimension, ion: more units of work).
@@ -42,7 +42,7 @@ constexpr int I64_WARPS = 4;     // ion pass: warps per block, MT tiles of 8 ion
 constexpr int ZG = 16;           // |nz| values per group (32 table columns)
 
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};"
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};"
         : "+d"(c[0]), "+d"(c[1])
         : "d"(a), "d"(b));
 }
@@ -135,27 +135,33 @@ __global__ void __launch_bounds__(32 * R64_WARPS, 2) k_rho64(Rho64Args a) {
     const int i0 = blockIdx.y * a.chunk, i1 = min(a.n, i0 + a.chunk);
     const int ns = (i1 - i0 + R64_TI - 1) / R64_TI;
     const int zs = a.t.e1 + 2 * a.t.K1 + 1;      // stage offset of the Z columns
-    auto issue = [&](int s, int b) {
-        // 16 threads per ion copy its row; positions past the chunk repeat a valid row and
-        // carry q = mu = 0
-        const int k = threadIdx.x >> 4, pos = i0 + s * R64_TI + k;
-        const int pc = min(pos, i1 - 1), ia = a.idx ? a.idx[pc] : pc;
-        const double2 *src = a.tab + (size_t)ia * a.t.w;
-        double2 *dst = sm + (b * R64_TI + k) * a.stw;
-        for (int x = threadIdx.x & 15; x < zs; x += 16) cp_async16(dst + x, src + x);
-        for (int x = threadIdx.x & 15; x < 4 * NTL; x += 16) cp_async16(dst + zs + x, src + a.t.z + ZG * zg + x);
-        if ((threadIdx.x & 15) == 0) {
-            double qa = 0.0;
-            double3 m = make_double3(0.0, 0.0, 0.0);
+    // 16 threads per ion copy its row; positions past the chunk repeat a valid row and carry
+    // q = mu = 0.  The ion's index, charge and dipole are read one stage before they are used.
+    const int ki = threadIdx.x >> 4, xi = threadIdx.x & 15;
+    int ia = 0;
+    double qn = 0.0;
+    double3 mn = make_double3(0.0, 0.0, 0.0);
+    auto fetch = [&](int s) {
+        const int pos = i0 + s * R64_TI + ki, pc = min(pos, i1 - 1);
+        ia = a.idx ? a.idx[pc] : pc;
+        if (xi == 0) {
+            qn = 0.0;
+            mn = make_double3(0.0, 0.0, 0.0);
             if (pos < i1) {
-                if (LQ) qa = a.q[ia];
-                if (LD) {
-                    const double3 u = a.mu[ia];
-                    m = to_phase(a.c, TPI_D * u.x, TPI_D * u.y, TPI_D * u.z);
-                }
+                if (LQ) qn = a.q[ia];
+                if (LD) mn = a.mu[ia];
             }
-            qm[(b * R64_TI + k) * 2] = make_double2(qa, m.x);
-            qm[(b * R64_TI + k) * 2 + 1] = make_double2(m.y, m.z);
+        }
+    };
+    auto issue = [&](int b) {
+        const double2 *src = a.tab + (size_t)ia * a.t.w;
+        double2 *dst = sm + (b * R64_TI + ki) * a.stw;
+        for (int x = xi; x < zs; x += 16) cp_async16(dst + x, src + x);
+        for (int x = xi; x < 4 * NTL; x += 16) cp_async16(dst + zs + x, src + a.t.z + ZG * zg + x);
+        if (xi == 0) {
+            const double3 m = LD ? to_phase(a.c, TPI_D * mn.x, TPI_D * mn.y, TPI_D * mn.z) : make_double3(0, 0, 0);
+            qm[(b * R64_TI + ki) * 2] = make_double2(qn, m.x);
+            qm[(b * R64_TI + ki) * 2 + 1] = make_double2(m.y, m.z);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -167,12 +173,20 @@ __global__ void __launch_bounds__(32 * R64_WARPS, 2) k_rho64(Rho64Args a) {
     const double nx = (double)R.nx, ny = (double)R.ny;
     const int x0 = R.nx, x1 = a.t.e1 + a.t.K1 + R.ny;
     const bool two = a.nbuf == 2;
-    if (ns > 0 && two) issue(0, 0);
+    fetch(0);
+    if (two) {
+        issue(0);
+        fetch(1);
+    }
     for (int s = 0; s < ns; s++) {
         const int b = two ? s & 1 : 0;
-        if (!two) issue(s, 0);
+        if (!two) {
+            issue(0);
+            fetch(s + 1);
+        }
         if (two && s + 1 < ns) {
-            issue(s + 1, b ^ 1);
+            issue(b ^ 1);
+            fetch(s + 2);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -326,7 +340,10 @@ __global__ void __launch_bounds__(256) k_rho64_sum(Red64Args a) {
             }
         }
     }
-    if (a.energy) last_block_slots(a.ppart, a.stride, a.slot, 7, a.scal, a.ticket);
+    if (a.energy) {
+        const int slots[7] = {a.slot, a.slot + 1, a.slot + 2, a.slot + 3, a.slot + 4, a.slot + 5, a.slot + 6};
+        last_block_warps(a.ppart, a.stride, slots, 7, a.scal, a.ticket);
+    }
 }
 
 // ---------------------------------------------------------------- ion pass
@@ -427,32 +444,54 @@ __device__ __forceinline__ double ion64_write(const Ion64Args &a, int i, const d
     return pap;
 }
 
-// grid (blocks of 32 MT ions, slices).  A warp keeps its ions' table columns (the A fragments
-// of all k steps) in registers and streams the weights (coalesced, shared by the block
-// through L1); the last block of an ion block to finish sums the slices in slice order and
-// writes the results (a separate combine launch cost 4-8 us of a 20-60 us pass).
-template <int KS, bool WF, int MT>
-__global__ void __launch_bounds__(32 * I64_WARPS) k_ion64(Ion64Args a) {
+// WS = 1: grid (blocks of 32 MT ions, slices), the block's four warps hold four tiles of 8 MT
+// ions.  WS = 8: grid (blocks of 8 MT ions, slices / 8), the block's eight warps take eight row
+// slices of the same ions and add them in shared memory (few ions: the chip fills without
+// partial sums in memory and their arrival counters, 11.8 -> 7.6 us at 128 ions, kmax 10).  A warp keeps
+// its ions' table columns (the A fragments of all k steps) in registers and streams the
+// weights (coalesced); with more than one slice in the grid the last block of an ion block to
+// finish sums them in slice order and writes the results.
+template <int KS, bool WF, int MT, int WS>
+__global__ void __launch_bounds__(WS == 1 ? 32 * I64_WARPS : 32 * WS) k_ion64(Ion64Args a) {
     grid_dep();
-    constexpr int NTT = WF ? 3 : 2, NV = WF ? 9 : 3;
+    constexpr int NTT = WF ? 3 : 2, NV = WF ? 9 : 3, IW = WS == 1 ? I64_WARPS : 1;   // warps over the ions
     const int l = threadIdx.x & 31, w = threadIdx.x >> 5, lk = l & 3, lr = l >> 2;
-    const int base = (blockIdx.x * I64_WARPS + w) * 8 * MT;
+    const int base = (blockIdx.x * IW + (WS == 1 ? w : 0)) * 8 * MT;
     const double2 *T[MT];
 #pragma unroll
     for (int m = 0; m < MT; m++) {
         const int pos = min(base + 8 * m + lr, a.cnt - 1);
         T[m] = a.tab + (size_t)(a.idx ? a.idx[pos] : pos) * a.t.w;
     }
-    const int u0 = (int)((long long)blockIdx.y * a.units / a.slices);
-    const int u1 = (int)((long long)(blockIdx.y + 1) * a.units / a.slices);
+    const int ns = a.slices * WS, sl = WS == 1 ? blockIdx.y : blockIdx.y * WS + w;
+    const int u0 = (int)((long long)sl * a.units / ns);
+    const int u1 = (int)((long long)(sl + 1) * a.units / ns);
     double A[MT][KS], S[MT][NV];
 #pragma unroll
     for (int m = 0; m < MT; m++)
 #pragma unroll
         for (int v = 0; v < NV; v++) S[m][v] = 0.0;
+    // the next unit's weights are read into the registers each k step frees, its rows' phase
+    // factors before the products, the (nx, ny) of its rows one unit earlier still
+    double B[NTT * KS];
+    double2 xy, e0[MT], e1[MT];
+    auto rows_of = [&](int u) { return a.rowxy[4 * (min(u, u1 - 1) % a.nrg) + lk]; };
+    auto factors = [&](double2 r) {
+        const int x0 = (int)r.x, x1 = a.t.e1 + a.t.K1 + (int)r.y;
+#pragma unroll
+        for (int m = 0; m < MT; m++) e0[m] = T[m][x0], e1[m] = T[m][x1];
+    };
     int zg = -1;
+    if (u0 < u1) {
+        const double *W = a.w + (size_t)u0 * 3 * KS * 32 + l;
+#pragma unroll
+        for (int s = 0; s < NTT * KS; s++) B[s] = W[s * 32];
+        xy = rows_of(u0);
+        factors(xy);
+    }
+    double2 xn = u0 < u1 ? rows_of(u0 + 1) : make_double2(0.0, 0.0);
     for (int u = u0; u < u1; u++) {
-        const int g = u / a.nrg, rg = u - g * a.nrg;
+        const int g = u / a.nrg;
         if (g != zg) {
             zg = g;
 #pragma unroll
@@ -460,79 +499,99 @@ __global__ void __launch_bounds__(32 * I64_WARPS) k_ion64(Ion64Args a) {
 #pragma unroll
                 for (int s = 0; s < KS; s++) A[m][s] = ((const double *)(T[m] + a.t.z + ZG * g))[4 * s + lk];
         }
-        const double2 xy = a.rowxy[4 * rg + lk];
-        const int x0 = (int)xy.x, x1 = a.t.e1 + a.t.K1 + (int)xy.y;
+        const double fx = xy.x, fy = xy.y;
+        double2 ph[MT];
+#pragma unroll
+        for (int m = 0; m < MT; m++)
+            ph[m] = make_double2(e0[m].x * e1[m].x - e0[m].y * e1[m].y, e0[m].x * e1[m].y + e0[m].y * e1[m].x);
+        xy = xn;
+        factors(xy);
+        xn = rows_of(u + 2);
         double acc[MT][NTT][2];
 #pragma unroll
         for (int m = 0; m < MT; m++)
 #pragma unroll
             for (int t = 0; t < NTT; t++) acc[m][t][0] = acc[m][t][1] = 0.0;
-        const double *W = a.w + (size_t)u * 3 * KS * 32 + l;
+        const double *W = a.w + (size_t)min(u + 1, u1 - 1) * 3 * KS * 32 + l;
 #pragma unroll
         for (int s = 0; s < KS; s++)
 #pragma unroll
             for (int t = 0; t < NTT; t++) {
-                const double b = W[(t * KS + s) * 32];
 #pragma unroll
-                for (int m = 0; m < MT; m++) dmma(acc[m][t], A[m][s], b);
+                for (int m = 0; m < MT; m++) dmma(acc[m][t], A[m][s], B[t * KS + s]);
+                B[t * KS + s] = W[(t * KS + s) * 32];
             }
 #pragma unroll
         for (int m = 0; m < MT; m++) {
-            const double2 e0 = T[m][x0], e1 = T[m][x1];
-            const double wx = e0.x * e1.x - e0.y * e1.y, wy = e0.x * e1.y + e0.y * e1.x;
+            const double wx = ph[m].x, wy = ph[m].y;
             const double Rg = wx * acc[m][0][1] - wy * acc[m][0][0], Rh = wx * acc[m][1][1] - wy * acc[m][1][0];
-            S[m][0] += xy.x * Rg;
-            S[m][1] += xy.y * Rg;
+            S[m][0] += fx * Rg;
+            S[m][1] += fy * Rg;
             S[m][2] += Rh;
             if (WF) {
                 const double Q0 = wx * acc[m][0][0] + wy * acc[m][0][1];
                 const double Q1 = wx * acc[m][1][0] + wy * acc[m][1][1];
                 const double Q2 = wx * acc[m][NTT - 1][0] + wy * acc[m][NTT - 1][1];
-                const double a0 = xy.x * Q0, a1 = xy.y * Q0;
-                S[m][NV - 6] += xy.x * a0;
-                S[m][NV - 5] += xy.x * a1;
-                S[m][NV - 4] += xy.x * Q1;
-                S[m][NV - 3] += xy.y * a1;
-                S[m][NV - 2] += xy.y * Q1;
+                const double a0 = fx * Q0, a1 = fy * Q0;
+                S[m][NV - 6] += fx * a0;
+                S[m][NV - 5] += fx * a1;
+                S[m][NV - 4] += fx * Q1;
+                S[m][NV - 3] += fy * a1;
+                S[m][NV - 2] += fy * Q1;
                 S[m][NV - 1] += Q2;
             }
         }
     }
-    double *part = a.part + (size_t)blockIdx.y * a.cnt * NV;
+    // the block's sums: per ion of the block, WS row slices each, in shared memory
+    constexpr int NI = 8 * MT * IW;   // ions of the block
+    __shared__ double red[WS][NI][NV];
 #pragma unroll
-    for (int m = 0; m < MT; m++) {
-        const int pos = base + 8 * m + lr;
+    for (int m = 0; m < MT; m++)
 #pragma unroll
         for (int v = 0; v < NV; v++) {
             double s = S[m][v];
             s += __shfl_xor_sync(0xffffffffu, s, 1);
             s += __shfl_xor_sync(0xffffffffu, s, 2);
-            if (lk == 0 && pos < a.cnt) part[(size_t)pos * NV + v] = s;
+            if (lk == 0) red[WS == 1 ? 0 : w][(WS == 1 ? 8 * MT * w : 0) + 8 * m + lr][v] = s;
         }
-    }
-    // last slice of this ion block
-    __shared__ bool last;
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) {
-        last = atomicAdd(a.btick + blockIdx.x, 1u) == (unsigned)a.slices - 1u;
-        if (last) a.btick[blockIdx.x] = 0u;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    const int li = blockIdx.x * 8 * MT * I64_WARPS + threadIdx.x;
-    double pap[1] = {0.0};
-    if (threadIdx.x < 8 * MT * I64_WARPS && li < a.cnt) {
-        double t[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        for (int s = 0; s < a.slices; s++) {
-            const double *o = a.part + ((size_t)s * a.cnt + li) * NV;
+    const int i0 = blockIdx.x * NI, ni = min(NI, a.cnt - i0);
+    for (int k = threadIdx.x; k < NI * NV; k += blockDim.x) {
+        const int q = k / NV, v = k - q * NV;
+        double s = red[0][q][v];
 #pragma unroll
-            for (int v = 0; v < NV; v++) t[v] += __ldcg(o + v);
-        }
-        pap[0] = ion64_write<WF>(a, a.idx ? a.idx[li] : li, t);
+        for (int x = 1; x < WS; x++) s += red[x][q][v];
+        if (a.slices == 1) red[0][q][v] = s;
+        else if (q < ni) a.part[((size_t)blockIdx.y * a.cnt + i0 + q) * NV + v] = s;
     }
-    if (!WF && a.cg.ap) {
+    if (a.slices > 1) {   // the last slice of this ion block goes on, with all slices added
+        __shared__ bool last;
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            last = atomicAdd(a.btick + blockIdx.x, 1u) == (unsigned)a.slices - 1u;
+            if (last) a.btick[blockIdx.x] = 0u;
+        }
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        for (int k = threadIdx.x; k < ni * NV; k += blockDim.x) {
+            const double *o = a.part + (size_t)i0 * NV + k;
+            double s = 0.0;
+#pragma unroll 4
+            for (int x = 0; x < a.slices; x++) s += __ldcg(o + (size_t)x * a.cnt * NV);
+            red[0][k / NV][k % NV] = s;
+        }
+    }
+    __syncthreads();
+    double pap[1] = {0.0};
+    if ((int)threadIdx.x < ni) {
+        double t[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+        for (int v = 0; v < NV; v++) t[v] = red[0][threadIdx.x][v];
+        pap[0] = ion64_write<WF>(a, a.idx ? a.idx[i0 + threadIdx.x] : i0 + threadIdx.x, t);
+    }
+    if (!WF && a.cg.ap && a.cg.part) {
         block_sum_to_part<1>(pap, a.cg.part, S_PAP, a.cg.stride);
         last_block_slots(a.cg.part, a.cg.stride, S_PAP, 1, a.cg.scal, a.cg.ticket);
     }
@@ -573,7 +632,7 @@ void setup_kspace64(Engine &e, const std::vector<KRow> &rows) {
     MDFF_CK(cudaMemcpy(e.d_rowxy, xy.data(), sizeof(double2) * xy.size(), cudaMemcpyHostToDevice));
     e.rho64_chunks_max = std::max(1, std::min(64, ceil_div(e.n, R64_TI)));
     e.d_rho_part = dalloc<double2>((size_t)e.rho64_chunks_max * e.nk);
-    e.d_btick = dalloc<unsigned>(ceil_div(e.n, 8 * I64_WARPS) + 1);
+    e.d_btick = dalloc<unsigned>(ceil_div(e.n, 8) + 1);
     e.ion64_slices_max = std::max(1, std::min({t.nzg * nrg, 32, std::max(4, 65536 / e.n)}));
     e.d_ion_part = dalloc<double>((size_t)e.ion64_slices_max * e.n * 9);
 }
@@ -598,16 +657,18 @@ static void rho64_ks(Engine &e, const Rho64Args &a, dim3 grid, size_t smem, bool
 }
 
 template <int KS, bool WF>
-static void ion64_mt(Engine &e, const Ion64Args &a, dim3 grid, int mt) {
-    if (mt == 4 && !WF) MDFF_LAUNCH(e, (k_ion64<KS, WF, WF ? 2 : 4>), grid, 32 * I64_WARPS, 0, a);
-    else if (mt == 2) MDFF_LAUNCH(e, (k_ion64<KS, WF, 2>), grid, 32 * I64_WARPS, 0, a);
-    else MDFF_LAUNCH(e, (k_ion64<KS, WF, 1>), grid, 32 * I64_WARPS, 0, a);
+static void ion64_mt(Engine &e, const Ion64Args &a, dim3 grid, int mt, int ws) {
+    constexpr int M4 = WF ? 2 : 4;
+    if (ws == 8 && mt == 2) MDFF_LAUNCH(e, (k_ion64<KS, WF, 2, 8>), grid, 256, 0, a);
+    else if (ws == 8) MDFF_LAUNCH(e, (k_ion64<KS, WF, 1, 8>), grid, 256, 0, a);
+    else if (mt == 4) MDFF_LAUNCH(e, (k_ion64<KS, WF, M4, 1>), grid, 32 * I64_WARPS, 0, a);
+    else MDFF_LAUNCH(e, (k_ion64<KS, WF, 2, 1>), grid, 32 * I64_WARPS, 0, a);
 }
 
 template <int KS>
-static void ion64_ks(Engine &e, const Ion64Args &a, dim3 grid, int mt, bool wf) {
-    if (wf) ion64_mt<KS, true>(e, a, grid, mt);
-    else ion64_mt<KS, false>(e, a, grid, mt);
+static void ion64_ks(Engine &e, const Ion64Args &a, dim3 grid, int mt, int ws, bool wf) {
+    if (wf) ion64_mt<KS, true>(e, a, grid, mt, ws);
+    else ion64_mt<KS, false>(e, a, grid, mt, ws);
 }
 
 template <class F>
@@ -745,27 +806,33 @@ void launch_rec64(Engine &e, const double *q, const double3 *mu, bool lq, bool l
     a.qself = o.self_q;
     a.muself = o.self_mu;
     a.cg = o.cg;
-    // tiles of 8 ions per warp and slices of the rows: whole waves of the SMs first, then the
-    // most reuse of each weight (a warp with 4 tiles loads a quarter of what 4 warps do)
-    int mt = 1;
+    // tiles of 8 ions per warp, row slices within the block (ws) and of the grid: time in units
+    // of one (row group, tile) per scheduler, plus the start of the block (8 units) and, with
+    // slices in memory, the arrival and second read (16); several tiles per warp share each
+    // weight load
+    int mt = 1, ws = 8;
     a.slices = 1;
     double best = 1e300;
-    for (int m = 1; m <= (wf ? 2 : 4); m *= 2) {
-        const int blocks = ceil_div(std::max(out_n, 1), 8 * m * I64_WARPS);
-        const double unit = m * (m == 1 ? 1.15 : (m == 2 ? 1.05 : 1.0));
-        for (int s = 1; s <= e.ion64_slices_max; s++) {
-            const double cost = ceil_div(blocks * s, e.nsm) * (ceil_div(a.units, s) * unit + 1.5);
-            if (cost < best) {
-                best = cost;
-                mt = m;
-                a.slices = s;
+    for (int w = 1; w <= 8; w += 7)
+        for (int m = w == 8 ? 1 : 2; m <= ((w == 8 || wf) ? 2 : 4); m *= 2) {
+            const int blocks = ceil_div(std::max(out_n, 1), w == 8 ? 8 * m : 8 * m * I64_WARPS);
+            const double unit = m * (m == 1 ? 1.3 : (m == 2 ? 1.1 : 1.0)) * (w == 8 ? 2.0 : 1.0);
+            for (int s = 1; s <= e.ion64_slices_max && s * w <= std::max(a.units, 8); s++) {
+                const double cost =
+                    ceil_div(blocks * s, e.nsm) * ceil_div(a.units, s * w) * unit + 8.0 + (s > 1 ? 16.0 : 0.0);
+                if (cost < best) {
+                    best = cost;
+                    mt = m;
+                    ws = w;
+                    a.slices = s;
+                }
             }
         }
-    }
-    const dim3 grid(ceil_div(std::max(out_n, 1), 8 * mt * I64_WARPS), a.slices);
+    const int per_block = ws == 8 ? 8 * mt : 8 * mt * I64_WARPS;
+    const dim3 grid(ceil_div(std::max(out_n, 1), per_block), a.slices);
     int pi = -1;
     e.prof_begin("k_rec_ion", &pi);
-    by_ksteps(ksteps64(e), [&](auto k) { ion64_ks<decltype(k)::value>(e, a, grid, mt, wf); });
+    by_ksteps(ksteps64(e), [&](auto k) { ion64_ks<decltype(k)::value>(e, a, grid, mt, ws, wf); });
     e.prof_end("k_rec_ion", pi, ion_flops_per_pair(wf) * (double)out_n * e.nk);
 }
 
