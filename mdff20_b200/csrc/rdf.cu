@@ -11,70 +11,189 @@
 // both ways round (negation is exact through every step), so each unordered pair is
 // evaluated once and counted for both orders.
 //
-// Layout: one block per (i tile, j tile) of the upper triangle of the pair matrix,
-// GR_TILE ions a side; the j tile is staged in shared memory, each thread runs one i
-// against it, and the counts go to a block-private shared histogram that is added to
-// the global 64-bit histogram once at the end (global atomics directly when the
-// histogram does not fit in shared memory).
+// What bounds it: instructions per pair (n^2 / 2 of them; half the pairs lie inside half the
+// box width).  The exact distance, square root and division in FP64 are about 100 issue slots;
+// only whether a pair is in range and its bin matter, so both are decided in FP32 where that is
+// certain, and by the FP64 operations where the distance is within its error of a bin edge or of
+// the cut-off (0.02% of the pairs at bins of 0.1 A and 35 A).  Coordinates are 32-bit fixed-point
+// fractions, whose differences wrap to the minimum image by themselves and keep the relative
+// error of the components; the error bound is GrErr's.  24000 ions, 351 bins: 965 -> 494 us a
+// configuration (46 issue slots per 32 pairs, 0.82 issued per cycle).
+//
+// Layout: persistent blocks over (i tile, j tile) pairs of the upper triangle, the j tile in
+// shared memory, one or two i per thread; each pair is counted once, under (type i, type j), in
+// a block-private shared histogram, and added to both orders of the global 64-bit histogram when
+// the block ends (global atomics directly when the histogram does not fit in shared memory).
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "engine.cuh"
 
 namespace mdffgpu {
 
-constexpr int GR_TILE = 128;
-constexpr int GR_SMEM_COUNTERS = 10240;   // 40 KB of 32-bit block counters (+ 4.5 KB of tile)
+constexpr int GR_THREADS = 256;
+constexpr int GR_JT = 256;                // most ions of a j tile
+constexpr int GR_SMEM_COUNTERS = 10240;   // 40 KB of 32-bit block counters (+ 4 KB of tile)
 
-__global__ void k_kardir(int n, Cell c, const double4 *r, double4 *s);
-
-__global__ void __launch_bounds__(GR_TILE)
-    k_gr_pairs(int n, Cell c, const double4 *__restrict__ s, const int *__restrict__ typ, int nt, int nbins,
-               double cut2, double resg, unsigned long long *__restrict__ hist, int private_hist) {
+// positions (one array per component, or null: r) -> exact fractions s, fixed-point fractions
+// with the type; *bad is set when a coordinate is not finite or so far out that its fraction
+// loses digits (every pair is then decided in FP64)
+__global__ void __launch_bounds__(256) k_gr_pack(int n, Cell c, const double *__restrict__ soa,
+                                                 const double4 *__restrict__ r, const int *__restrict__ typ,
+                                                 double4 *__restrict__ s, int4 *__restrict__ fx, int *bad) {
     grid_dep();
-    extern __shared__ unsigned int h_sh[];
-    __shared__ double4 tile[GR_TILE];
-    __shared__ int ttile[GR_TILE];
-    int bi = blockIdx.y, bj = blockIdx.x;
-    if (bj < bi) return;
-    int nh = nbins * nt * nt;
-    if (private_hist)
-        for (int k = threadIdx.x; k < nh; k += blockDim.x) h_sh[k] = 0u;
-    int j0 = bj * GR_TILE;
-    int jend = min(GR_TILE, n - j0);
-    if (threadIdx.x < jend) {
-        tile[threadIdx.x] = s[j0 + threadIdx.x];
-        ttile[threadIdx.x] = typ[j0 + threadIdx.x];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double x, y, z;
+    if (soa) {
+        x = soa[i], y = soa[n + i], z = soa[2 * (size_t)n + i];
+    } else {
+        const double4 q = r[i];
+        x = q.x, y = q.y, z = q.z;
     }
-    __syncthreads();
-    int i = bi * GR_TILE + threadIdx.x;
-    if (i < n) {
-        double4 si = s[i];
-        int ti = typ[i];
-        for (int jj = (bi == bj) ? threadIdx.x + 1 : 0; jj < jend; jj++) {
-            double4 sj = tile[jj];
-            double3 d = pbc_frac(c, dsub(si.x, sj.x), dsub(si.y, sj.y), dsub(si.z, sj.z));
-            double r2 = norm2_exact(d);
-            if (!(r2 < cut2)) continue;
-            int b = (int)__ddiv_rn(sqrt(r2), resg);
-            if (b < 0 || b >= nbins) continue;   // cannot happen for nbins > cutgr / resg
-            int tj = ttile[jj];
-            int k1 = (b * nt + ti) * nt + tj, k2 = (b * nt + tj) * nt + ti;
-            if (private_hist) {
-                atomicAdd(&h_sh[k1], 1u);
-                atomicAdd(&h_sh[k2], 1u);
-            } else {
-                atomicAdd(&hist[k1], 1ull);
-                atomicAdd(&hist[k2], 1ull);
+    const double3 f = kardir(c, x, y, z);
+    s[i] = make_double4(f.x, f.y, f.z, 0.0);
+    if (!(fabs(f.x) < 1e6 && fabs(f.y) < 1e6 && fabs(f.z) < 1e6)) *bad = 1;
+    auto fix = [](double u) { return (int)(unsigned)__double2ll_rn((u - rint(u)) * 4294967296.0); };
+    fx[i] = make_int4(fix(f.x), fix(f.y), fix(f.z), typ[i]);
+}
+
+// FP32 decision: a[k] lattice entries x 2^-32 (row-major), bin coordinate r / resg known to
+// within e1 (r / resg) + e0, in range below lo2 and out of range above hi2
+struct GrErr {
+    float a[9], inv, e1, e0, lo2, hi2;
+};
+struct GrArgs {
+    int n, nt, nbins, jt, priv;
+    Cell c;
+    GrErr w;
+    const double4 *s;
+    const int4 *fx;
+    double cut2, resg;
+    unsigned long long *hist;
+    const int *bad;
+};
+
+// the reference's bin of a pair, or -1 (outside)
+__device__ __noinline__ int gr_exact(const GrArgs &a, int i, int j) {
+    const double4 si = a.s[i], sj = a.s[j];
+    const double3 d = pbc_frac(a.c, dsub(si.x, sj.x), dsub(si.y, sj.y), dsub(si.z, sj.z));
+    const double r2 = norm2_exact(d);
+    if (!(r2 < a.cut2)) return -1;
+    const int b = (int)__ddiv_rn(sqrt(r2), a.resg);
+    return b < 0 || b >= a.nbins ? -1 : b;   // never past the end for nbins > cutgr / resg
+}
+
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+template <int IPT, bool ORTHO, bool PRIV>
+__global__ void __launch_bounds__(GR_THREADS) k_gr_pairs(const __grid_constant__ GrArgs a) {
+    grid_dep();
+    extern __shared__ unsigned h_sh[];
+    __shared__ int4 tile[GR_JT];
+    const int np = a.nt * a.nt, nh = a.nbins * np;
+    if (PRIV)
+        for (int k = threadIdx.x; k < nh; k += GR_THREADS) h_sh[k] = 0u;
+    const int nbi = (a.n + GR_THREADS * IPT - 1) / (GR_THREADS * IPT), nbj = (a.n + a.jt - 1) / a.jt;
+    GrErr w = a.w;
+    if (*a.bad != 0) w.hi2 = __int_as_float(0x7f800000), w.e0 = 1.0f;   // every pair in FP64
+    const float thr0 = 0.5f - w.e0 - 0.5f * w.e1;
+    // the certain counts of one block stay below 2^31 up to about 10^6 ions; past that they are
+    // added to the global histogram on the way
+    long long seen = 0;
+    auto flush = [&] {
+        __syncthreads();
+        for (int k = threadIdx.x; k < nh; k += GR_THREADS) {
+            const unsigned c = h_sh[k];
+            if (!c) continue;
+            const int b = k / np, q = k - b * np, ti = q / a.nt, tj = q - ti * a.nt;
+            atomicAdd(&a.hist[k], (unsigned long long)c);
+            atomicAdd(&a.hist[b * np + tj * a.nt + ti], (unsigned long long)c);
+            h_sh[k] = 0u;
+        }
+        __syncthreads();
+    };
+    for (long long t = blockIdx.x; t < (long long)nbi * nbj; t += gridDim.x) {
+        const int bi = (int)(t / nbj), bj = (int)(t - (long long)bi * nbj);
+        const int i0 = bi * GR_THREADS * IPT, j0 = bj * a.jt, jn = min(a.jt, a.n - j0);
+        if (j0 + jn - 1 <= i0) continue;   // no j > i here
+        __syncthreads();
+        for (int k = threadIdx.x; k < jn; k += GR_THREADS) tile[k] = a.fx[j0 + k];
+        __syncthreads();
+        int4 me[IPT];
+        int lo[IPT];   // first j of the tile past i
+#pragma unroll
+        for (int m = 0; m < IPT; m++) {
+            const int i = i0 + m * GR_THREADS + threadIdx.x;
+            me[m] = a.fx[min(i, a.n - 1)];
+            me[m].w *= a.nt;
+            lo[m] = i < a.n ? max(0, i + 1 - j0) : jn;
+        }
+        // straight-line per pair; the one branch is the FP64 decision of the warp's open pairs
+        auto scan = [&](auto diag) {
+            constexpr bool DIAG = decltype(diag)::value;   // tiles that hold pairs with j <= i, or i >= n
+#pragma unroll 2
+            for (int jj = 0; jj < jn; jj++) {
+                const int4 o = tile[jj];
+#pragma unroll
+                for (int m = 0; m < IPT; m++) {
+                    const int dx = me[m].x - o.x, dy = me[m].y - o.y, dz = me[m].z - o.z;
+                    const float u = (float)dx, v = (float)dy, q = (float)dz;
+                    float x, y, z;
+                    bool edge = false;
+                    if (ORTHO) {
+                        x = u * w.a[0], y = v * w.a[4], z = q * w.a[8];
+                    } else {
+                        x = u * w.a[0] + v * w.a[3] + q * w.a[6];
+                        y = u * w.a[1] + v * w.a[4] + q * w.a[7];
+                        z = u * w.a[2] + v * w.a[5] + q * w.a[8];
+                        // next to a half box edge the two images differ in a triclinic cell
+                        edge = fmaxf(fabsf(u), fmaxf(fabsf(v), fabsf(q))) > 2147483000.0f;
+                    }
+                    const float r2 = x * x + y * y + z * z;
+                    bool in = r2 < w.hi2 || edge;
+                    if (DIAG) in = in && jj >= lo[m];
+                    // floor by rounding x - 1/2; its distance to the halfway points is the
+                    // distance to the bin edges (a NaN or a bin past 2^22 fails the test)
+                    const float h = r2 * rsqrt_approx(r2) * w.inv - 0.5f;
+                    const float y0 = h + 12582912.0f, fr = h - (y0 - 12582912.0f);
+                    int b = __float_as_int(y0) - 0x4b400000;
+                    const bool sure = fabsf(fr) < thr0 - w.e1 * h && r2 < w.lo2 && !edge;
+                    if (__any_sync(0xffffffffu, in && !sure)) {
+                        if (in && !sure) {
+                            b = gr_exact(a, i0 + m * GR_THREADS + threadIdx.x, j0 + jj);
+                            in = b >= 0;
+                        }
+                    }
+                    const int k = b * np + me[m].w + o.w;
+                    if (in) {
+                        if (PRIV) {
+                            atomicAdd(&h_sh[k], 1u);
+                        } else {
+                            atomicAdd(&a.hist[k], 1ull);
+                            atomicAdd(&a.hist[b * np + o.w * a.nt + me[m].w / a.nt], 1ull);
+                        }
+                    }
+                }
             }
+        };
+        if (j0 < i0 + GR_THREADS * IPT) scan(std::true_type());
+        else scan(std::false_type());
+        seen += (long long)GR_THREADS * IPT * jn;
+        if (PRIV && seen > (1ll << 30)) {
+            flush();
+            seen = 0;
         }
     }
-    if (!private_hist) return;
-    __syncthreads();
-    for (int k = threadIdx.x; k < nh; k += blockDim.x)
-        if (h_sh[k]) atomicAdd(&hist[k], (unsigned long long)h_sh[k]);
+    if (PRIV) flush();
 }
 
 // lattice (src/cell.c:13-91) as far as kardir and pbc need it: A, B = (A_j x A_k) / omega
@@ -109,10 +228,12 @@ struct mdffgpu_rdf {
     int n = 0, nt = 0, nbins = 0, device = 0, nconf = 0;
     double cut2 = 0.0, resg = 0.0;
     cudaStream_t stream = nullptr;
-    double4 *d_r = nullptr, *d_s = nullptr;
-    int *d_typ = nullptr;
+    double *d_soa = nullptr;      // positions of the configuration, one array per component
+    double4 *d_s = nullptr;
+    int4 *d_fx = nullptr;
+    int *d_typ = nullptr, *d_bad = nullptr;
     unsigned long long *d_hist = nullptr;
-    double4 *h_r = nullptr;   // pinned staging
+    double *h_soa = nullptr;      // pinned staging
     long long launches = 0;
     std::string err;
 };
@@ -135,16 +256,70 @@ int rdf_guarded(mdffgpu_rdf *r, F &&f) {
     }
 }
 
-void launch_gr(mdffgpu_rdf &r, const mdffgpu::Cell &c, const double4 *d_s, const int *d_typ, cudaStream_t st) {
-    int nb = mdffgpu::ceil_div(r.n, mdffgpu::GR_TILE);
-    int nh = r.nbins * r.nt * r.nt;
-    int priv = nh <= mdffgpu::GR_SMEM_COUNTERS ? 1 : 0;
-    size_t smem = priv ? sizeof(unsigned int) * nh : 0;
-    dim3 grid(nb, nb);
-    mdffgpu::k_gr_pairs<<<grid, mdffgpu::GR_TILE, smem, st>>>(r.n, c, d_s, d_typ, r.nt, r.nbins, r.cut2, r.resg,
-                                                              r.d_hist, priv);
+// one configuration: soa, or the positions of a context
+void launch_gr(mdffgpu_rdf &r, const mdffgpu::Cell &c, const double *soa, const double4 *d_r, const int *d_typ,
+               cudaStream_t st) {
+    using namespace mdffgpu;
+    MDFF_CK(cudaMemsetAsync(r.d_bad, 0, sizeof(int), st));
+    k_gr_pack<<<ceil_div(r.n, 256), 256, 0, st>>>(r.n, c, soa, d_r, d_typ, r.d_s, r.d_fx, r.d_bad);
     MDFF_CK(cudaGetLastError());
-    r.launches++;
+    GrArgs a;
+    a.n = r.n;
+    a.nt = r.nt;
+    a.nbins = r.nbins;
+    a.c = c;
+    a.s = r.d_s;
+    a.fx = r.d_fx;
+    a.cut2 = r.cut2;
+    a.resg = r.resg;
+    a.hist = r.d_hist;
+    a.bad = r.d_bad;
+    const int nh = r.nbins * r.nt * r.nt;
+    a.priv = nh <= GR_SMEM_COUNTERS ? 1 : 0;
+    const size_t smem = a.priv ? sizeof(unsigned) * nh : 0;
+    // Error of the FP32 distance.  Each component: conversion of the fixed-point difference,
+    // lattice entry and product, 3 x 2^-24 relative of its terms; squares, sum and root of r^2
+    // half of 3 x 2^-24 more, the reciprocal root 2^-22, two products and 1 / resg 3 x 2^-24:
+    // below 7e-7 of r in an orthorhombic cell (e1 takes 1.2e-6).  In a triclinic one the terms
+    // cancel, which leaves 2e-7 of the lattice entries (e0 takes 1e-6 of their sum).  The
+    // fixed-point rounding is 2^-32 of a lattice entry per component (2e-9 taken).
+    double sum = 0.0;
+    bool ortho = true;
+    for (int k = 0; k < 9; k++) {
+        const double v = c.A[k / 3][k % 3];
+        sum += std::fabs(v);
+        if (k / 3 != k % 3 && v != 0.0) ortho = false;
+        a.w.a[k] = (float)(v / 4294967296.0);
+    }
+    const double abs_err = (ortho ? 2e-9 : 1e-6) * sum;
+    const double cut = std::min(std::sqrt(r.cut2), r.nbins * r.resg);   // certain pairs have a bin
+    a.w.inv = (float)(1.0 / r.resg);
+    a.w.e1 = 1.2e-6f;
+    a.w.e0 = (float)(abs_err / r.resg + 1e-7);
+    const double m = 1.2e-6 * cut + abs_err, l = std::max(0.0, cut - m), h = std::sqrt(r.cut2) * (1.0 + 1.2e-6) + abs_err;
+    a.w.lo2 = (float)(l * l * (1.0 - 2e-6));
+    a.w.hi2 = (float)(h * h * (1.0 + 2e-6));
+    int nsm = 148;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, r.device);
+    // two i per thread once that leaves several tile pairs per block; j tiles short enough for
+    // the same (a block's start and its flush cost about as much as 20000 pairs)
+    const int ipt = r.n >= 12288 ? 2 : 1, blocks = 4 * nsm;
+    a.jt = GR_JT;
+    while (a.jt > 32 && (long long)ceil_div(r.n, GR_THREADS * ipt) * ceil_div(r.n, a.jt) < 8ll * blocks) a.jt /= 2;
+    const long long tiles = (long long)ceil_div(r.n, GR_THREADS * ipt) * ceil_div(r.n, a.jt);
+    const int grid = (int)std::min<long long>(blocks, tiles);
+    auto go = [&](auto kernel) { kernel<<<grid, GR_THREADS, smem, st>>>(a); };
+    auto by_cell = [&](auto two, auto priv) {
+        constexpr int I = decltype(two)::value ? 2 : 1;
+        if (ortho) go(k_gr_pairs<I, true, decltype(priv)::value>);
+        else go(k_gr_pairs<I, false, decltype(priv)::value>);
+    };
+    if (ipt == 2 && a.priv) by_cell(std::true_type(), std::true_type());
+    else if (ipt == 2) by_cell(std::true_type(), std::false_type());
+    else if (a.priv) by_cell(std::false_type(), std::true_type());
+    else by_cell(std::false_type(), std::false_type());
+    MDFF_CK(cudaGetLastError());
+    r.launches += 2;
 }
 
 }  // namespace
@@ -172,11 +347,13 @@ int mdffgpu_rdf_create(int nion, int ntype, const int *nionit, double cutgr, dou
     r->resg = resg;
     int rc = rdf_guarded(r, [&](mdffgpu_rdf &x) {
         MDFF_CK(cudaStreamCreateWithFlags(&x.stream, cudaStreamNonBlocking));
-        x.d_r = mdffgpu::dalloc<double4>(nion);
+        x.d_soa = mdffgpu::dalloc<double>(3 * (size_t)nion);
         x.d_s = mdffgpu::dalloc<double4>(nion);
+        x.d_fx = mdffgpu::dalloc<int4>(nion);
+        x.d_bad = mdffgpu::dalloc<int>(1);
         x.d_typ = mdffgpu::dalloc<int>(nion);
         x.d_hist = mdffgpu::dalloc<unsigned long long>((size_t)nbins * ntype * ntype);
-        MDFF_CK(cudaMallocHost((void **)&x.h_r, sizeof(double4) * nion));
+        MDFF_CK(cudaMallocHost((void **)&x.h_soa, 3 * sizeof(double) * nion));
         std::vector<int> typ(nion);
         for (int t = 0, ia = 0; t < ntype; t++)
             for (int k = 0; k < nionit[t]; k++) typ[ia++] = t;
@@ -193,11 +370,13 @@ int mdffgpu_rdf_create(int nion, int ntype, const int *nionit, double cutgr, dou
 int mdffgpu_rdf_destroy(mdffgpu_rdf *r) {
     if (!r) return MDFFGPU_ERR_ARG;
     cudaSetDevice(r->device);
-    cudaFree(r->d_r);
+    cudaFree(r->d_soa);
     cudaFree(r->d_s);
+    cudaFree(r->d_fx);
+    cudaFree(r->d_bad);
     cudaFree(r->d_typ);
     cudaFree(r->d_hist);
-    if (r->h_r) cudaFreeHost(r->h_r);
+    if (r->h_soa) cudaFreeHost(r->h_soa);
     if (r->stream) cudaStreamDestroy(r->stream);
     delete r;
     return MDFFGPU_OK;
@@ -217,12 +396,12 @@ int mdffgpu_rdf_add(mdffgpu_rdf *r, const double *cell, const double *rx, const 
     if (!cell || !rx || !ry || !rz) return MDFFGPU_ERR_ARG;
     return rdf_guarded(r, [&](mdffgpu_rdf &x) {
         mdffgpu::Cell c = mdffgpu::cell_of(cell);
-        for (int i = 0; i < x.n; i++) x.h_r[i] = make_double4(rx[i], ry[i], rz[i], 0.0);
-        MDFF_CK(cudaMemcpyAsync(x.d_r, x.h_r, sizeof(double4) * x.n, cudaMemcpyHostToDevice, x.stream));
-        mdffgpu::k_kardir<<<mdffgpu::ceil_div(x.n, 256), 256, 0, x.stream>>>(x.n, c, x.d_r, x.d_s);
-        MDFF_CK(cudaGetLastError());
-        x.launches++;
-        launch_gr(x, c, x.d_s, x.d_typ, x.stream);
+        const size_t b = sizeof(double) * x.n;
+        memcpy(x.h_soa, rx, b);
+        memcpy(x.h_soa + x.n, ry, b);
+        memcpy(x.h_soa + 2 * (size_t)x.n, rz, b);
+        MDFF_CK(cudaMemcpyAsync(x.d_soa, x.h_soa, 3 * b, cudaMemcpyHostToDevice, x.stream));
+        launch_gr(x, c, x.d_soa, nullptr, x.d_typ, x.stream);
         MDFF_CK(cudaStreamSynchronize(x.stream));
         x.nconf++;
     });
@@ -235,10 +414,7 @@ int mdffgpu_rdf_add_ctx(mdffgpu_rdf *r, mdffgpu_ctx *ctx) {
         if (e->n != x.n || e->nt != x.nt || e->device != x.device)
             throw Error(MDFFGPU_ERR_ARG, "rdf_add_ctx: the context holds another system or device");
         // the context's positions and types, on its stream (one less host round trip)
-        mdffgpu::k_kardir<<<mdffgpu::ceil_div(x.n, 256), 256, 0, e->stream>>>(x.n, e->cell, e->d_r, x.d_s);
-        MDFF_CK(cudaGetLastError());
-        x.launches++;
-        launch_gr(x, e->cell, x.d_s, e->d_typ, e->stream);
+        launch_gr(x, e->cell, nullptr, e->d_r, e->d_typ, e->stream);
         MDFF_CK(cudaStreamSynchronize(e->stream));
         x.nconf++;
     });
