@@ -298,7 +298,7 @@ static int sr_call(mdffgpu_ctx *ctx, bool lj, double *u, double *pvir, double *t
         if (!lj && !(e.p.lbhmft || e.p.lbhmftd)) throw Error(MDFFGPU_ERR_STATE, "lbhmft/lbhmftd is not set");
         e.ensure_lists();
         mdffgpu::launch_kardir(e, e.d_r, e.d_s);
-        e.sr_forces(lj, nullptr, nullptr, nullptr);
+        mdffgpu::launch_sr(e, lj);
         e.sync_scalars();
         const mdffgpu::DevScalars &o = *e.h_out;
         if (u) *u = lj ? o.u_lj : o.u_bh;

@@ -122,6 +122,21 @@ __device__ __forceinline__ void block_sum_to_part(double (&v)[NV], double *part,
     }
 }
 
+// A block's arrival, after its threads' global writes; true in the last block of the grid, which
+// then sees every block's writes (and has reset the ticket)
+__device__ __forceinline__ bool last_block(unsigned *ticket) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        if (last) *ticket = 0u;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
 // The last block of a kernel to finish reduces the partials of slots first..first+nslots-1
 // exactly as k_reduce_slots does (same order), so the separate reduction launch is not
 // needed; ticket (zero between calls) counts the finished blocks.  The writers of the
@@ -154,28 +169,25 @@ __device__ __forceinline__ bool last_block_slots(const double *part, int stride,
     return true;
 }
 
-// The same with one warp per slot (nslots <= warps of the block, slots[k] the slot of warp k):
+// The same with one warp per slot:
 // a last block of eight warps sums seven slots of 3000 partials in 4 us instead of 12.
-__device__ __forceinline__ bool last_block_warps(const double *part, int stride, const int *slots, int nslots,
-                                                 double *scal, unsigned *ticket) {
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (w < nslots) {
+__device__ __forceinline__ void sum_slots(const double *part, int stride, const int *slots, int nslots, int nparts,
+                                          double *scal) {
+    const int l = threadIdx.x & 31, nw = (int)blockDim.x >> 5;
+    for (int w = threadIdx.x >> 5; w < nslots; w += nw) {
         const double *p = part + (size_t)slots[w] * stride;
         double a = 0.0;
 #pragma unroll 8
-        for (int k = l; k < (int)gridDim.x; k += 32) a += __ldcg(p + k);
+        for (int k = l; k < nparts; k += 32) a += __ldcg(p + k);
         a = warp_sum(a);
         if (l == 0) scal[slots[w]] = a;
     }
     __syncthreads();
-    if (threadIdx.x == 0) *ticket = 0u;
+}
+__device__ __forceinline__ bool last_block_warps(const double *part, int stride, const int *slots, int nslots,
+                                                 double *scal, unsigned *ticket) {
+    if (!last_block(ticket)) return false;
+    sum_slots(part, stride, slots, nslots, (int)gridDim.x, scal);
     return true;
 }
 

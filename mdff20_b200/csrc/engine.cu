@@ -19,13 +19,7 @@ __global__ void k_self_sums(int n, const double *q, const double3 *mu, double *p
 __global__ void k_self_plus_dir(int n, double self2, const double3 *mu, const double3 *efd, double3 *ef);
 __global__ void k_axpy3(int n, double a, const double3 *x, double3 *y);
 __global__ void k_efg_self_dir(int n, double self2, const double *q, const double *efgd, double *efg);
-__global__ void k_finalize_sr(const double *scal, int slot, double inveOmegaPU, double *u, double *pvir,
-                              double *tau);
-struct CoulFin {
-    double alpha, coul, inveOmegaPU, ttpiV;
-    int do_dir, do_rec, do_stress;
-};
-__global__ void k_finalize_coul(const double *scal, CoulFin c, double *u, double *pvir, double *tau);
+__global__ void k_finalize_coul(CoulFin c);
 __global__ void k_induced(int n, const int *polar, const double *pol, const double3 *ef, double3 *mu);
 __global__ void k_aspc_predict(int n, AspcCoef cf, int es, double *hist, double3 *mu);
 __global__ void k_aspc_correct(int n, double W, const int *polar, const double *pol, const double3 *ef,
@@ -48,21 +42,8 @@ __global__ void k_cg_step(int n, int nk, const int *polar, const double *pol, do
                           const double3 *ap, double3 *x, double3 *r, double3 *z, const double2 *rho_p, double2 *acc,
                           double *part, int stride, unsigned *ticket, CgTest test);
 __global__ void k_cg_test(CgTest t, const double *scal);
-__global__ void k_vv1(int n, double dt, double dtsq2, const double *invm, double4 *r, const double3 *v,
-                      const double3 *f, double3 *fs);
-__global__ void k_vv2(int n, double dt2, const double *invm, const double *mass, double3 *v, const double3 *f,
-                      const double3 *fs, double *part, int stride);
-__global__ void k_pv1(int n, double dt, double dt2, const double *invm, double4 *r, double3 *v, const double3 *f);
-__global__ void k_pv2(int n, double dt2, const double *invm, const double *mass, double3 *v, const double3 *f,
-                      double *part, int stride, double *scal, unsigned *ticket, const double4 *r, unsigned *status);
-__global__ void k_scale_kin(ScaleKinArgs a);
 __global__ void k_lf(int n, double dtsq, double idt, const double *invm, const double *mass, double4 *r,
                      double3 *rs, double3 *v, const double3 *f, double *part, int stride);
-struct NhcArgs {
-    int nn, yo, mults;
-    double dt, temp, L, w[7];
-};
-void launch_nhc_chain(Engine &e, const NhcArgs &a, double *nhc, const double *scal, DevScalars *out);
 __global__ void k_set_ekin(const double *scal, DevScalars *out);
 __global__ void k_check_finite(int n, const double4 *r, const double3 *f, unsigned *status);
 __global__ void k_sort_cells(int ncell, int cell_cap, const int *start, const int *cnt, int *ions, const double4 *s,
@@ -152,10 +133,10 @@ Engine::Engine(const mdffgpu_params &prm, int dev) : p(prm) {
     d_muzero = dalloc<double3>(n);
     d_svl = dalloc<double4>(n);
     d_rebuild = dalloc<int>(1);
-    d_status = dalloc<unsigned>(1);
     d_ticket = dalloc<unsigned>(16);
     d_scal = dalloc<double>(NSLOT);
     d_out = dalloc<DevScalars>(1);
+    d_status = (unsigned *)&d_out->status;   // one copy brings both to the host
     d_nhc = dalloc<double>(48);
     MDFF_CK(cudaMallocHost((void **)&h_out, sizeof(DevScalars)));
     d_soa = dalloc<double>(9 * (size_t)n);
@@ -230,7 +211,6 @@ Engine::~Engine() {
                     (void *)d_ft, (void *)d_theta, (void *)d_fres})
         cudaFree(x);
     cudaFree(d_out);
-    cudaFree(d_status);
     cudaFree(d_ticket);
     if (h_out) cudaFreeHost(h_out);
     cudaFree(d_soa);
@@ -631,7 +611,6 @@ void Engine::get_state(double *rx, double *ry, double *rz, double *vx, double *v
 
 void Engine::sync_scalars() {
     MDFF_CK(cudaMemcpyAsync(h_out, d_out, sizeof(DevScalars), cudaMemcpyDeviceToHost, stream));
-    MDFF_CK(cudaMemcpyAsync(&h_out->status, d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
     MDFF_CK(cudaStreamSynchronize(stream));
 }
 
@@ -674,13 +653,11 @@ int Engine::check_verletlist(bool reset_status) {
         return 1;
     }
     if (reset_status) MDFF_CK(cudaMemsetAsync(d_status, 0, sizeof(unsigned), stream));
-    if (capturing) {
-        // the rebuild as an IF node: on the steps without one its kernels do not launch
-        record_if([&](cudaGraphConditionalHandle h) { launch_check_list(*this, &h); },
-                  [&] { launch_build_lists(*this, false); });
-        return 0;   // the host reads the rebuild flag and status after the step
-    }
     launch_check_list(*this);
+    return rebuild_if_due();
+}
+
+int Engine::rebuild_if_due() {
     launch_build_lists(*this, false);
     int rb = 0;
     unsigned st = 0;
@@ -704,24 +681,6 @@ void Engine::ensure_lists() {
 }
 
 // ---------------------------------------------------------------- force evaluation
-void Engine::sr_forces(bool lj, double *u, double *pvir, double *tau) {
-    launch_sr(*this, lj);
-    sr_finish(lj);
-    (void)u;
-    (void)pvir;
-    (void)tau;
-}
-
-void Engine::sr_finish(bool lj) {
-    int slot = lj ? S_LJ_U : S_BH_U;
-    reduce(slot, 7, ceil_div(n, 8));
-    DevScalars *o = d_out;
-    if (lj)
-        MDFF_LAUNCH(*this, k_finalize_sr, 1, 1, 0, d_scal, slot, cell.inveOmegaPU, &o->u_lj, &o->pvir_lj, o->tau_lj);
-    else
-        MDFF_LAUNCH(*this, k_finalize_sr, 1, 1, 0, d_scal, slot, cell.inveOmegaPU, &o->u_bh, &o->pvir_bh, o->tau_bh);
-}
-
 static double self2_of(double alpha) {
     const double rpi = 1.7724538509055160273;
     double selfa = alpha / rpi, selfa2 = 2.0 * selfa * alpha * alpha / 3.0;
@@ -737,9 +696,10 @@ void Engine::field_of(const double *d_qv, const double3 *d_muv, bool lq, bool ld
         if (use32 && real32) launch_pol_field32(*this, d_muv, d_tmp3);
         else launch_dir_field_cached(*this, d_muv, d_tmp3);
     } else if (use32 && real32) {
-        launch_dir32(*this, d_qv, d_muv, p.alphaES, lq, ld, damp, false, true, d_tmp3, nullptr);
+        launch_dir32(*this, d_qv, d_muv, p.alphaES, lq, ld, damp, false, true, d_tmp3, nullptr, false);
     } else {
-        launch_dir(*this, d_qv, d_muv, p.alphaES, lq, ld, damp, false, true, false, false, d_tmp3, nullptr, nullptr);
+        launch_dir(*this, d_qv, d_muv, p.alphaES, lq, ld, damp, false, true, false, false, d_tmp3, nullptr, nullptr,
+                   false);
     }
     RecOut o;
     o.ef = d_ef_out;
@@ -1017,10 +977,10 @@ void Engine::pim_cg(bool fused) {
         on_side(SIDE_PREP, [&] {
             if (use32 && real32)
                 launch_dir32(*this, d_q, d_mu_tot, p.alphaES, lqch != 0, true, ldmp != 0, false, true, d_tmp3,
-                             nullptr, sub ? d_pidx : nullptr, npol);
+                             nullptr, false, sub ? d_pidx : nullptr, npol);
             else
                 launch_dir(*this, d_q, d_mu_tot, p.alphaES, lqch != 0, true, ldmp != 0, false, true, false, false,
-                           d_tmp3, nullptr, nullptr);
+                           d_tmp3, nullptr, nullptr, false);
         });
         RecOut o;
         o.ef = d_ef_ind;
@@ -1231,31 +1191,38 @@ void Engine::get_dipoles() {
     launch_pim_finish(*this, cont);
 }
 
-void Engine::finalize_coul(bool stress) {
+CoulFin Engine::coul_fin(double alpha, bool dir, bool rec, bool stress) {
     CoulFin cf;
-    cf.alpha = p.alphaES;
+    cf.on = 1;
+    cf.alpha = alpha;
     cf.coul = coul_unit;
     cf.inveOmegaPU = cell.inveOmegaPU;
     cf.ttpiV = 2.0 * TPI_D * cell.inveOmega;
-    cf.do_dir = 1;
-    cf.do_rec = 1;
+    cf.do_dir = dir;
+    cf.do_rec = rec;
     cf.do_stress = stress;
-    MDFF_LAUNCH(*this, k_finalize_coul, 1, 1, 0, d_scal, cf, &d_out->u_coul, &d_out->pvir_coul, d_out->tau_coul);
+    cf.scal = d_scal;
+    cf.u = &d_out->u_coul;
+    cf.pvir = &d_out->pvir_coul;
+    cf.tau = d_out->tau_coul;
+    return cf;
 }
 
 // engforce, src/field.c:352-407
-void Engine::engforce(bool check_finite) {
+void Engine::engforce(bool check_finite, bool opened) {
     ensure_lists();
-    MDFF_CK(cudaMemsetAsync(d_f, 0, sizeof(double3) * n, stream));
-    launch_kardir(*this, d_r, d_s);
+    if (!opened || !p.lverletL) launch_kardir(*this, d_r, d_s, d_f);   // (a list build at each call moves d_s)
     // side branches from here (they read the fractional coordinates): the short-range
-    // pairs, which add into d_f (joined before the k-space force combine reads it), and
+    // pairs, which add into d_f (joined before the k-space force pass reads it), and
     // in mixed precision the in-cutoff lists (joined before the dipole solve)
-    if (p.lnmlj || p.lbhmft || p.lbhmftd)
-        on_side(SIDE_SR, [&] {
-            if (p.lnmlj) sr_forces(true, nullptr, nullptr, nullptr);
-            if (p.lbhmft || p.lbhmftd) sr_forces(false, nullptr, nullptr, nullptr);
-        });
+    if (p.lnmlj || p.lbhmft || p.lbhmftd) {
+        auto sr = [&] {
+            if (p.lnmlj) launch_sr(*this, true);
+            if (p.lbhmft || p.lbhmftd) launch_sr(*this, false);
+        };
+        if (p.lcoulombic) on_side(SIDE_SR, sr);
+        else sr();
+    }
     if (p.lcoulombic && use32 && real32) {
         on_side(SIDE_PREP, [&] { launch_pair_prep32(*this); });
         prep_issued = true;
@@ -1273,18 +1240,17 @@ void Engine::engforce(bool check_finite) {
             else
                 launch_dir(*this, d_q, d_mu_tot, p.alphaES, lqch != 0, ld, ldmp != 0, true, false, false, false,
                            nullptr, nullptr, d_tmp3);
-            reduce(S_DIR_U, 7, ceil_div(n, 8));
         };
         on_side(SIDE_DIR, direct);
         RecOut o;
         o.f = d_f;
         o.f_dir = d_tmp3;
         o.coul = coul_unit;
+        o.fin = coul_fin(p.alphaES, true, true, true);
         if (rho_acc_ready) o.rho_acc = d_rho_acc;   // rho(k) of (q, mu_tot) from the fused CG
         rho_acc_ready = false;
         launch_rec(*this, d_q, d_mu_tot, lqch != 0, ld, o);
         join_side(SIDE_DIR);
-        finalize_coul(true);
     }
     for (int k = 0; k < NSIDE; k++) join_side(k);
     prep_issued = false;
@@ -1315,7 +1281,6 @@ void Engine::multipole_es_dev(const double *d_qv, const double3 *d_muv, double a
     if (dir) {
         launch_dir(*this, d_qv, d_muv, alpha, lq, ld, damp, fo || st, ef, want_efg_dir, efg, ef ? efd : nullptr,
                    want_efg_dir ? egd : nullptr, fd);
-        reduce(S_DIR_U, 7, ceil_div(n, 8));
     }
     if (rec) {
         RecOut o;
@@ -1339,16 +1304,8 @@ void Engine::multipole_es_dev(const double *d_qv, const double3 *d_muv, double a
     }
     MDFF_LAUNCH(*this, k_self_sums, nb, 256, 0, n, d_qv, d_muv, d_part, part_stride);
     reduce(S_Q2, 2, nb);
-    CoulFin cf;
-    cf.alpha = alpha;
-    cf.coul = coul_unit;
-    cf.inveOmegaPU = cell.inveOmegaPU;
-    cf.ttpiV = 2.0 * TPI_D * cell.inveOmega;
-    cf.do_dir = dir;
-    cf.do_rec = rec;
-    cf.do_stress = st;
     MDFF_CK(cudaMemsetAsync(d_out->tau_coul, 0, sizeof(double) * 9, stream));
-    MDFF_LAUNCH(*this, k_finalize_coul, 1, 1, 0, d_scal, cf, &d_out->u_coul, &d_out->pvir_coul, d_out->tau_coul);
+    MDFF_LAUNCH(*this, k_finalize_coul, 1, 1, 0, coul_fin(alpha, dir, rec, st));
 }
 
 // ---------------------------------------------------------------- kernel timing
@@ -1392,7 +1349,7 @@ void Engine::prof_result(double *ms, long long *count, double *flops) {
 }
 
 // ---------------------------------------------------------------- integration
-void Engine::prop_agate(int step) {
+void Engine::prop_agate(int step, const StepCheck &check) {
     istep = step;
     int nb = ceil_div(n, 256);
     switch (p.egrator) {
@@ -1402,80 +1359,19 @@ void Engine::prop_agate(int step) {
                     part_stride);
         reduce(S_KIN, 1, nb);
         MDFF_LAUNCH(*this, k_set_ekin, 1, 1, 0, d_scal, d_out);
+        if (check.on) launch_check_list(*this, check.h);
         break;
     }
-    case 2: {  // nhcn, src/integration.c:140-182
-        NhcArgs a;
-        a.nn = p.nhc_n;
-        a.yo = p.nhc_yosh_order;
-        a.mults = p.nhc_mults;
-        a.dt = dt;
-        a.temp = temp;
-        a.L = 3.0 * (double)n;
-        for (int k = 0; k < 7; k++) a.w[k] = 0.0;
-        switch (a.yo) {  // Yoshida weights, src/integration.c:205-236
-        case 1: a.w[0] = 1.0; break;
-        case 3:
-            a.w[0] = 1.0 / (2.0 - std::pow(2.0, 1.0 / 3.0));
-            a.w[1] = 1.0 - 2.0 * a.w[0];
-            a.w[2] = a.w[0];
-            break;
-        case 5:
-            a.w[0] = 1.0 / (4.0 - std::pow(4.0, 1.0 / 3.0));
-            a.w[1] = a.w[2] = a.w[3] = a.w[0];
-            a.w[4] = 1.0 - 4.0 * a.w[0];
-            break;
-        case 7:
-            a.w[0] = .78451361047756;
-            a.w[1] = .235573213359357;
-            a.w[2] = -1.17767998417887;
-            a.w[3] = 1.0 - 2.0 * (a.w[0] + a.w[1] + a.w[2]);
-            a.w[4] = a.w[2];
-            a.w[5] = a.w[1];
-            a.w[6] = a.w[0];
-            break;
-        default: throw Error(MDFFGPU_ERR_ARG, "nhc_yosh_order must be 1, 3, 5 or 7");
-        }
-        if (a.nn < 2 || a.nn > 16) throw Error(MDFFGPU_ERR_ARG, "nhc_n must be in 2..16");
-        // the kinetic sums are reduced by the last block of the kernel that forms them
-        ScaleKinArgs sk;
-        sk.n = n;
-        sk.energy = 0;
-        sk.nn = a.nn;
-        sk.L = a.L;
-        sk.temp = temp;
-        sk.out_s = d_out;
-        sk.mass = d_mass;
-        sk.nhc = d_nhc;
-        sk.v = d_v;
-        sk.part = d_part;
-        sk.scal = d_scal;
-        sk.stride = part_stride;
-        sk.ticket = d_ticket + 6;
-        sk.out = d_out;
-        sk.scale = 0;
-        MDFF_LAUNCH(*this, k_scale_kin, nb, 256, 0, sk);
-        launch_nhc_chain(*this, a, d_nhc, d_scal, d_out);
-        sk.scale = 1;
-        MDFF_LAUNCH(*this, k_scale_kin, nb, 256, 0, sk);
-        MDFF_LAUNCH(*this, k_pv1, nb, 256, 0, n, dt, dt * 0.5, d_invmass, d_r, d_v, d_f);
-        engforce(false);   // the finiteness check runs in k_pv2
-        MDFF_LAUNCH(*this, k_pv2, nb, 256, 0, n, dt * 0.5, d_invmass, d_mass, d_v, d_f, d_part, part_stride,
-                    d_scal, d_ticket + 6, d_r, d_status);
-        launch_nhc_chain(*this, a, d_nhc, d_scal, d_out);
-        sk.energy = 1;   // then e_kin and e_nvt
-        MDFF_LAUNCH(*this, k_scale_kin, nb, 256, 0, sk);
+    case 2:  // nhcn, src/integration.c:140-182
+        step_nhc_open(*this);
+        engforce(false, true);
+        step_nhc_close(*this, check);
         break;
-    }
-    default: {  // prop_velocity_verlet, src/integration.c:22-63
-        double dtsq2 = dt * dt * 0.5, dt2 = dt * 0.5;
-        MDFF_LAUNCH(*this, k_vv1, nb, 256, 0, n, dt, dtsq2, d_invmass, d_r, d_v, d_f, d_f2);
-        engforce();
-        MDFF_LAUNCH(*this, k_vv2, nb, 256, 0, n, dt2, d_invmass, d_mass, d_v, d_f, d_f2, d_part, part_stride);
-        reduce(S_KIN, 1, nb);
-        MDFF_LAUNCH(*this, k_set_ekin, 1, 1, 0, d_scal, d_out);
+    default:  // prop_velocity_verlet, src/integration.c:22-63
+        step_vv_open(*this);
+        engforce(false, true);
+        step_vv_close(*this, check);
         break;
-    }
     }
 }
 
@@ -1511,9 +1407,10 @@ void Engine::capture_step(int step) {
     capturing = true;
     cudaGraph_t graph = nullptr;
     try {
-        MDFF_CK(cudaMemsetAsync(d_status, 0, sizeof(unsigned), stream));
-        prop_agate(step);
-        check_verletlist(false);
+        if (p.egrator == 0) MDFF_CK(cudaMemsetAsync(d_status, 0, sizeof(unsigned), stream));
+        // the rebuild as an IF node: on the steps without one its kernels do not launch
+        record_if([&](cudaGraphConditionalHandle h) { prop_agate(step, StepCheck{true, &h}); },
+                  [&] { launch_build_lists(*this, false); });
     } catch (...) {
         capturing = false;
         forget_sides();
@@ -1583,9 +1480,9 @@ void Engine::md_steps(int first, int nsteps, double *thermo, const double *const
             istep = step;
             MDFF_CK(cudaGraphLaunch(step_exec, stream));
         } else {
-            MDFF_CK(cudaMemsetAsync(d_status, 0, sizeof(unsigned), stream));
-            prop_agate(step);
-            if (p.lverletL) check_verletlist(false);
+            if (p.egrator == 0) MDFF_CK(cudaMemsetAsync(d_status, 0, sizeof(unsigned), stream));
+            prop_agate(step, StepCheck{p.lverletL != 0, nullptr});
+            if (p.lverletL) rebuild_if_due();
         }
         if (s == nsteps - 1) queue_out();   // on the last step's synchronisation
         sync_scalars();

@@ -129,17 +129,18 @@ inline T *dalloc(size_t count) {
 
 // ---------------------------------------------------------------- launchers
 // lists.cu
-void launch_kardir(Engine &e, const double4 *r, double4 *s);
+void launch_kardir(Engine &e, const double4 *r, double4 *s, double3 *f = nullptr);   // f: zeroed too
 // sets e.d_rebuild on the device (and, given a handle, the condition of a recorded IF node)
 void launch_check_list(Engine &e, const cudaGraphConditionalHandle *h = nullptr);
 void launch_build_lists(Engine &e, bool force); // gated by d_rebuild unless force
 // pair.cu
-void launch_sr(Engine &e, bool lj);            // adds forces into e.d_f, partials into slots
+void launch_sr(Engine &e, bool lj);            // adds forces into e.d_f; u, virial, stress into d_out
 // real-space multipole sum on e.d_s (fractional positions); q, mu per ion.  forces:
-// per-ion force into out_f plus energy/virial partials (slots S_DIR_*); ef: field into
+// per-ion force into out_f; energy: u and virial summed into the slots S_DIR_*; ef: field into
 // out_ef; efg: EFG into out_efg (efg_q adds the charge part, src/ewald.c:724-729).
 void launch_dir(Engine &e, const double *q, const double3 *mu, double alpha, bool lq, bool ld, bool damp,
-                bool forces, bool ef, bool efg, bool efg_q, double3 *out_ef, double *out_efg, double3 *out_f);
+                bool forces, bool ef, bool efg, bool efg_q, double3 *out_ef, double *out_efg, double3 *out_f,
+                bool energy = true);
 // per list entry (F1/d^3, 3 F2/d^5) for the current positions, then the dipole-only
 // field from them (the induced-dipole iterations of one force evaluation)
 void launch_dir_prep(Engine &e, double alpha);
@@ -157,7 +158,17 @@ struct CgAp {
     double *scal = nullptr;
     unsigned *ticket = nullptr;
 };
+// composition of u_coul, pvir_coul, tau_coul (finalize_coul) by the first block of a force pass:
+// the real-space, k-space and self sums are complete before it starts
+struct CoulFin {
+    int on = 0;
+    double alpha, coul, inveOmegaPU, ttpiV;
+    int do_dir, do_rec, do_stress;
+    const double *scal;
+    double *u, *pvir, *tau;
+};
 struct RecOut {
+    CoulFin fin;
     double3 *ef = nullptr;            // self2*mu + ef_dir + E_rec
     const double3 *ef_dir = nullptr;
     double self2 = 0.0;
@@ -190,19 +201,18 @@ struct AspcCoef {
     double c[6];     // their coefficients, newest first
 };
 AspcCoef aspc_coef(int e, bool poly);
-// k_scale_kin: v *= nhc_s (scale), the kinetic sum into scal[S_KIN], then (energy) e_kin
-// and e_nvt
-struct ScaleKinArgs {
-    int n, scale, energy, nn;
-    double L, temp;
-    const DevScalars *out_s;
-    const double *mass, *nhc;
-    double3 *v;
-    double *part, *scal;
-    int stride;
-    unsigned *ticket;
-    DevScalars *out;
+// integrate.cu: the integrators around one force evaluation.  Each opens with the new positions
+// (and their fractional coordinates, zeroed forces and a cleared status word, so the evaluation
+// starts at its pair kernels) and closes with the kinetic sum, the finiteness check and, with
+// check, the list test of check_verletlist (handle h: it sets the condition of a recorded IF node)
+struct StepCheck {
+    bool on = false;
+    const cudaGraphConditionalHandle *h = nullptr;
 };
+void step_vv_open(Engine &e);
+void step_vv_close(Engine &e, const StepCheck &c);
+void step_nhc_open(Engine &e);
+void step_nhc_close(Engine &e, const StepCheck &c);
 void launch_reduce_slots(Engine &e, int first_slot, int nslots, int nparts);
 // true once the FP32 pair/k-space kernels exist in this build
 inline bool mixed_available() { return true; }
@@ -213,7 +223,10 @@ inline bool mixed_available() { return true; }
 // dipole-field records (zero at the others)
 void launch_pair_prep32(Engine &e);
 void launch_dir32(Engine &e, const double *q, const double3 *mu, double alpha, bool lq, bool ld, bool damp,
-                  bool forces, bool ef, double3 *out_ef, double3 *out_f, const int *idx = nullptr, int cnt = 0);
+                  bool forces, bool ef, double3 *out_ef, double3 *out_f, bool energy = true, const int *idx = nullptr,
+                  int cnt = 0);
+// pair.cu: whether a pair kernel of that many blocks sums its energy slots in its last block
+bool sum_in_last(const Engine &e, int blocks);
 void launch_pol_field32(Engine &e, const double3 *p, double3 *out_ef);
 // kspace32.cu: per force evaluation, the phase tables of the current positions
 void launch_coords32(Engine &e);
@@ -496,11 +509,11 @@ struct Engine {
                    double *fy, double *fz);
     void gen_verletlist();
     int check_verletlist(bool reset_status = true);
+    int rebuild_if_due();      // after the device's skin test: the gated build, its flags read back
     void ensure_lists();
     void half_list(int which, int *point, int *list, int cap, int *count);
-    void engforce(bool check_finite = true);   // check_finite: ST_NONFINITE from r and f
-    void sr_forces(bool lj, double *u, double *pvir, double *tau);
-    void sr_finish(bool lj);   // reduce the short-range slot, u / virial / stress into d_out
+    // check_finite: ST_NONFINITE from r and f; opened: d_s, d_f = 0 and the status word are set
+    void engforce(bool check_finite = true, bool opened = false);
     void multipole_es_dev(const double *d_qv, const double3 *d_muv, double alpha, int flags, double3 *d_ef_out,
                           double *d_efg_out, double3 *d_f_out);
     void field_of(const double *d_qv, const double3 *d_muv, bool lq, bool ld, bool damp, double3 *d_ef_out,
@@ -514,7 +527,7 @@ struct Engine {
     void pim_ko();
     void ko_inner(double3 *d_dmu, const double3 *d_find);
     double rmsd_of(const double3 *d_mu, const double3 *d_ef, double *upol_sum);
-    void prop_agate(int step);
+    void prop_agate(int step, const StepCheck &check = StepCheck());
     // in: 6 host arrays (rx..vz) copied in first, out: 9 host arrays (rx..fz) filled after
     // the last step; both optional, entries may be null (mdffgpu_md_steps_host)
     void md_steps(int first, int nsteps, double *thermo, const double *const *in = nullptr,
@@ -549,7 +562,7 @@ struct Engine {
     void drop_graph();
     void sync_scalars();
     void check_status();
-    void finalize_coul(bool stress);
+    CoulFin coul_fin(double alpha, bool dir, bool rec, bool stress);
     void reduce(int first_slot, int nslots, int nparts) { launch_reduce_slots(*this, first_slot, nslots, nparts); }
 };
 

@@ -579,11 +579,12 @@ void Engine::coul_forces(const double *d_qv, const double3 *d_muv, bool lq, bool
     // mixed: the FP32 real-space pass reads the context's charges from the packed
     // fractional coordinates, so d_qv may only be the charges themselves or absent (lq)
     if (use32 && real32)
-        launch_dir32(*this, d_qv, d_muv, p.alphaES, lq, ld, ldmp != 0, true, false, nullptr, d_tmp3);
+        launch_dir32(*this, d_qv, d_muv, p.alphaES, lq, ld, ldmp != 0, true, false, nullptr, d_tmp3, false);
     else
         launch_dir(*this, d_qv, d_muv, p.alphaES, lq, ld, ldmp != 0, true, false, false, false, nullptr, nullptr,
-                   d_tmp3);
+                   d_tmp3, false);
     RecOut o;
+    o.energy = false;
     o.f = out;
     o.f_dir = d_tmp3;
     o.coul = coul_unit;
@@ -669,6 +670,7 @@ void Engine::fit_issue(const double3 *d_ft, double scale, int tSi, int tO, const
     for (int comp = 0; comp < 3; comp++) {
         MDFF_LAUNCH(*this, k_scale_by_w, nb, 256, 0, n, comp, q, d_mu_tot, d_w, d_qw, d_muw);
         RecOut o;
+        o.energy = false;
         o.rho_raw = d_rw + (size_t)comp * nk;
         launch_rec(*this, d_qw, d_muw, true, true, o);
     }
@@ -676,12 +678,14 @@ void Engine::fit_issue(const double3 *d_ft, double scale, int tSi, int tO, const
                 d_rw + 3 * (size_t)nk);
     {
         RecOut o;
+        o.energy = false;
         o.ef = d_fa;   // E_rec of drho_w (no self, no direct part)
         o.rho_acc = d_rw + 3 * (size_t)nk;
         launch_rec(*this, q, d_mu_tot, false, true, o);
     }
     {
         RecOut o;   // EFG_rec of (q, mu)
+        o.energy = false;
         o.efg = d_efg_rec;
         o.ef = d_fb;
         launch_rec(*this, q, d_mu_tot, true, true, o);

@@ -1,7 +1,9 @@
 // Per-ion vector kernels: reductions, integrators (velocity Verlet, leap-frog,
 // Nose-Hoover chain), induced-dipole updates (Jacobi/ASPC, CG) and the composition of
 // the reference's energy/virial/stress globals.
-#include "engine.cuh"
+#include <cmath>
+
+#include "step.cuh"
 
 namespace mdffgpu {
 
@@ -92,54 +94,10 @@ __global__ void k_efg_self_dir(int n, double self2, const double *__restrict__ q
 }
 
 // ---------------------------------------------------------------- composition
-// u, pvir, tau of a short-range evaluator from its slots (src/nmlj.c:351-363):
-// slot 0 holds the full-list energy sum (each pair twice), slots 1..6 the full-list
-// sum of r_a f_b + r_b f_a.
-__global__ void k_finalize_sr(const double *__restrict__ scal, int slot, double inveOmegaPU, double *u, double *pvir,
-                              double *tau) {
+__global__ void k_finalize_coul(CoulFin c) {
     grid_dep();
     if (threadIdx.x || blockIdx.x) return;
-    *u = 0.5 * scal[slot];
-    double t[6];
-    for (int k = 0; k < 6; k++) t[k] = 0.25 * scal[slot + 1 + k] * inveOmegaPU;
-    double full[9] = {t[0], t[1], t[2], t[1], t[3], t[4], t[2], t[4], t[5]};
-    double pv = 0.0;
-    for (int k = 0; k < 9; k++) tau[k] = full[k];
-    for (int k = 0; k < 3; k++) pv += full[4 * k] * (1.0 / 3.0);
-    *pvir = pv;
-}
-
-// u_coul, tau_coul (src/ewald.c:209-307): dir (full-list sums), rec, self
-struct CoulFin {
-    double alpha, coul, inveOmegaPU, ttpiV;
-    int do_dir, do_rec, do_stress;
-};
-__global__ void k_finalize_coul(const double *__restrict__ scal, CoulFin c, double *u, double *pvir, double *tau) {
-    grid_dep();
-    if (threadIdx.x || blockIdx.x) return;
-    const double rpi = 1.7724538509055160273;
-    double alpha2 = c.alpha * c.alpha, selfa = c.alpha / rpi, selfa2 = 2.0 * selfa * alpha2 / 3.0;
-    double u_self = -selfa * scal[S_Q2] + -selfa2 * scal[S_MU2];
-    double u_dir = c.do_dir ? 0.5 * scal[S_DIR_U] : 0.0;
-    double u_rec = c.do_rec ? scal[S_REC_U] * c.ttpiV : 0.0;
-    *u = (u_dir + u_rec + u_self) * c.coul;
-    if (c.do_stress) {
-        double td[6], tr[6];
-        for (int k = 0; k < 6; k++) {
-            td[k] = 0.25 * scal[S_DIR_TAU + k] * c.inveOmegaPU;
-            tr[k] = scal[S_REC_TAU + k] * c.ttpiV * c.inveOmegaPU;
-        }
-        int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-        for (int k = 0; k < 9; k++) {
-            double t = 0.0;
-            if (c.do_dir) t += td[map[k]] * c.coul;
-            if (c.do_rec) t += tr[map[k]] * c.coul;
-            tau[k] = t;
-        }
-    }
-    double pv = 0.0;
-    for (int k = 0; k < 3; k++) pv += tau[4 * k] * (1.0 / 3.0);
-    *pvir = pv;
+    finalize_coul(c);
 }
 
 // ---------------------------------------------------------------- PIM
@@ -409,156 +367,99 @@ __global__ void k_cg_dir(int n, const double *__restrict__ scal, const double3 *
 }
 
 // ---------------------------------------------------------------- integrators
+// What bounds them: launches.  Velocity Verlet is two kernels around the force evaluation, the
+// Nose-Hoover step four: the coordinates, sums, checks and the skin test that follow from a
+// kernel's own ions are formed there or in its last block.  As kernels of their own (kardir,
+// the force memset, kinetic sum, finiteness check, list check, the chain) they were 9 more
+// launches of 1.3-5 us in a velocity-Verlet step, 6 more in a Nose-Hoover one.
+struct StepArgs {
+    int n;
+    Cell c;
+    double dt;
+    const double *mass, *invm;
+    double4 *r, *s;
+    double3 *v, *f, *fs;
+    double *part, *scal;
+    int stride;
+    unsigned *ticket, *status;
+    DevScalars *out;
+};
+static StepArgs step_args(Engine &e) {
+    StepArgs a;
+    a.n = e.n;
+    a.c = e.cell;
+    a.dt = e.dt;
+    a.mass = e.d_mass;
+    a.invm = e.d_invmass;
+    a.r = e.d_r;
+    a.s = e.d_s;
+    a.v = e.d_v;
+    a.f = e.d_f;
+    a.fs = e.d_f2;
+    a.part = e.d_part;
+    a.scal = e.d_scal;
+    a.stride = e.part_stride;
+    a.ticket = e.d_ticket + 6;
+    a.status = e.d_status;
+    a.out = e.d_out;
+    return a;
+}
+
+// the new position of an ion: stored, its fractional coordinates, zeroed force
+__device__ __forceinline__ void open_ion(const StepArgs &a, int i, double4 x) {
+    a.r[i] = x;
+    const double3 q = kardir(a.c, x.x, x.y, x.z);
+    a.s[i] = make_double4(q.x, q.y, q.z, x.w);
+    a.f[i] = make_double3(0.0, 0.0, 0.0);
+}
+
 // prop_velocity_verlet first half (src/integration.c:33-38)
-__global__ void k_vv1(int n, double dt, double dtsq2, const double *__restrict__ invm, double4 *__restrict__ r,
-                      const double3 *__restrict__ v, const double3 *__restrict__ f, double3 *__restrict__ fs) {
+__global__ void __launch_bounds__(256) k_vv1(StepArgs a) {
     grid_dep();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double4 x = r[i];
-    double3 vv = v[i], ff = f[i];
-    double im = invm[i];
-    fs[i] = ff;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *a.status = 0u;
+    if (i >= a.n) return;
+    const double dt = a.dt, dtsq2 = dt * dt * 0.5;
+    double4 x = a.r[i];
+    const double3 vv = a.v[i], ff = a.f[i];
+    const double im = a.invm[i];
+    a.fs[i] = ff;
     x.x += vv.x * dt + (ff.x * dtsq2) * im;
     x.y += vv.y * dt + (ff.y * dtsq2) * im;
     x.z += vv.z * dt + (ff.z * dtsq2) * im;
-    r[i] = x;
+    open_ion(a, i, x);
 }
 
-// prop_velocity_verlet second half (src/integration.c:47-57) + kinetic partials
-__global__ void k_vv2(int n, double dt2, const double *__restrict__ invm, const double *__restrict__ mass,
-                      double3 *__restrict__ v, const double3 *__restrict__ f, const double3 *__restrict__ fs,
-                      double *part, int stride) {
+// prop_velocity_verlet second half (src/integration.c:47-57), e_kin
+__global__ void __launch_bounds__(256) k_vv2(StepArgs a, CheckArgs c) {
     grid_dep();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double k[1] = {0.0};
-    if (i < n) {
-        double3 vv = v[i], ff = f[i], f0 = fs[i];
-        double im = invm[i];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const double dt2 = a.dt * 0.5;
+    double k[1] = {0.0}, m = 0.0;
+    if (i < a.n) {
+        double3 vv = a.v[i];
+        const double3 ff = a.f[i], f0 = a.fs[i];
+        const double4 x = a.r[i];
+        const double im = a.invm[i];
+        if (!isfinite(x.x + x.y + x.z + ff.x + ff.y + ff.z)) atomicOr(a.status, ST_NONFINITE);
         vv.x += (f0.x + ff.x) * dt2 * im;
         vv.y += (f0.y + ff.y) * dt2 * im;
         vv.z += (f0.z + ff.z) * dt2 * im;
-        v[i] = vv;
-        k[0] = (vv.x * vv.x + vv.y * vv.y + vv.z * vv.z) * mass[i];
-    }
-    block_sum_to_part<1>(k, part, S_KIN, stride);
-}
-
-// prop_pos_vel_verlet (src/integration.c:66-90): half kick + drift ...
-__global__ void k_pv1(int n, double dt, double dt2, const double *__restrict__ invm, double4 *__restrict__ r,
-                      double3 *__restrict__ v, const double3 *__restrict__ f) {
-    grid_dep();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double4 x = r[i];
-    double3 vv = v[i], ff = f[i];
-    double im = invm[i];
-    vv.x += ff.x * dt2 * im;
-    vv.y += ff.y * dt2 * im;
-    vv.z += ff.z * dt2 * im;
-    x.x += vv.x * dt;
-    x.y += vv.y * dt;
-    x.z += vv.z * dt;
-    v[i] = vv;
-    r[i] = x;
-}
-
-// ... and the second half kick + kinetic partials
-// second half kick of prop_velocity_verlet within nhcn (src/integration.c:165-167), the
-// kinetic sum reduced by the last block into scal[S_KIN]; with r: the finiteness check of
-// positions and forces (ST_NONFINITE) in the same pass
-__global__ void __launch_bounds__(256) k_pv2(int n, double dt2, const double *__restrict__ invm,
-                                             const double *__restrict__ mass, double3 *__restrict__ v,
-                                             const double3 *__restrict__ f, double *part, int stride,
-                                             double *scal, unsigned *ticket, const double4 *__restrict__ r,
-                                             unsigned *status) {
-    grid_dep();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double k[1] = {0.0};
-    if (i < n) {
-        double3 vv = v[i], ff = f[i];
-        double im = invm[i];
-        if (r) {
-            double4 x = r[i];
-            if (!isfinite(x.x + x.y + x.z + ff.x + ff.y + ff.z)) atomicOr(status, ST_NONFINITE);
-        }
-        vv.x += ff.x * dt2 * im;
-        vv.y += ff.y * dt2 * im;
-        vv.z += ff.z * dt2 * im;
-        v[i] = vv;
-        k[0] = (vv.x * vv.x + vv.y * vv.y + vv.z * vv.z) * mass[i];
-    }
-    block_sum_to_part<1>(k, part, S_KIN, stride);
-    last_block_slots(part, stride, S_KIN, 1, scal, ticket);
-}
-
-// kinetic partials, optionally after scaling v by the NHC factor s (src/integration.c:281-287)
-// e_kin and the NHC conserved-quantity term e_nvt (src/integration.c:156-176) from the
-// kinetic sum in scal[S_KIN]; one thread
-__device__ void nhc_energy(int nn, double L, double temp, const double *__restrict__ nhc,
-                           const double *__restrict__ scal, DevScalars *out) {
-    const double *xi = nhc, *vxi = nhc + 16, *Q = nhc + 32;
-    out->e_kin = 0.5 * scal[S_KIN];
-    double nvt1 = L * temp * xi[0], nvt2 = vxi[0] * vxi[0] * 0.5 / Q[0], nvt3 = 0.0, nvt4 = 0.0;
-    for (int i = 1; i < nn; i++) {
-        nvt3 += vxi[i] * vxi[i] * 0.5 / Q[i];
-        nvt4 += temp * xi[i];
-    }
-    out->e_nvt = nvt1 + nvt2 + nvt3 + nvt4;
-    for (int i = 0; i < 16; i++) {
-        out->xi[i] = xi[i];
-        out->vxi[i] = vxi[i];
-    }
-}
-
-// v *= s (scale) and the kinetic sum sum m v^2: block partials in the S_KIN slot, which
-// the last block reduces into scal[S_KIN] as k_reduce_slots does (256-thread blocks);
-// energy: then e_kin and e_nvt (nhc_energy)
-__global__ void __launch_bounds__(256) k_scale_kin(ScaleKinArgs a) {
-    grid_dep();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double k[1] = {0.0};
-    if (i < a.n) {
-        double3 vv = a.v[i];
-        if (a.scale) {
-            double s = a.out_s->nhc_s;
-            vv.x *= s;
-            vv.y *= s;
-            vv.z *= s;
-            a.v[i] = vv;
-        }
+        a.v[i] = vv;
         k[0] = (vv.x * vv.x + vv.y * vv.y + vv.z * vv.z) * a.mass[i];
+        if (c.on) m = check_moved(c, a.s[i], i);
     }
     block_sum_to_part<1>(k, a.part, S_KIN, a.stride);
-    const bool last = last_block_slots(a.part, a.stride, S_KIN, 1, a.scal, a.ticket);
-    if (last && a.energy && threadIdx.x == 0) nhc_energy(a.nn, a.L, a.temp, a.nhc, a.scal, a.out);
-}
-
-// leap-frog (src/integration.c:93-137)
-__global__ void k_lf(int n, double dtsq, double idt, const double *__restrict__ invm, const double *__restrict__ mass,
-                     double4 *__restrict__ r, double3 *__restrict__ rs, double3 *__restrict__ v,
-                     const double3 *__restrict__ f, double *part, int stride) {
-    grid_dep();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double k[1] = {0.0};
-    if (i < n) {
-        double4 x = r[i];
-        double3 o = rs[i], ff = f[i];
-        double im = invm[i];
-        double ux = 2.0 * x.x - o.x + ff.x * dtsq * im;
-        double uy = 2.0 * x.y - o.y + ff.y * dtsq * im;
-        double uz = 2.0 * x.z - o.z + ff.z * dtsq * im;
-        double3 vv = make_double3(idt * (ux - o.x), idt * (uy - o.y), idt * (uz - o.z));
-        v[i] = vv;
-        k[0] = (vv.x * vv.x + vv.y * vv.y + vv.z * vv.z) * mass[i];
-        rs[i] = make_double3(x.x, x.y, x.z);
-        r[i] = make_double4(ux, uy, uz, x.w);
-    }
-    block_sum_to_part<1>(k, part, S_KIN, stride);
+    if (c.on) check_block(c, m);
+    if (!last_block(a.ticket)) return;
+    const int slot = S_KIN;
+    sum_slots(a.part, a.stride, &slot, 1, (int)gridDim.x, a.scal);
+    if (threadIdx.x == 0) a.out->e_kin = 0.5 * a.scal[S_KIN];
+    if (c.on) check_last(c);
 }
 
 // chain_nhcn (src/integration.c:189-294) on one thread: thermostat variables in
-// d_nhc (xi[16], vxi[16]); kin from the S_KIN slot (sum m v^2); writes s.  The
+// nhc (xi[16], vxi[16], Q[16]); kin from the S_KIN slot (sum m v^2); writes s.  The
 // second sweep stops at nhc_n-2 as in the reference (src/integration.c:269).  NN > 0:
 // the chain length known at compile time, the chain held in registers (the loops
 // unrolled); NN = 0: any length up to 16, the chain in local memory.  Either way the
@@ -566,11 +467,11 @@ __global__ void k_lf(int n, double dtsq, double idt, const double *__restrict__ 
 struct NhcArgs {
     int nn, yo, mults;
     double dt, temp, L, w[7];
+    double *nhc;
 };
 template <int NN>
-__global__ void k_nhc_chain(NhcArgs a, double *__restrict__ nhc, const double *__restrict__ scal, DevScalars *out) {
-    grid_dep();
-    if (threadIdx.x || blockIdx.x) return;
+__device__ void nhc_chain(const NhcArgs &a, const double *scal, DevScalars *out) {
+    double *nhc = a.nhc;
     constexpr int M = NN > 0 ? NN : 16;
     const int nn = NN > 0 ? NN : a.nn;
     double xi[M], vxi[M], Q[M], G[M];
@@ -623,14 +524,198 @@ __global__ void k_nhc_chain(NhcArgs a, double *__restrict__ nhc, const double *_
     out->nhc_s = s;
 }
 
-void launch_nhc_chain(Engine &e, const NhcArgs &a, double *nhc, const double *scal, DevScalars *out) {
-    switch (a.nn) {
-    case 2: MDFF_LAUNCH(e, k_nhc_chain<2>, 1, 1, 0, a, nhc, scal, out); break;
-    case 3: MDFF_LAUNCH(e, k_nhc_chain<3>, 1, 1, 0, a, nhc, scal, out); break;
-    case 4: MDFF_LAUNCH(e, k_nhc_chain<4>, 1, 1, 0, a, nhc, scal, out); break;
-    case 5: MDFF_LAUNCH(e, k_nhc_chain<5>, 1, 1, 0, a, nhc, scal, out); break;
-    default: MDFF_LAUNCH(e, k_nhc_chain<0>, 1, 1, 0, a, nhc, scal, out); break;
+// The kinetic sum and, in the last block, the chain.  KICK: the second half kick of
+// prop_pos_vel_verlet first (src/integration.c:66-90), with the finiteness check of positions
+// and forces (ST_NONFINITE); otherwise the step's opening (clears the status word).
+template <int NN, bool KICK>
+__global__ void __launch_bounds__(256) k_kin_chain(StepArgs a, NhcArgs h) {
+    grid_dep();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const double dt2 = a.dt * 0.5;
+    double k[1] = {0.0};
+    if (!KICK && i == 0) *a.status = 0u;
+    if (i < a.n) {
+        double3 vv = a.v[i];
+        if (KICK) {
+            const double3 ff = a.f[i];
+            const double4 x = a.r[i];
+            const double im = a.invm[i];
+            if (!isfinite(x.x + x.y + x.z + ff.x + ff.y + ff.z)) atomicOr(a.status, ST_NONFINITE);
+            vv.x += ff.x * dt2 * im;
+            vv.y += ff.y * dt2 * im;
+            vv.z += ff.z * dt2 * im;
+            a.v[i] = vv;
+        }
+        k[0] = (vv.x * vv.x + vv.y * vv.y + vv.z * vv.z) * a.mass[i];
     }
+    block_sum_to_part<1>(k, a.part, S_KIN, a.stride);
+    if (!last_block(a.ticket)) return;
+    const int slot = S_KIN;
+    sum_slots(a.part, a.stride, &slot, 1, (int)gridDim.x, a.scal);
+    if (threadIdx.x == 0) nhc_chain<NN>(h, a.scal, a.out);
+}
+
+// v *= s (src/integration.c:281-287), then half kick and drift of prop_pos_vel_verlet
+__global__ void __launch_bounds__(256) k_scale_pv1(StepArgs a) {
+    grid_dep();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.n) return;
+    const double s = a.out->nhc_s, dt = a.dt, dt2 = dt * 0.5;
+    double4 x = a.r[i];
+    double3 vv = a.v[i];
+    const double3 ff = a.f[i];
+    const double im = a.invm[i];
+    vv.x *= s;
+    vv.y *= s;
+    vv.z *= s;
+    vv.x += ff.x * dt2 * im;
+    vv.y += ff.y * dt2 * im;
+    vv.z += ff.z * dt2 * im;
+    x.x += vv.x * dt;
+    x.y += vv.y * dt;
+    x.z += vv.z * dt;
+    a.v[i] = vv;
+    open_ion(a, i, x);
+}
+
+// e_kin and the NHC conserved-quantity term e_nvt (src/integration.c:156-176) from the
+// kinetic sum in scal[S_KIN]; one thread
+__device__ void nhc_energy(int nn, double L, double temp, const double *__restrict__ nhc,
+                           const double *__restrict__ scal, DevScalars *out) {
+    const double *xi = nhc, *vxi = nhc + 16, *Q = nhc + 32;
+    out->e_kin = 0.5 * scal[S_KIN];
+    double nvt1 = L * temp * xi[0], nvt2 = vxi[0] * vxi[0] * 0.5 / Q[0], nvt3 = 0.0, nvt4 = 0.0;
+    for (int i = 1; i < nn; i++) {
+        nvt3 += vxi[i] * vxi[i] * 0.5 / Q[i];
+        nvt4 += temp * xi[i];
+    }
+    out->e_nvt = nvt1 + nvt2 + nvt3 + nvt4;
+    for (int i = 0; i < 16; i++) {
+        out->xi[i] = xi[i];
+        out->vxi[i] = vxi[i];
+    }
+}
+
+// the step's end: v *= s, kinetic sum, e_kin and e_nvt, the list check
+__global__ void __launch_bounds__(256) k_nhc_end(StepArgs a, NhcArgs h, CheckArgs c) {
+    grid_dep();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double k[1] = {0.0}, m = 0.0;
+    if (i < a.n) {
+        double3 vv = a.v[i];
+        const double s = a.out->nhc_s;
+        vv.x *= s;
+        vv.y *= s;
+        vv.z *= s;
+        a.v[i] = vv;
+        k[0] = (vv.x * vv.x + vv.y * vv.y + vv.z * vv.z) * a.mass[i];
+        if (c.on) m = check_moved(c, a.s[i], i);
+    }
+    block_sum_to_part<1>(k, a.part, S_KIN, a.stride);
+    if (c.on) check_block(c, m);
+    if (!last_block(a.ticket)) return;
+    const int slot = S_KIN;
+    sum_slots(a.part, a.stride, &slot, 1, (int)gridDim.x, a.scal);
+    if (threadIdx.x == 0) nhc_energy(h.nn, h.L, h.temp, h.nhc, a.scal, a.out);
+    if (c.on) check_last(c);
+}
+
+static CheckArgs step_check(Engine &e, const StepCheck &c) {
+    if (c.on) return check_args(e, c.h);
+    CheckArgs a{};
+    return a;
+}
+
+void step_vv_open(Engine &e) {
+    MDFF_LAUNCH(e, k_vv1, ceil_div(e.n, 256), 256, 0, step_args(e));
+    e.phase64_ready = false;
+}
+void step_vv_close(Engine &e, const StepCheck &c) {
+    MDFF_LAUNCH(e, k_vv2, ceil_div(e.n, 256), 256, 0, step_args(e), step_check(e, c));
+}
+
+static NhcArgs nhc_args(Engine &e) {
+    NhcArgs a;
+    a.nn = e.p.nhc_n;
+    a.yo = e.p.nhc_yosh_order;
+    a.mults = e.p.nhc_mults;
+    a.dt = e.dt;
+    a.temp = e.temp;
+    a.L = 3.0 * (double)e.n;
+    a.nhc = e.d_nhc;
+    for (int k = 0; k < 7; k++) a.w[k] = 0.0;
+    switch (a.yo) {  // Yoshida weights, src/integration.c:205-236
+    case 1: a.w[0] = 1.0; break;
+    case 3:
+        a.w[0] = 1.0 / (2.0 - std::pow(2.0, 1.0 / 3.0));
+        a.w[1] = 1.0 - 2.0 * a.w[0];
+        a.w[2] = a.w[0];
+        break;
+    case 5:
+        a.w[0] = 1.0 / (4.0 - std::pow(4.0, 1.0 / 3.0));
+        a.w[1] = a.w[2] = a.w[3] = a.w[0];
+        a.w[4] = 1.0 - 4.0 * a.w[0];
+        break;
+    case 7:
+        a.w[0] = .78451361047756;
+        a.w[1] = .235573213359357;
+        a.w[2] = -1.17767998417887;
+        a.w[3] = 1.0 - 2.0 * (a.w[0] + a.w[1] + a.w[2]);
+        a.w[4] = a.w[2];
+        a.w[5] = a.w[1];
+        a.w[6] = a.w[0];
+        break;
+    default: throw Error(MDFFGPU_ERR_ARG, "nhc_yosh_order must be 1, 3, 5 or 7");
+    }
+    if (a.nn < 2 || a.nn > 16) throw Error(MDFFGPU_ERR_ARG, "nhc_n must be in 2..16");
+    return a;
+}
+
+template <bool KICK>
+static void launch_kin_chain(Engine &e, const NhcArgs &h) {
+    const int nb = ceil_div(e.n, 256);
+    const StepArgs a = step_args(e);
+    switch (h.nn) {
+    case 2: MDFF_LAUNCH(e, (k_kin_chain<2, KICK>), nb, 256, 0, a, h); break;
+    case 3: MDFF_LAUNCH(e, (k_kin_chain<3, KICK>), nb, 256, 0, a, h); break;
+    case 4: MDFF_LAUNCH(e, (k_kin_chain<4, KICK>), nb, 256, 0, a, h); break;
+    case 5: MDFF_LAUNCH(e, (k_kin_chain<5, KICK>), nb, 256, 0, a, h); break;
+    default: MDFF_LAUNCH(e, (k_kin_chain<0, KICK>), nb, 256, 0, a, h); break;
+    }
+}
+
+void step_nhc_open(Engine &e) {
+    launch_kin_chain<false>(e, nhc_args(e));
+    MDFF_LAUNCH(e, k_scale_pv1, ceil_div(e.n, 256), 256, 0, step_args(e));
+    e.phase64_ready = false;
+}
+void step_nhc_close(Engine &e, const StepCheck &c) {
+    const NhcArgs h = nhc_args(e);
+    launch_kin_chain<true>(e, h);
+    MDFF_LAUNCH(e, k_nhc_end, ceil_div(e.n, 256), 256, 0, step_args(e), h, step_check(e, c));
+}
+
+// leap-frog (src/integration.c:93-137)
+__global__ void k_lf(int n, double dtsq, double idt, const double *__restrict__ invm, const double *__restrict__ mass,
+                     double4 *__restrict__ r, double3 *__restrict__ rs, double3 *__restrict__ v,
+                     const double3 *__restrict__ f, double *part, int stride) {
+    grid_dep();
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double k[1] = {0.0};
+    if (i < n) {
+        double4 x = r[i];
+        double3 o = rs[i], ff = f[i];
+        double im = invm[i];
+        double ux = 2.0 * x.x - o.x + ff.x * dtsq * im;
+        double uy = 2.0 * x.y - o.y + ff.y * dtsq * im;
+        double uz = 2.0 * x.z - o.z + ff.z * dtsq * im;
+        double3 vv = make_double3(idt * (ux - o.x), idt * (uy - o.y), idt * (uz - o.z));
+        v[i] = vv;
+        k[0] = (vv.x * vv.x + vv.y * vv.y + vv.z * vv.z) * mass[i];
+        rs[i] = make_double3(x.x, x.y, x.z);
+        r[i] = make_double4(ux, uy, uz, x.w);
+    }
+    block_sum_to_part<1>(k, part, S_KIN, stride);
 }
 
 __global__ void k_set_ekin(const double *__restrict__ scal, DevScalars *out) {

@@ -21,7 +21,7 @@ namespace mdffgpu {
 __device__ __forceinline__ void rho_finish(int k, int nk, double2 rho, const double *__restrict__ Ak,
                                            const double *__restrict__ kcoe, const double3 *__restrict__ kv,
                                            double2 *__restrict__ rho_s, double *__restrict__ ppart, int slot,
-                                           int stride) {
+                                           int stride, bool energy) {
     int l = threadIdx.x & 31;
     double v[7] = {0, 0, 0, 0, 0, 0, 0};
     if (k < nk) {
@@ -37,6 +37,7 @@ __device__ __forceinline__ void rho_finish(int k, int nk, double2 rho, const dou
         v[5] = -co * kk.y * kk.z * str;
         v[6] = (1.0 - co * kk.z * kk.z) * str;
     }
+    if (!energy) return;
 #pragma unroll
     for (int q = 0; q < 7; q++) v[q] = warp_sum(v[q]);
     if (l < 7) {
@@ -51,12 +52,13 @@ __device__ __forceinline__ void rho_finish(int k, int nk, double2 rho, const dou
 // sum the ion-chunk partials of rho(k) in a fixed order, then rho_finish. A block owns
 // RHOR_K consecutive k (one per lane); its 8 warps take every 8th chunk and warp 0 adds
 // the 8 warp sums in warp order. rho_raw (optional) receives rho(k) itself.  Partials
-// are FP64 (kspace.cu) or FP32 (kspace32.cu: sums over one chunk of ions), added in FP64.
+// are FP32 sums over one chunk of ions, added in FP64.  scal set: energies too, the k sums by the
+// last block.
 __global__ void __launch_bounds__(256) k_rho_reduce(int nk, int nchunks, const float2 *__restrict__ part,
                                                     const double *__restrict__ Ak, const double *__restrict__ kcoe,
                                                     const double3 *__restrict__ kv, double2 *__restrict__ rho_s,
                                                     double2 *__restrict__ rho_raw, double *__restrict__ ppart,
-                                                    int slot, int stride) {
+                                                    int slot, int stride, double *scal, unsigned *ticket) {
     grid_dep();
     __shared__ double2 ws[8][RHOR_K];
     int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -81,26 +83,34 @@ __global__ void __launch_bounds__(256) k_rho_reduce(int nk, int nchunks, const f
     double2 acc = make_double2((a0.x + a1.x) + (a2.x + a3.x), (a0.y + a1.y) + (a2.y + a3.y));
     ws[w][l] = acc;
     __syncthreads();
-    if (w) return;
-    double2 rho = ws[0][l];
+    if (w == 0) {
+        double2 rho = ws[0][l];
 #pragma unroll
-    for (int q = 1; q < 8; q++) {
-        rho.x += ws[q][l].x;
-        rho.y += ws[q][l].y;
+        for (int q = 1; q < 8; q++) {
+            rho.x += ws[q][l].x;
+            rho.y += ws[q][l].y;
+        }
+        if (rho_raw && k < nk) rho_raw[k] = rho;
+        rho_finish(k, nk, rho, Ak, kcoe, kv, rho_s, ppart, slot, stride, scal != nullptr);
     }
-    if (rho_raw && k < nk) rho_raw[k] = rho;
-    rho_finish(k, nk, rho, Ak, kcoe, kv, rho_s, ppart, slot, stride);
+    if (!scal) return;
+    const int slots[7] = {slot, slot + 1, slot + 2, slot + 3, slot + 4, slot + 5, slot + 6};
+    last_block_warps(ppart, stride, slots, 7, scal, ticket);
 }
 
 // rho_finish on a rho(k) assembled elsewhere (one warp per RHOR_K k)
 __global__ void __launch_bounds__(32) k_rho_from_acc(int nk, const double2 *__restrict__ acc,
                                                      const double *__restrict__ Ak, const double *__restrict__ kcoe,
                                                      const double3 *__restrict__ kv, double2 *__restrict__ rho_s,
-                                                     double *__restrict__ ppart, int slot, int stride) {
+                                                     double *__restrict__ ppart, int slot, int stride, double *scal,
+                                                     unsigned *ticket) {
     grid_dep();
     int k = blockIdx.x * RHOR_K + threadIdx.x;
     double2 rho = k < nk ? acc[k] : make_double2(0.0, 0.0);
-    rho_finish(k, nk, rho, Ak, kcoe, kv, rho_s, ppart, slot, stride);
+    rho_finish(k, nk, rho, Ak, kcoe, kv, rho_s, ppart, slot, stride, scal != nullptr);
+    if (!scal) return;
+    const int slots[7] = {slot, slot + 1, slot + 2, slot + 3, slot + 4, slot + 5, slot + 6};
+    last_block_warps(ppart, stride, slots, 7, scal, ticket);
 }
 
 // ---------------------------------------------------------------- launcher
@@ -112,15 +122,15 @@ __global__ void __launch_bounds__(32) k_rho_from_acc(int nk, const double2 *__re
 static void launch_rec32(Engine &e, const double *q, const double3 *mu, bool lq, bool ld, const RecOut &o) {
     int nbr = ceil_div(e.nk, RHOR_K);
     int cnt = o.idx ? o.cnt : e.n;
+    double *scal = o.energy ? e.d_scal : nullptr;   // energy and virial sums wanted
     if (o.rho_acc) {
         MDFF_LAUNCH(e, k_rho_from_acc, nbr, 32, 0, e.nk, o.rho_acc, e.d_Ak, e.d_kcoe, e.d_kvec, e.d_rho, e.d_part,
-                    (int)S_REC_U, e.part_stride);
+                    (int)S_REC_U, e.part_stride, scal, e.d_ticket + 2);
     } else {
         launch_rho32(e, q, mu, lq, ld, o.idx, cnt);
         MDFF_LAUNCH(e, k_rho_reduce, nbr, 256, 0, e.nk, e.rho_chunks_used, e.d_rho_part32, e.d_Ak, e.d_kcoe,
-                    e.d_kvec, e.d_rho, o.rho_raw, e.d_part, (int)S_REC_U, e.part_stride);
+                    e.d_kvec, e.d_rho, o.rho_raw, e.d_part, (int)S_REC_U, e.part_stride, scal, e.d_ticket + 2);
     }
-    if (o.energy) e.reduce(S_REC_U, 7, nbr);
     if (!o.ef && !o.f) return;
     if (o.out_idx) launch_ion32(e, lq ? q : nullptr, mu, ld, o, o.out_idx, o.out_cnt);
     else launch_ion32(e, lq ? q : nullptr, mu, ld, o, o.idx, cnt);

@@ -30,7 +30,7 @@
 //             ION32_RUN rows and by FP32 steps in ny between.  Row sums FP32, rows FP64.
 // Both passes take an optional ion index list (the polarisable ions of an induced-
 // dipole iteration, whose search directions vanish elsewhere).
-#include "engine.cuh"
+#include "step.cuh"
 
 namespace mdffgpu {
 
@@ -531,12 +531,14 @@ struct Comb32Args {
     double3 *ef;
     const double3 *f_dir;
     double3 *f;
+    CoulFin fin;
     CgAp cg;
 };
 
 template <bool WF>
 __global__ void k_combine32(Comb32Args a) {
     grid_dep();
+    if (WF && a.fin.on && blockIdx.x == 0 && threadIdx.x == 0) finalize_coul(a.fin);
     int li = blockIdx.x * blockDim.x + threadIdx.x;
     double pap[1] = {0.0};
     if (li < a.cnt) {
@@ -802,6 +804,7 @@ void launch_combine32(Engine &e, const double *q, const double3 *mu, bool ld, co
     b.f_dir = o.f_dir;
     b.f = o.f;
     b.cg = o.cg;
+    b.fin = o.fin;
     if (b.cg.ap && (wf || !o.ef)) throw Error(MDFFGPU_ERR_STATE, "the CG product needs a field-only pass");
     int nb = ceil_div(std::max(cnt, 1), 256);
     if (wf) MDFF_LAUNCH(e, k_combine32<true>, nb, 256, 0, b);

@@ -31,7 +31,7 @@
 #include <algorithm>
 #include <type_traits>
 
-#include "engine.cuh"
+#include "step.cuh"
 
 namespace mdffgpu {
 
@@ -371,6 +371,7 @@ struct Ion64Args {
     const double *qself;     // self terms use q and mu whatever lq/ld (src/ewald.c:201-224)
     const double3 *muself;
     CgAp cg;
+    CoulFin fin;
 };
 
 // the results of one ion from its sums S = sum n Im, Hm = sum n n^T Re (n-space)
@@ -454,6 +455,7 @@ __device__ __forceinline__ double ion64_write(const Ion64Args &a, int i, const d
 template <int KS, bool WF, int MT, int WS>
 __global__ void __launch_bounds__(WS == 1 ? 32 * I64_WARPS : 32 * WS) k_ion64(Ion64Args a) {
     grid_dep();
+    if (WF && a.fin.on && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) finalize_coul(a.fin);
     constexpr int NTT = WF ? 3 : 2, NV = WF ? 9 : 3, IW = WS == 1 ? I64_WARPS : 1;   // warps over the ions
     const int l = threadIdx.x & 31, w = threadIdx.x >> 5, lk = l & 3, lr = l >> 2;
     const int base = (blockIdx.x * IW + (WS == 1 ? w : 0)) * 8 * MT;
@@ -806,6 +808,7 @@ void launch_rec64(Engine &e, const double *q, const double3 *mu, bool lq, bool l
     a.qself = o.self_q;
     a.muself = o.self_mu;
     a.cg = o.cg;
+    a.fin = o.fin;
     // tiles of 8 ions per warp, row slices within the block (ws) and of the grid: time in units
     // of one (row group, tile) per scheduler, plus the start of the block (8 units) and, with
     // slices in memory, the arrival and second read (16); several tiles per warp share each

@@ -10,126 +10,45 @@
 #include <algorithm>
 #include <cmath>
 
-#include "engine.cuh"
+#include "step.cuh"
 
 namespace mdffgpu {
 
-// s = kardir(r), w = charge
-__global__ void k_kardir(int n, Cell c, const double4 *__restrict__ r, double4 *__restrict__ s) {
+// s = kardir(r), w = charge; f (may be null) = 0
+__global__ void k_kardir(int n, Cell c, const double4 *__restrict__ r, double4 *__restrict__ s,
+                         double3 *__restrict__ f) {
     grid_dep();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double4 ri = r[i];
-    double3 f = kardir(c, ri.x, ri.y, ri.z);
-    s[i] = make_double4(f.x, f.y, f.z, ri.w);
+    double3 q = kardir(c, ri.x, ri.y, ri.z);
+    s[i] = make_double4(q.x, q.y, q.z, ri.w);
+    if (f) f[i] = make_double3(0.0, 0.0, 0.0);
 }
 
-void launch_kardir(Engine &e, const double4 *r, double4 *s) {
-    MDFF_LAUNCH(e, k_kardir, ceil_div(e.n, 256), 256, 0, e.n, e.cell, r, s);
+void launch_kardir(Engine &e, const double4 *r, double4 *s, double3 *f) {
+    MDFF_LAUNCH(e, k_kardir, ceil_div(e.n, 256), 256, 0, e.n, e.cell, r, s, f);
     e.phase64_ready = false;   // the positions may have moved
 }
 
 // ---------------------------------------------------------------- check_verletlist
-// displacement since the last build, largest and second largest (src/verlet.c:134-147)
-__device__ __forceinline__ void top2_insert(double &m1, double &m2, double d) {
-    if (d > m1) {
-        m2 = m1;
-        m1 = d;
-    } else if (d > m2) {
-        m2 = d;
-    }
-}
-
-// warp merge of per-lane top-2 pairs (the two largest values, whatever the order they
-// are met in)
-__device__ __forceinline__ void top2_warp(double &m1, double &m2) {
-    for (int o = 16; o > 0; o >>= 1) {
-        double o1 = __shfl_xor_sync(0xffffffffu, m1, o);
-        double o2 = __shfl_xor_sync(0xffffffffu, m2, o);
-        double n1 = fmax(m1, o1);
-        double n2 = fmax(fmin(m1, o1), fmax(m2, o2));
-        m1 = n1;
-        m2 = n2;
-    }
-}
-
 // check_verletlist in one launch: the fractional coordinates of the current positions
 // (kardir, written to s for a rebuild), each ion's displacement since the last build and
-// per block its two largest (src/verlet.c:134-147); the last block to finish merges the
-// block pairs and tests them against the skin (src/verlet.c:148).  On a rebuild it also
-// zeroes the cell counts the binning adds to, and in a recorded step it sets the
-// condition of the IF node that holds the rebuild (use_h).
-struct CheckArgs {
-    int n, ncell;
-    Cell c;
-    const double4 *r;
-    double4 *s;
-    const double4 *svl;
-    double *part1, *part2;
-    unsigned *ticket;
-    double skindiff;
-    int *rebuild, *cell_cnt;
-    DevScalars *out;
-    cudaGraphConditionalHandle h;
-    int use_h;
-};
-__global__ void __launch_bounds__(256) k_check_list(CheckArgs a) {
+// the skin test in the last block (step.cuh).  The kernels that close a step do the same
+// without a launch of their own.
+__global__ void __launch_bounds__(256) k_check_list(CheckArgs a, const double4 *__restrict__ r, unsigned *ticket) {
     grid_dep();
-    __shared__ double sm1[8], sm2[8];
-    __shared__ bool last;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double m1 = 0.0, m2 = 0.0;
+    double m = 0.0;
     if (i < a.n) {
-        const double4 ri = a.r[i];
+        const double4 ri = r[i];
         const double3 f = kardir(a.c, ri.x, ri.y, ri.z);
-        a.s[i] = make_double4(f.x, f.y, f.z, ri.w);
-        const double4 b = a.svl[i];
-        const double3 d = pbc_frac(a.c, dsub(f.x, b.x), dsub(f.y, b.y), dsub(f.z, b.z));
-        m1 = __dsqrt_rn(norm2_exact(d));
+        const double4 si = make_double4(f.x, f.y, f.z, ri.w);
+        a.s[i] = si;
+        m = check_moved(a, si, i);
     }
-    top2_warp(m1, m2);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) {
-        sm1[w] = m1;
-        sm2[w] = m2;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double a1 = 0.0, a2 = 0.0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) {
-            top2_insert(a1, a2, sm1[k]);
-            top2_insert(a1, a2, sm2[k]);
-        }
-        a.part1[blockIdx.x] = a1;
-        a.part2[blockIdx.x] = a2;
-        __threadfence();
-        last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    __shared__ int rb_s;
-    if (w == 0) {
-        const volatile double *p1 = a.part1, *p2 = a.part2;
-        double b1 = 0.0, b2 = 0.0;
-        for (int k = l; k < (int)gridDim.x; k += 32) {
-            top2_insert(b1, b2, p1[k]);
-            top2_insert(b1, b2, p2[k]);
-        }
-        top2_warp(b1, b2);
-        if (l == 0) {
-            const int rb = (b1 + b2 > a.skindiff) ? 1 : 0;   // src/verlet.c:148
-            *a.rebuild = rb;
-            a.out->rebuild = rb;
-            if (rb) a.out->nbuilds += 1;
-            if (a.use_h) cudaGraphSetConditional(a.h, rb ? 1u : 0u);
-            *a.ticket = 0u;
-            rb_s = rb;
-        }
-    }
-    __syncthreads();
-    if (rb_s)
-        for (int k = threadIdx.x; k < a.ncell; k += blockDim.x) a.cell_cnt[k] = 0;
+    check_block(a, m);
+    if (last_block(ticket)) check_last(a);
 }
 
 __global__ void k_force_rebuild(int *rebuild, DevScalars *out) {
@@ -139,24 +58,27 @@ __global__ void k_force_rebuild(int *rebuild, DevScalars *out) {
     out->nbuilds += 1;
 }
 
-void launch_check_list(Engine &e, const cudaGraphConditionalHandle *h) {
+CheckArgs check_args(Engine &e, const cudaGraphConditionalHandle *h) {
     CheckArgs a;
+    a.on = 1;
     a.n = e.n;
     a.ncell = e.ncell;
     a.c = e.cell;
-    a.r = e.d_r;
     a.s = e.d_s;
     a.svl = e.d_svl;
     a.part1 = e.d_part + (size_t)S_DISP1 * e.part_stride;
     a.part2 = e.d_part + (size_t)S_DISP2 * e.part_stride;
-    a.ticket = e.d_ticket + 5;
     a.skindiff = e.p.skindiff;
     a.rebuild = e.d_rebuild;
     a.cell_cnt = e.d_cell_cnt;
     a.out = e.d_out;
     a.h = h ? *h : cudaGraphConditionalHandle{};
     a.use_h = h != nullptr;
-    MDFF_LAUNCH(e, k_check_list, ceil_div(e.n, 256), 256, 0, a);
+    return a;
+}
+
+void launch_check_list(Engine &e, const cudaGraphConditionalHandle *h) {
+    MDFF_LAUNCH(e, k_check_list, ceil_div(e.n, 256), 256, 0, check_args(e, h), e.d_r, e.d_ticket + 5);
 }
 
 // ---------------------------------------------------------------- cell binning

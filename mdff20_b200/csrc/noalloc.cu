@@ -14,7 +14,7 @@
 
 namespace mdffgpu {
 
-__global__ void k_kardir(int n, Cell c, const double4 *r, double4 *s);
+__global__ void k_kardir(int n, Cell c, const double4 *r, double4 *s, double3 *f);
 __global__ void k_bin(int n, int3 nc, const double4 *s, int *cell_of, int *cnt, double4 *svl, const int *rebuild);
 __global__ void k_scan_cells(int ncell, const int *cnt, int *start, int *cur, int cell_cap, unsigned *status,
                              const int *rebuild);
@@ -138,7 +138,7 @@ extern "C" int mdffgpu_build_lists_noalloc(const double *d_pos, int n, const dou
     if (cudaMemsetAsync(P.rebuild, 1, sizeof(int), st) != cudaSuccess) return MDFFGPU_ERR_CUDA;
     int3 g = make_int3(nc[0], nc[1], nc[2]);
     int nb = (n + 255) / 256;
-    k_kardir<<<nb, 256, 0, st>>>(n, c, (const double4 *)d_pos, P.s);
+    k_kardir<<<nb, 256, 0, st>>>(n, c, (const double4 *)d_pos, P.s, (double3 *)nullptr);
     k_bin<<<nb, 256, 0, st>>>(n, g, P.s, P.cell_of, P.cnt, (double4 *)nullptr, P.rebuild);
     k_scan_cells<<<1, 1024, 0, st>>>(ncell, P.cnt, P.start, P.cur, NA_CELL_CAP, P.status, P.rebuild);
     k_fill_cells<<<nb, 256, 0, st>>>(n, P.cell_of, P.start, P.cur, P.ions, P.rebuild);

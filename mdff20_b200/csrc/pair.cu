@@ -3,8 +3,8 @@
 // ion's FULL neighbour list; each lane takes every 32nd neighbour, per-ion sums are
 // combined with warp shuffles and written by lane 0 (no atomics); energies and
 // virials go to per-block partial sums reduced in a fixed order.
-#include "engine.cuh"
 #include "sr_pair.cuh"
+#include "step.cuh"
 
 namespace mdffgpu {
 
@@ -32,13 +32,19 @@ __device__ __forceinline__ void block_partials(const double (&v)[NV], double *pa
 // Buckingham): bhm_pair_fast, the same function with fewer roundings and divisions, in
 // FP64: in FP32 the repulsion A exp(-B r) carries the rounding of r times B r (about 8 at
 // Si-O contact), which measured an 8e-6 relative force error on the bench system.
+// The sums of the slots follow in the last block (fin.ticket set) or in a launch of their own.
+struct SrFin {
+    unsigned *ticket;
+    double *scal;
+    double inveOmegaPU, *u, *pvir, *tau;
+};
 template <bool LJ, bool FAST = false>
 __global__ void __launch_bounds__(PAIR_WARPS * 32, FAST ? 3 : 1) k_sr(int n, Cell c, const double4 *__restrict__ s,
                                                         const int *__restrict__ typ, const PairSR *__restrict__ pr,
                                                         int nt, const int *__restrict__ nbl,
                                                         const int *__restrict__ nbn, int cap, double srcutsq,
                                                         int trunctype, int damped, TT tt, double3 *__restrict__ f,
-                                                        double *__restrict__ part, int slot, int stride) {
+                                                        double *__restrict__ part, int slot, int stride, SrFin fin) {
     grid_dep();
     int i = blockIdx.x * PAIR_WARPS + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
@@ -88,23 +94,57 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32, FAST ? 3 : 1) k_sr(int n, Cel
         for (int k = 0; k < 7; k++) acc[k] = 0.0;
     }
     block_partials<7>(acc, part, slot, stride);
+    if (!fin.ticket) return;
+    const int slots[7] = {slot, slot + 1, slot + 2, slot + 3, slot + 4, slot + 5, slot + 6};
+    if (last_block_warps(part, stride, slots, 7, fin.scal, fin.ticket) && threadIdx.x == 0)
+        finalize_sr(fin.scal, slot, fin.inveOmegaPU, fin.u, fin.pvir, fin.tau);
 }
+
+// the slot sums and their composition in one block, four warps per slot (with one warp per slot
+// 1700 partials took 7.1 us)
+__global__ void __launch_bounds__(896) k_sum_sr(const double *part, int stride, int nparts, int slot, SrFin fin) {
+    grid_dep();
+    __shared__ double sh[28];
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const double *p = part + (size_t)(slot + (w >> 2)) * stride;
+    double a = 0.0;
+#pragma unroll 8
+    for (int k = 32 * (w & 3) + l; k < nparts; k += 128) a += p[k];
+    a = warp_sum(a);
+    if (l == 0) sh[w] = a;
+    __syncthreads();
+    if (threadIdx.x < 7) {
+        const double *q = sh + 4 * threadIdx.x;
+        fin.scal[slot + threadIdx.x] = (q[0] + q[1]) + (q[2] + q[3]);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) finalize_sr(fin.scal, slot, fin.inveOmegaPU, fin.u, fin.pvir, fin.tau);
+}
+
+// whether a pair kernel's last block sums its slots: up to one wave of blocks (n <= 4736), where
+// it saves two launches of 2 us each; with several waves the arrivals of the blocks cost more
+bool sum_in_last(const Engine &e, int blocks) { return blocks <= 4 * e.nsm; }
 
 void launch_sr(Engine &e, bool lj) {
     TT tt = make_tt();
     int nb = ceil_div(e.n, PAIR_WARPS);
+    DevScalars *o = e.d_out;
+    const int slot = lj ? S_LJ_U : S_BH_U;
+    SrFin fin{sum_in_last(e, nb) ? e.d_ticket + 7 : nullptr, e.d_scal, e.cell.inveOmegaPU, lj ? &o->u_lj : &o->u_bh,
+              lj ? &o->pvir_lj : &o->pvir_bh, lj ? o->tau_lj : o->tau_bh};
     if (lj)
         MDFF_LAUNCH(e, k_sr<true>, nb, PAIR_WARPS * 32, 0, e.n, e.cell, e.d_s, e.d_typ, e.d_pair, e.nt, e.d_nb,
                     e.d_nbn, e.cap_nb, e.srcutsq, e.p.trunctype, 0, tt, e.d_f, e.d_part, (int)S_LJ_U,
-                    e.part_stride);
+                    e.part_stride, fin);
     else if (e.use32)
         MDFF_LAUNCH(e, (k_sr<false, true>), nb, PAIR_WARPS * 32, 0, e.n, e.cell, e.d_s, e.d_typ, e.d_pair, e.nt,
                     e.d_nb, e.d_nbn, e.cap_nb, e.srcutsq, e.p.trunctype, e.p.lbhmftd, tt, e.d_f, e.d_part,
-                    (int)S_BH_U, e.part_stride);
+                    (int)S_BH_U, e.part_stride, fin);
     else
         MDFF_LAUNCH(e, k_sr<false>, nb, PAIR_WARPS * 32, 0, e.n, e.cell, e.d_s, e.d_typ, e.d_pair, e.nt, e.d_nb,
                     e.d_nbn, e.cap_nb, e.srcutsq, e.p.trunctype, e.p.lbhmftd, tt, e.d_f, e.d_part, (int)S_BH_U,
-                    e.part_stride);
+                    e.part_stride, fin);
+    if (!fin.ticket) MDFF_LAUNCH(e, k_sum_sr, 1, 896, 0, e.d_part, e.part_stride, nb, slot, fin);
 }
 
 // ---------------------------------------------------------------- real-space Ewald
@@ -133,6 +173,8 @@ struct DirArgs {
     double3 *f;
     double *part;
     int slot, stride;
+    double *scal;
+    unsigned *ticket;            // the last block sums the slots (null: a launch of its own does)
 };
 
 template <bool FORCES, bool EF, bool EFG>
@@ -295,11 +337,16 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32) k_dir(DirArgs a) {
 #pragma unroll
         for (int k = 0; k < 7; k++) acc[k] = 0.0;
     }
-    if (a.part) block_partials<7>(acc, a.part, a.slot, a.stride);
+    if (!a.part) return;
+    block_partials<7>(acc, a.part, a.slot, a.stride);
+    if (!a.ticket) return;
+    const int slots[7] = {a.slot, a.slot + 1, a.slot + 2, a.slot + 3, a.slot + 4, a.slot + 5, a.slot + 6};
+    last_block_warps(a.part, a.stride, slots, 7, a.scal, a.ticket);
 }
 
 void launch_dir(Engine &e, const double *q, const double3 *mu, double alpha, bool lq, bool ld, bool damp,
-                bool forces, bool ef, bool efg, bool efg_q, double3 *out_ef, double *out_efg, double3 *out_f) {
+                bool forces, bool ef, bool efg, bool efg_q, double3 *out_ef, double *out_efg, double3 *out_f,
+                bool energy) {
     const double4 *s = e.d_s;
     DirArgs a;
     a.n = e.n;
@@ -324,16 +371,19 @@ void launch_dir(Engine &e, const double *q, const double3 *mu, double alpha, boo
     a.ef = out_ef;
     a.efg = out_efg;
     a.f = out_f;
-    a.part = e.d_part;
+    int nb = ceil_div(e.n, PAIR_WARPS);
+    a.part = energy ? e.d_part : nullptr;
     a.slot = S_DIR_U;
     a.stride = e.part_stride;
-    int nb = ceil_div(e.n, PAIR_WARPS);
+    a.scal = e.d_scal;
+    a.ticket = energy && sum_in_last(e, nb) ? e.d_ticket + 8 : nullptr;
     if (efg || (ef && forces))
         MDFF_LAUNCH(e, (k_dir<true, true, true>), nb, PAIR_WARPS * 32, 0, a);
     else if (forces)
         MDFF_LAUNCH(e, (k_dir<true, false, false>), nb, PAIR_WARPS * 32, 0, a);
     else
         MDFF_LAUNCH(e, (k_dir<false, true, false>), nb, PAIR_WARPS * 32, 0, a);
+    if (energy && !a.ticket) e.reduce(S_DIR_U, 7, nb);
 }
 
 // ---------------------------------------------------------------- cached dipole field

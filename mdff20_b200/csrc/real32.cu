@@ -210,6 +210,8 @@ struct Dir32bArgs {
     float alpha;
     int lq, ld, ldamp;
     double3 *ef, *f;
+    double *scal;
+    unsigned *ticket;   // the last block sums the slots (null: a launch of its own does)
     double *part;
     int slot, stride;
 };
@@ -391,6 +393,10 @@ __global__ void __launch_bounds__(PW32 * 32) k_dir32b(Dir32bArgs a) {
             for (int k = 0; k < PW32; k++) t += sh[k][threadIdx.x];
             a.part[(size_t)(a.slot + threadIdx.x) * a.stride + blockIdx.x] = t;
         }
+        if (a.ticket) {
+            const int slots[7] = {a.slot, a.slot + 1, a.slot + 2, a.slot + 3, a.slot + 4, a.slot + 5, a.slot + 6};
+            last_block_warps(a.part, a.stride, slots, 7, a.scal, a.ticket);
+        }
     }
 }
 
@@ -479,7 +485,7 @@ static void dir32_launch(Engine &e, const Dir32bArgs &a, int ktt) {
 }
 
 void launch_dir32(Engine &e, const double *q, const double3 *mu, double alpha, bool lq, bool ld, bool damp,
-                  bool forces, bool ef, double3 *out_ef, double3 *out_f, const int *idx, int cnt) {
+                  bool forces, bool ef, double3 *out_ef, double3 *out_f, bool energy, const int *idx, int cnt) {
     if (idx && forces) throw Error(MDFFGPU_ERR_STATE, "ion subsets are for field-only passes");
     (void)q;   // charges travel in the w component of the fractional coordinates
     if (ld) MDFF_LAUNCH(e, k_pack_mu32, ceil_div(e.n, 256), 256, 0, e.n, mu, e.d_typ, e.d_qm32);
@@ -502,15 +508,20 @@ void launch_dir32(Engine &e, const double *q, const double3 *mu, double alpha, b
     a.ldamp = damp;
     a.ef = out_ef;
     a.f = out_f;
-    a.part = e.d_part;
+    const int nb = ceil_div(a.cnt, PW32);
+    energy = energy && forces;
+    a.part = energy ? e.d_part : nullptr;
     a.slot = S_DIR_U;
     a.stride = e.part_stride;
+    a.scal = e.d_scal;
+    a.ticket = energy && sum_in_last(e, nb) ? e.d_ticket + 8 : nullptr;
     int ktt = uniform_tt_order(e);
     int pd = -1;
     e.prof_begin("k_dir", &pd);
     if (forces) dir32_launch<true, false>(e, a, ktt);
     else dir32_launch<false, true>(e, a, ktt);
     e.prof_end("k_dir", pd, 0.0);
+    if (energy && !a.ticket) e.reduce(S_DIR_U, 7, nb);
     (void)ef;
 }
 
