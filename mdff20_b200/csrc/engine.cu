@@ -138,6 +138,8 @@ Engine::Engine(const mdffgpu_params &prm, int dev) : p(prm) {
     d_out = dalloc<DevScalars>(1);
     d_status = (unsigned *)&d_out->status;   // one copy brings both to the host
     d_nhc = dalloc<double>(48);
+    d_rec = dalloc<DevScalars>(STEP_BATCH + 1);
+    d_rec_count = dalloc<int>(1);
     MDFF_CK(cudaMallocHost((void **)&h_out, sizeof(DevScalars)));
     d_soa = dalloc<double>(9 * (size_t)n);
     memset(h_out, 0, sizeof(DevScalars));
@@ -213,6 +215,10 @@ Engine::~Engine() {
     cudaFree(d_out);
     cudaFree(d_ticket);
     if (h_out) cudaFreeHost(h_out);
+    if (h_rec) cudaFreeHost(h_rec);
+    cudaFree(d_rec);
+    cudaFree(d_rec_count);
+    cudaFree(d_snap);
     cudaFree(d_soa);
     if (step_exec) cudaGraphExecDestroy(step_exec);
     if (fit_exec) cudaGraphExecDestroy(fit_exec);
@@ -1434,7 +1440,73 @@ void Engine::capture_step(int step) {
     graph_gen = gen;
 }
 
-// run_md's loop body (src/md.c:229-241)
+// ---------------------------------------------------------------- batches of steps
+// the arrays a step starts from, into one block (or back)
+struct SnapArgs {
+    double *a[8];
+    size_t n[8];
+    int cnt, restore;
+    double *snap;
+    int *rec_count;
+};
+__global__ void __launch_bounds__(256) k_snapshot(SnapArgs s) {
+    grid_dep();
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, T = (size_t)gridDim.x * blockDim.x;
+    if (t == 0) *s.rec_count = 0;
+    double *b = s.snap;
+    for (int k = 0; k < s.cnt; k++) {
+        if (s.restore)
+            for (size_t i = t; i < s.n[k]; i += T) s.a[k][i] = b[i];
+        else
+            for (size_t i = t; i < s.n[k]; i += T) b[i] = s.a[k][i];
+        b += s.n[k];
+    }
+}
+
+void Engine::snapshot(bool restore) {
+    SnapArgs s{};
+    size_t total = 0;
+    auto add = [&](void *p, size_t doubles) {
+        s.a[s.cnt] = (double *)p;
+        s.n[s.cnt++] = doubles;
+        total += doubles;
+    };
+    const size_t N = n;
+    add(d_r, 4 * N);
+    add(d_v, 3 * N);
+    add(d_f, 3 * N);
+    add(d_svl, 4 * N);
+    if (lpol) {
+        add(d_mu_ind, 3 * N);
+        add(d_hist, 3 * ASPC_DEPTH * N);
+    }
+    add(d_nhc, 48);
+    add(d_out, sizeof(DevScalars) / sizeof(double));
+    if (!d_snap) {
+        d_snap = dalloc<double>(total);
+        MDFF_CK(cudaMallocHost((void **)&h_rec, sizeof(DevScalars) * (STEP_BATCH + 1)));
+    }
+    s.restore = restore;
+    s.snap = d_snap;
+    s.rec_count = d_rec_count;
+    MDFF_LAUNCH(*this, k_snapshot, std::min(ceil_div(total, 1024), 2 * nsm), 256, 0, s);
+    if (!restore) return;
+    // the lists of that state, from the positions of their build
+    int nb = 0;
+    MDFF_CK(cudaMemcpyAsync(&nb, &d_out->nbuilds, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    MDFF_CK(cudaMemcpyAsync(d_s, d_svl, sizeof(double4) * N, cudaMemcpyDeviceToDevice, stream));
+    launch_build_lists(*this, true);
+    MDFF_CK(cudaMemcpyAsync(&d_out->nbuilds, &nb, sizeof(int), cudaMemcpyHostToDevice, stream));
+    MDFF_CK(cudaMemsetAsync(d_status, 0, sizeof(unsigned), stream));
+    launch_kardir(*this, d_r, d_s);
+    MDFF_CK(cudaStreamSynchronize(stream));
+}
+
+// run_md's loop body (src/md.c:229-241).  Recorded steps are issued STEP_BATCH at a time and
+// read back together (a step of a few hundred ions takes less than the synchronisation that
+// followed each one).  A step that needs the host (a list that outgrew its capacity) or fails
+// shows in its status word: the batch is then undone and its steps run one by one, so that the
+// error, the state it leaves and the records before it are those of single steps.
 void Engine::md_steps(int first, int nsteps, double *thermo, const double *const *in, double *const *out) {
     if (in) {
         // the caller's positions and velocities, packed on the device (no synchronisation:
@@ -1472,11 +1544,61 @@ void Engine::md_steps(int first, int nsteps, double *thermo, const double *const
         return;
     }
     if (p.lverletL && !list_ready) gen_verletlist();
-    for (int s = 0; s < nsteps; s++) {
-        int step = first + s;
-        bool graphed = graph_ok(step);
+    // the bookkeeping of a recorded step, and a step's thermo record
+    auto counted = [&](const DevScalars &o) {
+        launches += graph_outer + graph_body * std::max(o.scf_iter, 0) + (o.rebuild ? graph_if : 0);
+        if (p.lcoulombic && lpol) {
+            last_scf_iter = o.scf_iter;
+            last_rmsd = o.scf_rmsd;
+        }
+    };
+    auto record = [&](int s, const DevScalars &o) {
+        if (!thermo) return;
+        double *t = thermo + 12 * (size_t)s;
+        t[0] = o.e_kin;
+        t[1] = o.u_lj;
+        t[2] = o.u_bh;
+        t[3] = o.u_coul;
+        t[4] = o.u_pol;
+        t[5] = o.e_nvt;
+        t[6] = o.pvir_lj;
+        t[7] = o.pvir_bh;
+        t[8] = o.pvir_coul;
+        t[9] = (double)o.nbuilds;
+        t[10] = (double)last_scf_iter;
+        t[11] = last_rmsd;
+    };
+    int single_until = 0;   // steps below it run one by one
+    for (int s = 0; s < nsteps;) {
+        const int step = first + s;
+        const bool graphed = graph_ok(step);
+        if (graphed && (!step_exec || graph_gen != gen)) capture_step(step);
+        const int batch = (graphed && p.egrator != 0 && s >= single_until) ? std::min(nsteps - s, STEP_BATCH) : 1;
+        if (batch > 1) {
+            const int istep0 = istep;
+            snapshot(false);
+            for (int b = 0; b < batch; b++) MDFF_CK(cudaGraphLaunch(step_exec, stream));
+            istep = step + batch - 1;
+            if (s + batch == nsteps) queue_out();
+            MDFF_CK(cudaMemcpyAsync(h_rec, d_rec, sizeof(DevScalars) * batch, cudaMemcpyDeviceToHost, stream));
+            sync_scalars();
+            unsigned st = (unsigned)h_out->status;
+            for (int b = 1; b < batch; b++) st |= (unsigned)h_rec[b].status;
+            if (st) {
+                snapshot(true);
+                istep = istep0;
+                single_until = s + batch;
+                continue;
+            }
+            for (int b = 0; b < batch; b++) {
+                const DevScalars &o = b + 1 < batch ? h_rec[b + 1] : *h_out;
+                counted(o);
+                record(s + b, o);
+            }
+            s += batch;
+            continue;
+        }
         if (graphed) {
-            if (!step_exec || graph_gen != gen) capture_step(step);
             istep = step;
             MDFF_CK(cudaGraphLaunch(step_exec, stream));
         } else {
@@ -1486,32 +1608,16 @@ void Engine::md_steps(int first, int nsteps, double *thermo, const double *const
         }
         if (s == nsteps - 1) queue_out();   // on the last step's synchronisation
         sync_scalars();
+        const DevScalars o = *h_out;
         if (graphed) {
-            launches += graph_outer + graph_body * std::max(h_out->scf_iter, 0) + (h_out->rebuild ? graph_if : 0);
-            if (p.lcoulombic && lpol) {
-                last_scf_iter = h_out->scf_iter;
-                last_rmsd = h_out->scf_rmsd;
-            }
-            unsigned st = (unsigned)h_out->status;
+            counted(o);
+            unsigned st = (unsigned)o.status;
             if (st & ST_SCF) throw Error(MDFFGPU_ERR_SCF, "CG did not converge in max_scf_pim_iter");
             if (st & ST_LIST_OVERFLOW) gen_verletlist();   // positions unchanged: rebuild larger
         }
         check_status();
-        if (thermo) {
-            double *t = thermo + 12 * (size_t)s;
-            t[0] = h_out->e_kin;
-            t[1] = h_out->u_lj;
-            t[2] = h_out->u_bh;
-            t[3] = h_out->u_coul;
-            t[4] = h_out->u_pol;
-            t[5] = h_out->e_nvt;
-            t[6] = h_out->pvir_lj;
-            t[7] = h_out->pvir_bh;
-            t[8] = h_out->pvir_coul;
-            t[9] = (double)h_out->nbuilds;
-            t[10] = (double)last_scf_iter;
-            t[11] = last_rmsd;
-        }
+        record(s, o);
+        s++;
     }
 }
 

@@ -61,6 +61,9 @@ struct DevScalars {
     int scf_iter, nbuilds, rebuild, status;
 };
 
+// steps issued without a host synchronisation between them (Engine::md_steps)
+constexpr int STEP_BATCH = 16;
+
 // the stopping test of a recorded CG loop, evaluated by the last block of k_cg_step (or by
 // k_cg_test before the first iteration): mode 1, the induced-dipole test
 // rmsd = sqrt(r.r / npol) > tol (the reference's residual measure, src/pim.c:431-449);
@@ -385,6 +388,12 @@ struct Engine {
     unsigned *d_status = nullptr;
     unsigned *d_ticket = nullptr;   // block-arrival counters of kernels that finish their own reductions
     double *d_nhc = nullptr;     // xi[16], vxi[16], Q[16]
+    // a batch of recorded steps: the results of each step but the last, written by the next
+    // step's first kernel (entry 0: those before the batch), and the state it started from
+    DevScalars *d_rec = nullptr, *h_rec = nullptr;
+    int *d_rec_count = nullptr;
+    double *d_snap = nullptr;
+    void snapshot(bool restore);
 
     // per-kernel timing of one chosen kernel family (CUDA events on `stream`)
     std::string prof_name;

@@ -383,6 +383,8 @@ struct StepArgs {
     int stride;
     unsigned *ticket, *status;
     DevScalars *out;
+    DevScalars *rec;             // results of the steps before this one (StepBatch)
+    int *rec_count;
 };
 static StepArgs step_args(Engine &e) {
     StepArgs a;
@@ -402,7 +404,24 @@ static StepArgs step_args(Engine &e) {
     a.ticket = e.d_ticket + 6;
     a.status = e.d_status;
     a.out = e.d_out;
+    a.rec = e.d_rec;
+    a.rec_count = e.d_rec_count;
     return a;
+}
+
+// block 0 of a step's first kernel: the results of the step before it into the record (the
+// steps of a batch are read back together), then the status word cleared
+__device__ __forceinline__ void open_step(const StepArgs &a) {
+    if (blockIdx.x) return;
+    const int k = min(*a.rec_count, STEP_BATCH);
+    static_assert(sizeof(DevScalars) % sizeof(double) == 0, "copied by doubles");
+    for (int w = threadIdx.x; w < (int)(sizeof(DevScalars) / sizeof(double)); w += blockDim.x)
+        ((double *)(a.rec + k))[w] = ((const double *)a.out)[w];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *a.rec_count = k + 1;
+        *a.status = 0u;
+    }
 }
 
 // the new position of an ion: stored, its fractional coordinates, zeroed force
@@ -417,7 +436,7 @@ __device__ __forceinline__ void open_ion(const StepArgs &a, int i, double4 x) {
 __global__ void __launch_bounds__(256) k_vv1(StepArgs a) {
     grid_dep();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) *a.status = 0u;
+    open_step(a);
     if (i >= a.n) return;
     const double dt = a.dt, dtsq2 = dt * dt * 0.5;
     double4 x = a.r[i];
@@ -533,7 +552,7 @@ __global__ void __launch_bounds__(256) k_kin_chain(StepArgs a, NhcArgs h) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const double dt2 = a.dt * 0.5;
     double k[1] = {0.0};
-    if (!KICK && i == 0) *a.status = 0u;
+    if (!KICK) open_step(a);
     if (i < a.n) {
         double3 vv = a.v[i];
         if (KICK) {
