@@ -45,9 +45,13 @@ void download(Engine &e, void *dst, const void *src, size_t bytes) {
 
 }  // namespace
 
-// ions from which the mixed k space runs on the tensor cores by default (the batched fit's
-// configurations of 96 to 1536 ions evaluate faster on the CUDA-core passes)
+// ions from which the mixed k space runs on the tensor cores by default
 constexpr int TC_MIN_IONS = 4096;
+// ions below which it runs in FP64 (kspace64.cu: matrix instructions at half the FP32 rate, but
+// two launches fewer per pass and no table of its own): polarisable MD, 10 steps, FP32 on CUDA
+// cores against FP64: 192 ions 2885 / 2126 us, 648 ions 2187 / 1725, 1536 ions 2740 / 2580, 3000
+// ions 3396 / 3429
+constexpr int REC64_IONS = 2048;
 
 struct mdffgpu_fit_plan {
     std::vector<mdffgpu_ctx *> ctx;
@@ -138,9 +142,10 @@ int mdffgpu_set_precision(mdffgpu_ctx *ctx, int precision) {
         }
         if (const char *v = getenv("MDFFGPU_PIM_SUBSET")) e.subset32 = atoi(v) != 0;
         // the rho and ion passes on the tensor cores (kspace_tc.cu, kspace_ion_tc.cu) from
-        // TC_MIN_IONS ions on; below, where a pass is a few microseconds, the CUDA-core passes
-        // (fewer kernels per pass).  MDFFGPU_RHO_TC / MDFFGPU_ION_TC = 0 / 1 override.
+        // TC_MIN_IONS ions on, on CUDA cores below, in FP64 below REC64_IONS; MDFFGPU_RHO_TC /
+        // MDFFGPU_ION_TC = 1 or 0 select the tensor-core or the CUDA-core FP32 pass at any size
         e.rho_tc = e.ion_tc = e.n >= TC_MIN_IONS;
+        e.rec64 = e.n < REC64_IONS && !getenv("MDFFGPU_RHO_TC") && !getenv("MDFFGPU_ION_TC");
         if (const char *v = getenv("MDFFGPU_RHO_TC")) e.rho_tc = atoi(v) != 0;
         if (const char *v = getenv("MDFFGPU_ION_TC")) e.ion_tc = atoi(v) != 0;
     });
@@ -355,7 +360,7 @@ int mdffgpu_get_dipoles(mdffgpu_ctx *ctx, double *mu, double *upol) {
         if (!e.p.lcoulombic) throw Error(MDFFGPU_ERR_STATE, "lcoulombic is not set");
         e.ensure_lists();
         mdffgpu::launch_kardir(e, e.d_r, e.d_s);
-        if (e.use32) mdffgpu::launch_coords32(e);
+        if (e.use32 && e.rec32 && !e.rec64) mdffgpu::launch_coords32(e);
         e.get_dipoles();
         e.sync_scalars();
         if (mu) download(e, mu, e.d_mu_tot, sizeof(double3) * e.n);

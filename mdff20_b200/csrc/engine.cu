@@ -760,9 +760,11 @@ void Engine::tune_launch(int reps, int *choice, double *ms) {
     if (!(use32 && real32 && rec32 && p.lcoulombic && lpol && npol > 0))
         throw Error(MDFFGPU_ERR_STATE, "launch tuning applies to the mixed-precision polarisable k space");
     reps = std::max(reps, 1);
+    const bool by64 = rec64;   // the default of few ions: one more candidate
+    rec64 = false;
     engforce();
     struct Cand {
-        int tc, chunks, slices, rtc;
+        int tc, chunks, slices, rtc, f64 = 0;
     };
     std::vector<int> chunk_set;
     for (int c : {std::max(1, rho32_chunks / 2), rho32_chunks, std::min(rho32_chunks_max, 2 * rho32_chunks)})
@@ -785,9 +787,11 @@ void Engine::tune_launch(int reps, int *choice, double *ms) {
             cudaEventDestroy(b);
         }
     } evs{t0, t1};
+    if (by64) cands.push_back({0, rho32_chunks, 0, 0, 1});
     Cand best{ion_tc ? 1 : 0, rho32_chunks, ion_tc_slices_set, rho_tc ? 1 : 0};
     double best_ms = 1e300;
     auto apply = [&](const Cand &c) {
+        rec64 = c.f64 != 0;
         ion_tc = c.tc != 0;
         rho32_chunks = c.chunks;
         ion_tc_slices_set = c.slices;
@@ -815,7 +819,7 @@ void Engine::tune_launch(int reps, int *choice, double *ms) {
     gen++;   // recorded steps use the chosen shapes from now on
     if (choice) {
         choice[0] = best.tc;
-        choice[1] = best.rtc ? 0 : best.chunks;
+        choice[1] = best.rtc ? 0 : best.chunks;   // (the FP64 passes report as the CUDA-core ones)
         choice[2] = best.slices;
         choice[3] = best.rtc;
     }
@@ -1233,7 +1237,7 @@ void Engine::engforce(bool check_finite, bool opened) {
         on_side(SIDE_PREP, [&] { launch_pair_prep32(*this); });
         prep_issued = true;
     }
-    if (use32) launch_coords32(*this);
+    if (use32 && rec32 && !rec64) launch_coords32(*this);
     if (p.lcoulombic) {
         rho_acc_ready = false;
         get_dipoles();
@@ -1271,7 +1275,7 @@ void Engine::multipole_es_dev(const double *d_qv, const double3 *d_muv, double a
     bool efg = flags & MDFFGPU_ES_EFG, dir = flags & MDFFGPU_ES_DIR, rec = flags & MDFFGPU_ES_REC;
     ensure_lists();
     launch_kardir(*this, d_r, d_s);
-    if (use32) launch_coords32(*this);
+    if (use32 && rec32 && !rec64) launch_coords32(*this);
     int nb = ceil_div(n, 256);
     double self2 = self2_of(alpha);
     // efg_dir accumulates the charge part when do_efg and the dipole part when do_efg

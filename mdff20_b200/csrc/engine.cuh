@@ -321,6 +321,7 @@ struct Engine {
     // parts of the mixed path (all on by default; MDFFGPU_MIXED_PARTS=real|rec keeps
     // only that part in FP32, MDFFGPU_PIM_SUBSET=0 runs the CG field over all ions)
     bool real32 = true, rec32 = true, subset32 = true;
+    bool rec64 = false;          // mixed precision with few ions: the k space in FP64 all the same
     // mixed-precision real space (real32.cu), sized like the Coulomb list
     int *d_nl32 = nullptr, *d_nln32 = nullptr;   // in-cutoff neighbours [n][cap32]
     int *d_pl32 = nullptr, *d_pln32 = nullptr;   // polarisable neighbours of polarisable ions

@@ -137,8 +137,8 @@ static void launch_rec32(Engine &e, const double *q, const double3 *mu, bool lq,
 }
 
 void launch_rec(Engine &e, const double *q, const double3 *mu, bool lq, bool ld, const RecOut &o) {
-    // FP32 passes in mixed precision (no FP32 EFG: EFG requests run in FP64)
-    if (e.use32 && e.rec32 && o.efg == nullptr) {
+    // FP32 passes in mixed precision (no FP32 EFG: EFG requests run in FP64, as do few ions)
+    if (e.use32 && e.rec32 && !e.rec64 && o.efg == nullptr) {
         launch_rec32(e, q, mu, lq, ld, o);
         return;
     }
