@@ -207,6 +207,8 @@ Engine::~Engine() {
     cudaFree(d_ion_wtab);
     cudaFree(d_ion_part);
     cudaFree(d_coef);
+    cudaFree(d_pcol);
+    cudaFree(d_pcon);
     dfree32();
     for (void *x : {(void *)d_fpart, (void *)d_fscal, (void *)d_w, (void *)d_lam, (void *)d_sv, (void *)d_fa,
                     (void *)d_fb, (void *)d_fc, (void *)d_qw, (void *)d_efg_rec, (void *)d_muw, (void *)d_rw,
@@ -546,7 +548,13 @@ void Engine::alloc_lists(int cnb, int cco) {
     d_co = dalloc<int>((size_t)n * cap_co);
     d_con = dalloc<int>(n);
     dfree(d_coef);
-    if (p.lcoulombic && lpol) d_coef = dalloc<double2>((size_t)n * cap_co);
+    dfree(d_pcol);
+    dfree(d_pcon);
+    if (p.lcoulombic && lpol) {
+        d_coef = dalloc<double2>((size_t)n * cap_co);
+        d_pcol = dalloc<int>((size_t)n * cap_co);
+        d_pcon = dalloc<int>(n);
+    }
     list_ready = false;
     coef_ready = false;
 }

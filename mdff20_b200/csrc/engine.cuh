@@ -316,7 +316,9 @@ struct Engine {
     // ---- neighbour lists (full lists, row-major [n][cap])
     int cap_nb = 0, cap_co = 0;
     int *d_nb = nullptr, *d_nbn = nullptr, *d_co = nullptr, *d_con = nullptr;
-    double2 *d_coef = nullptr;   // [n][cap_co] cached dipole-field pair factors
+    double2 *d_coef = nullptr;   // [n][cap_co] cached dipole-field pair factors (k_dir_prep) ...
+    int *d_pcol = nullptr;       // ... of the polarisable pairs inside the cut-off, d_pcon[i] per ion
+    int *d_pcon = nullptr;
     bool use32 = false;          // mixed precision: FP32 Ewald kernels
     // parts of the mixed path (all on by default; MDFFGPU_MIXED_PARTS=real|rec keeps
     // only that part in FP32, MDFFGPU_PIM_SUBSET=0 runs the CG field over all ions)

@@ -3,6 +3,7 @@
 // ion's FULL neighbour list; each lane takes every 32nd neighbour, per-ion sums are
 // combined with warp shuffles and written by lane 0 (no atomics); energies and
 // virials go to per-block partial sums reduced in a fixed order.
+#include "pairq.cuh"
 #include "sr_pair.cuh"
 #include "step.cuh"
 
@@ -177,6 +178,15 @@ struct DirArgs {
     unsigned *ticket;            // the last block sums the slots (null: a launch of its own does)
 };
 
+//
+// Bound by the FP64 pipe and the latency of its long dependent chains (128 registers: 16 warps
+// per SM): per pair one reciprocal square root, one exponential, one erfc and up to two
+// Tang-Toennies functions.  Pairs are taken in full groups of 32 from the queue of pairq.cuh,
+// divisions by d^2 are products, a damping function is evaluated only where it enters (a zero
+// dipole or c = 0 leaves it out exactly), energy and virial only when asked for.  6000 ions, cut
+// off 10 + 1 A: forces 118 -> 84 us, field 89 -> 64; 3000 ions 73 -> 55 and 56 -> 43.  A third
+// block per SM (80 registers, 240 bytes spilled) took the forces to 112 us; erfcx times the
+// exponential at hand in place of erfc changed nothing (82.6 / 61.4 us).
 template <bool FORCES, bool EF, bool EFG>
 __global__ void __launch_bounds__(PAIR_WARPS * 32) k_dir(DirArgs a) {
     grid_dep();
@@ -185,47 +195,39 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32) k_dir(DirArgs a) {
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};   // u, V6
     double fi[3] = {0, 0, 0}, ei[3] = {0, 0, 0};
     double gi[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const double alpha = a.alpha, alpha2 = alpha * alpha, alpha3 = alpha2 * alpha, alpha5 = alpha3 * alpha2;
-    const double rpi = 1.7724538509055160273;  // sqrt(pi), src/constants.c:20
+    const bool en = a.part != nullptr;   // energy and virial wanted
+    __shared__ PairQ queue[PAIR_WARPS];
     if (i < a.n) {
         double4 si = a.s[i];
         double qi = a.lq ? a.q[i] : 0.0;
         double3 mi = a.ld ? a.mu[i] : make_double3(0, 0, 0);
         bool dip_i = (mi.x != 0.0) || (mi.y != 0.0) || (mi.z != 0.0);
         int ti = a.typ[i];
-        int m = a.con[i];
-        if (m > a.cap) m = a.cap;
-        const int *L = a.col + (size_t)i * a.cap;
-        for (int k = lane; k < m; k += 32) {
-            int j = L[k];
-            double4 sj = a.s[j];
-            double3 r = pbc_frac(a.c, dsub(si.x, sj.x), dsub(si.y, sj.y), dsub(si.z, sj.z));
-            double d2 = norm2_exact(r);
-            if (d2 > a.lrcutsq) continue;
+        auto pair = [&](int j, const double3 &r, double d2) {
             double qj = a.lq ? a.q[j] : 0.0;
             double3 mj = a.ld ? a.mu[j] : make_double3(0, 0, 0);
             bool dip_j = (mj.x != 0.0) || (mj.y != 0.0) || (mj.z != 0.0);
-            double d = sqrt(d2), d3 = d2 * d, d5 = d3 * d2;
-            double dm1 = 1.0 / d, dm3 = dm1 / d2, dm5 = dm3 / d2, dm7 = dm5 / d2;
-            double expon = exp(-alpha2 * d2) / rpi;
-            double F0 = erfc(alpha * d);
-            double F1 = F0 + 2.0 * alpha * d * expon;
-            double F2 = F1 + 4.0 * alpha3 * d3 * expon / 3.0;
-            double F3 = F2 + 8.0 * alpha5 * d5 * expon / 15.0;
-            // Tang-Toennies damping of the charge->dipole field, src/ewald.c:505-539
+            const Screened v = screened(d2, a.alpha);
+            const double d = v.d, dm1 = v.dm1, dm3 = v.dm3, dm5 = v.dm5, F0 = v.F0, F1 = v.F1, F2 = v.F2;
+            // Tang-Toennies damping of the charge->dipole field, src/ewald.c:505-539: of the charge j
+            // at i's dipole (1; the field at any i) and of the charge i at j's dipole (2)
             double F1d1 = 0.0, F1d2 = 0.0, F2d1 = 0.0, F2d2 = 0.0;
             bool damp = false;
-            if (a.ldamp) {
+            if (a.ldamp && a.lq) {
                 const PairDamp &D = a.damp[ti * a.nt + a.typ[j]];
                 if (D.ldamp) {
                     damp = true;
-                    double fd1, fdd1, fd2, fdd2;
-                    tt_damp(a.tt, D.b1, D.c1, d, D.k1, fd1, fdd1);
-                    tt_damp(a.tt, D.b2, D.c2, d, D.k2, fd2, fdd2);
-                    F1d1 = -fd1 + 1.0;
-                    F1d2 = -fd2 + 1.0;
-                    F2d1 = F1d1 + (d / 3.0) * fdd1;
-                    F2d2 = F1d2 + (d / 3.0) * fdd2;
+                    double f, fd;
+                    if ((EF || dip_i) && D.c1 != 0.0) {   // (c = 0: f = 1)
+                        tt_damp(a.tt, D.b1, D.c1, d, D.k1, f, fd);
+                        F1d1 = 1.0 - f;
+                        F2d1 = F1d1 + d * (1.0 / 3.0) * fd;
+                    }
+                    if (dip_j && D.c2 != 0.0) {
+                        tt_damp(a.tt, D.b2, D.c2, d, D.k2, f, fd);
+                        F1d2 = 1.0 - f;
+                        F2d2 = F1d2 + d * (1.0 / 3.0) * fd;
+                    }
                 }
             }
             double F1_dm3 = F1 * dm3, F2_dm5 = 3.0 * F2 * dm5;
@@ -264,7 +266,10 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32) k_dir(DirArgs a) {
                     ei[1] += F2_dm5 * rmj * r.y - F1_dm3 * mj.y;
                     ei[2] += F2_dm5 * rmj * r.z - F1_dm3 * mj.z;
                 }
-                double F3_dm7 = F3 * dm7 * 15.0;
+                // F3 = F2 + 8 (alpha d)^5 exp / 15
+                const double ad2 = a.alpha * a.alpha * d2;
+                const double F3_dm7 =
+                    (15.0 * F2 + 8.0 * (ad2 * ad2 * a.alpha * d) * v.ex) * (dm5 * dm1 * dm1);
                 if (FORCES) {
                     double c1 = -F3_dm7 * rmi * rmj, c2 = F2_dm5;
                     fij[0] -= c1 * r.x + c2 * (mm * r.x + mi.x * rmj + mj.x * rmi);
@@ -304,20 +309,26 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32) k_dir(DirArgs a) {
                 fi[0] -= fij[0];
                 fi[1] -= fij[1];
                 fi[2] -= fij[2];
-                acc[0] += u;
-                acc[1] += -(r.x * fij[0] + r.x * fij[0]);
-                acc[2] += -(r.x * fij[1] + r.y * fij[0]);
-                acc[3] += -(r.x * fij[2] + r.z * fij[0]);
-                acc[4] += -(r.y * fij[1] + r.y * fij[1]);
-                acc[5] += -(r.y * fij[2] + r.z * fij[1]);
-                acc[6] += -(r.z * fij[2] + r.z * fij[2]);
-            } else {
-                acc[0] += u;
             }
-        }
+            if (en) {
+                acc[0] += u;
+                if (FORCES) {
+                    acc[1] += -(r.x * fij[0] + r.x * fij[0]);
+                    acc[2] += -(r.x * fij[1] + r.y * fij[0]);
+                    acc[3] += -(r.x * fij[2] + r.z * fij[0]);
+                    acc[4] += -(r.y * fij[1] + r.y * fij[1]);
+                    acc[5] += -(r.y * fij[2] + r.z * fij[1]);
+                    acc[6] += -(r.z * fij[2] + r.z * fij[2]);
+                }
+            }
+        };
+        pairs_in_cut<false>(a.c, a.s, si, a.col + (size_t)i * a.cap, min(a.con[i], a.cap), a.lrcutsq,
+                            queue[threadIdx.x >> 5], pair);
     }
+    if (en) {
 #pragma unroll
-    for (int k = 0; k < 7; k++) acc[k] = warp_sum(acc[k]);
+        for (int k = 0; k < 7; k++) acc[k] = warp_sum(acc[k]);
+    }
     if (FORCES) {
         for (int k = 0; k < 3; k++) fi[k] = warp_sum(fi[k]);
     }
@@ -389,45 +400,44 @@ void launch_dir(Engine &e, const double *q, const double3 *mu, double alpha, boo
 // ---------------------------------------------------------------- cached dipole field
 // Within one force evaluation the positions are fixed while the induced dipoles are
 // iterated (src/pim.c:236-278), so the screened pair factors F1/d^3 and 3 F2/d^5 of
-// the dipole field (the T2 tensor, src/ewald.c:581-603) are computed once per list
-// entry and reused by every iteration: the iteration kernel then does no erfc/exp.
+// the dipole field (the T2 tensor, src/ewald.c:581-603) are computed once per pair
+// and reused by every iteration: the iteration kernel then does no erfc/exp.  Induced dipoles
+// sit on polarisable ions and act on those only, so the records are the pairs of polarisable
+// ions inside the cut-off, in list order: pcol, pcon and coef.  Bound by the FP64 pipe (prep) and
+// by the gathers of 88 bytes per pair from L2 (field).  6000 ions, silica, cut-off 10 + 1 A, against
+// factors for every list entry (three per record): prep 47 -> 22 us, field 18 -> 11 us; 3000 ions
+// prep 25 -> 12, field 13 -> 6.
 __global__ void __launch_bounds__(PAIR_WARPS * 32) k_dir_prep(int n, Cell c, const double4 *__restrict__ s,
+                                                             const int *__restrict__ polar,
                                                              const int *__restrict__ col,
                                                              const int *__restrict__ con, int cap, double lrcutsq,
-                                                             double alpha, double2 *__restrict__ coef) {
+                                                             double alpha, int *__restrict__ pcol,
+                                                             int *__restrict__ pcon, double2 *__restrict__ coef) {
     grid_dep();
     int i = blockIdx.x * PAIR_WARPS + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
     if (i >= n) return;
-    const double rpi = 1.7724538509055160273;
-    const double alpha2 = alpha * alpha, alpha3 = alpha2 * alpha;
-    double4 si = s[i];
-    int m = min(con[i], cap);
-    const int *L = col + (size_t)i * cap;
-    double2 *C = coef + (size_t)i * cap;
-    for (int k = lane; k < m; k += 32) {
-        double4 sj = s[L[k]];
-        double3 r = pbc_frac(c, dsub(si.x, sj.x), dsub(si.y, sj.y), dsub(si.z, sj.z));
-        double d2 = norm2_exact(r);
-        double2 out = make_double2(0.0, 0.0);
-        if (!(d2 > lrcutsq)) {
-            double d = sqrt(d2), d3 = d2 * d;
-            double dm1 = 1.0 / d, dm3 = dm1 / d2, dm5 = dm3 / d2;
-            double expon = exp(-alpha2 * d2) / rpi;
-            double F0 = erfc(alpha * d);
-            double F1 = F0 + 2.0 * alpha * d * expon;
-            double F2 = F1 + 4.0 * alpha3 * d3 * expon / 3.0;
-            out = make_double2(F1 * dm3, 3.0 * F2 * dm5);
-        }
-        C[k] = out;
+    int cnt = 0;
+    if (polar[i]) {
+        __shared__ PairQ queue[PAIR_WARPS];
+        int *P = pcol + (size_t)i * cap;
+        double2 *C = coef + (size_t)i * cap;
+        pairs_in_cut<false>(c, s, s[i], col + (size_t)i * cap, min(con[i], cap), lrcutsq, queue[threadIdx.x >> 5],
+                            [&](int j) { return polar[j] != 0; }, cnt,
+                            [&](int at, int j, const double3 &, double d2) {
+                                const Screened v = screened(d2, alpha);
+                                P[at] = j;
+                                C[at] = make_double2(v.F1 * v.dm3, 3.0 * v.F2 * v.dm5);
+                            });
     }
+    if (lane == 0) pcon[i] = cnt;
 }
 
 // field of the dipoles mu from the cached factors: E_i = sum_j (3F2/d^5 (r.mu_j) r - F1/d^3 mu_j),
 // only when mu_i and mu_j are non-zero (src/ewald.c:737-749)
 __global__ void __launch_bounds__(PAIR_WARPS * 32) k_dir_field_cached(int n, Cell c, const double4 *__restrict__ s,
-                                                                     const int *__restrict__ col,
-                                                                     const int *__restrict__ con, int cap,
+                                                                     const int *__restrict__ pcol,
+                                                                     const int *__restrict__ pcon, int cap,
                                                                      const double2 *__restrict__ coef,
                                                                      const double3 *__restrict__ mu,
                                                                      double3 *__restrict__ ef) {
@@ -435,26 +445,28 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32) k_dir_field_cached(int n, Cel
     int i = blockIdx.x * PAIR_WARPS + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
     if (i >= n) return;
-    double3 mi = mu[i];
-    bool dip_i = (mi.x != 0.0) || (mi.y != 0.0) || (mi.z != 0.0);
     double ex = 0.0, ey = 0.0, ez = 0.0;
-    if (dip_i) {
-        double4 si = s[i];
-        int m = min(con[i], cap);
-        const int *L = col + (size_t)i * cap;
-        const double2 *C = coef + (size_t)i * cap;
-        for (int k = lane; k < m; k += 32) {
-            double2 cf = C[k];
-            if (cf.x == 0.0 && cf.y == 0.0) continue;
-            int j = L[k];
-            double3 mj = mu[j];
-            if (mj.x == 0.0 && mj.y == 0.0 && mj.z == 0.0) continue;
-            double4 sj = s[j];
-            double3 r = pbc_frac(c, dsub(si.x, sj.x), dsub(si.y, sj.y), dsub(si.z, sj.z));
-            double rmj = r.x * mj.x + r.y * mj.y + r.z * mj.z;
-            ex += cf.y * rmj * r.x - cf.x * mj.x;
-            ey += cf.y * rmj * r.y - cf.x * mj.y;
-            ez += cf.y * rmj * r.z - cf.x * mj.z;
+    const int m = pcon[i];
+    if (m > 0) {
+        double3 mi = mu[i];
+        if ((mi.x != 0.0) || (mi.y != 0.0) || (mi.z != 0.0)) {
+            double4 si = s[i];
+            const int *L = pcol + (size_t)i * cap;
+            const double2 *C = coef + (size_t)i * cap;
+            int jn = lane < m ? L[lane] : 0;
+#pragma unroll 2
+            for (int k = lane; k < m; k += 32) {
+                const int j = jn;
+                if (k + 32 < m) jn = L[k + 32];
+                const double2 cf = C[k];
+                const double3 mj = mu[j];
+                const double4 sj = s[j];
+                const double3 r = pbc_frac(c, dsub(si.x, sj.x), dsub(si.y, sj.y), dsub(si.z, sj.z));
+                const double rmj = r.x * mj.x + r.y * mj.y + r.z * mj.z;
+                ex += cf.y * rmj * r.x - cf.x * mj.x;
+                ey += cf.y * rmj * r.y - cf.x * mj.y;
+                ez += cf.y * rmj * r.z - cf.x * mj.z;
+            }
         }
     }
     ex = warp_sum(ex);
@@ -465,15 +477,15 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32) k_dir_field_cached(int n, Cel
 
 void launch_dir_prep(Engine &e, double alpha) {
     int nb = ceil_div(e.n, PAIR_WARPS);
-    MDFF_LAUNCH(e, k_dir_prep, nb, PAIR_WARPS * 32, 0, e.n, e.cell, e.d_s, e.d_co, e.d_con, e.cap_co, e.lrcutsq,
-                alpha, e.d_coef);
+    MDFF_LAUNCH(e, k_dir_prep, nb, PAIR_WARPS * 32, 0, e.n, e.cell, e.d_s, e.d_polar, e.d_co, e.d_con, e.cap_co,
+                e.lrcutsq, alpha, e.d_pcol, e.d_pcon, e.d_coef);
 }
 
 void launch_dir_field_cached(Engine &e, const double3 *mu, double3 *out_ef) {
     int nb = ceil_div(e.n, PAIR_WARPS);
     int pd = -1;
     e.prof_begin("k_dir", &pd);
-    MDFF_LAUNCH(e, k_dir_field_cached, nb, PAIR_WARPS * 32, 0, e.n, e.cell, e.d_s, e.d_co, e.d_con, e.cap_co,
+    MDFF_LAUNCH(e, k_dir_field_cached, nb, PAIR_WARPS * 32, 0, e.n, e.cell, e.d_s, e.d_pcol, e.d_pcon, e.cap_co,
                 e.d_coef, mu, out_ef);
     e.prof_end("k_dir", pd, 0.0);
 }
