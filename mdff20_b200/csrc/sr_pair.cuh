@@ -38,39 +38,21 @@ __device__ __forceinline__ void tt_damp(const TT &tt, double b, double c, double
     fd = tt.E[order] * powi(br, order) * ex * b;
 }
 
-// pair energy u and w = -(du/dr)/r of one pair at squared distance r2 (inside the cut-off)
-template <bool LJ>
-__device__ __forceinline__ void sr_pair(const PairSR &P, double r2, int trunctype, int damped, const TT &tt,
-                                        double &u, double &w) {
-    if (LJ) {
-        double sr2 = P.sigsq / r2;
-        double srp = P.ip >= 0 ? powi(sr2, P.ip) : pow(sr2, P.ptwo);
-        double srq = P.iq >= 0 ? powi(sr2, P.iq) : pow(sr2, P.qtwo);
-        u = (trunctype == 2) ? 0.0 : P.epsqp * (P.plj * srq - P.qlj * srp) - (trunctype == 1 ? P.uc : 0.0);
-        w = P.fc * (srq - srp) * sr2;
-    } else {
-        double ir2 = 1.0 / r2, d = sqrt(r2);
-        double erh = P.A * exp(-P.B * d);
-        double ir6 = ir2 * ir2 * ir2, ir8 = ir6 * ir2;
-        ir6 *= P.C;
-        ir8 *= P.D;
-        double f6 = 1.0, f8 = 1.0, fd6 = 0.0, fd8 = 0.0;
-        if (damped) {
-            tt_damp(tt, P.BD, 1.0, d, 6, f6, fd6);
-            tt_damp(tt, P.BD, 1.0, d, 8, f8, fd8);
-        }
-        double ir6d = ir6 * f6, ir8d = ir8 * f8;
-        double ir7 = 6.0 * ir6d / d, ir9 = 8.0 * ir8d / d;
-        u = erh - ir6d - ir8d;
-        w = (P.B * erh - ir7 - ir9 + ir6 * fd6 + ir8 * fd8) / d;
-    }
+// n-m Lennard-Jones: pair energy u and w = -(du/dr)/r of one pair at squared distance r2 (inside
+// the cut-off)
+__device__ __forceinline__ void lj_pair(const PairSR &P, double r2, int trunctype, double &u, double &w) {
+    double sr2 = P.sigsq / r2;
+    double srp = P.ip >= 0 ? powi(sr2, P.ip) : pow(sr2, P.ptwo);
+    double srq = P.iq >= 0 ? powi(sr2, P.iq) : pow(sr2, P.qtwo);
+    u = (trunctype == 2) ? 0.0 : P.epsqp * (P.plj * srq - P.qlj * srp) - (trunctype == 1 ? P.uc : 0.0);
+    w = P.fc * (srq - srp) * sr2;
 }
 
-// BHMFT(D) pair term of sr_pair<false> with shared subexpressions, for the mixed-precision
-// path: one FP64 reciprocal square root in place of the square root and four divisions,
-// and one Tang-Toennies exponential and one set of powers of b r for both dispersion
-// orders (f8's polynomial is f6's plus the k = 7, 8 terms).  Same function, other roundings.
-__device__ __forceinline__ void bhm_pair_fast(const PairSR &P, double r2, int damped, double &u, double &w) {
+// BHMFT(D), the same of A exp(-B d) - C f6 / d^6 - D f8 / d^8: one FP64 reciprocal square root in
+// place of the square root and four divisions, and one Tang-Toennies exponential and one set
+// of powers of b r for both dispersion orders (f8's polynomial is f6's plus the k = 7, 8 terms):
+// k_sr of 6000 ions 23.5 -> 15.4 us in FP64 precision, where each was evaluated on its own.
+__device__ __forceinline__ void bhm_pair(const PairSR &P, double r2, int damped, double &u, double &w) {
     constexpr double E6 = 1.0 / 720.0, E7 = 1.0 / 5040.0, E8 = 1.0 / 40320.0;
     double id = rsqrt(r2), d = r2 * id, ir2 = id * id;
     double erh = P.A * exp(-P.B * d);
