@@ -29,22 +29,22 @@ __device__ __forceinline__ void block_partials(const double (&v)[NV], double *pa
 // ---------------------------------------------------------------- short range
 // engforce_nmlj_pbc (src/nmlj.c:254-385) when LJ, engforce_bhmftd_pbc
 // (src/bhmftd.c:117-271) otherwise.  Adds forces into f; slot gets u (x2) and the
-// virial sum over the full list of (r_a f_b + r_b f_a).  FAST (mixed precision,
-// Buckingham): bhm_pair_fast, the same function with fewer roundings and divisions, in
-// FP64: in FP32 the repulsion A exp(-B r) carries the rounding of r times B r (about 8 at
-// Si-O contact), which measured an 8e-6 relative force error on the bench system.
+// virial sum over the full list of (r_a f_b + r_b f_a).  (The queue of pairq.cuh does not pay
+// here: 24000 ions 45 us without, 56 with.)  FP64 in mixed precision too: in FP32 the
+// repulsion A exp(-B r) carries the rounding of r times B r (about 8 at Si-O contact), which
+// measured an 8e-6 relative force error on the bench system.
 // The sums of the slots follow in the last block (fin.ticket set) or in a launch of their own.
 struct SrFin {
     unsigned *ticket;
     double *scal;
     double inveOmegaPU, *u, *pvir, *tau;
 };
-template <bool LJ, bool FAST = false>
-__global__ void __launch_bounds__(PAIR_WARPS * 32, FAST ? 3 : 1) k_sr(int n, Cell c, const double4 *__restrict__ s,
+template <bool LJ>
+__global__ void __launch_bounds__(PAIR_WARPS * 32, LJ ? 1 : 3) k_sr(int n, Cell c, const double4 *__restrict__ s,
                                                         const int *__restrict__ typ, const PairSR *__restrict__ pr,
                                                         int nt, const int *__restrict__ nbl,
                                                         const int *__restrict__ nbn, int cap, double srcutsq,
-                                                        int trunctype, int damped, TT tt, double3 *__restrict__ f,
+                                                        int trunctype, int damped, double3 *__restrict__ f,
                                                         double *__restrict__ part, int slot, int stride, SrFin fin) {
     grid_dep();
     int i = blockIdx.x * PAIR_WARPS + (threadIdx.x >> 5);
@@ -54,8 +54,7 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32, FAST ? 3 : 1) k_sr(int n, Cel
     if (i < n) {
         double4 si = s[i];
         int ti = typ[i];
-        int m = nbn[i];
-        if (m > cap) m = cap;
+        const int m = min(nbn[i], cap);
         const int *L = nbl + (size_t)i * cap;
         // neighbour types and positions one round ahead, indices two rounds ahead
         int jc = lane < m ? L[lane] : 0;
@@ -76,8 +75,8 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32, FAST ? 3 : 1) k_sr(int n, Cel
             double r2 = norm2_exact(r);
             if (!(r2 < srcutsq)) continue;
             double u, w;
-            if (FAST && !LJ) bhm_pair_fast(P, r2, damped, u, w);
-            else sr_pair<LJ>(P, r2, trunctype, damped, tt, u, w);
+            if (LJ) lj_pair(P, r2, trunctype, u, w);
+            else bhm_pair(P, r2, damped, u, w);
             sr_accumulate(r, u, w, fx, fy, fz, acc);
         }
     }
@@ -127,7 +126,6 @@ __global__ void __launch_bounds__(896) k_sum_sr(const double *part, int stride, 
 bool sum_in_last(const Engine &e, int blocks) { return blocks <= 4 * e.nsm; }
 
 void launch_sr(Engine &e, bool lj) {
-    TT tt = make_tt();
     int nb = ceil_div(e.n, PAIR_WARPS);
     DevScalars *o = e.d_out;
     const int slot = lj ? S_LJ_U : S_BH_U;
@@ -135,15 +133,11 @@ void launch_sr(Engine &e, bool lj) {
               lj ? &o->pvir_lj : &o->pvir_bh, lj ? o->tau_lj : o->tau_bh};
     if (lj)
         MDFF_LAUNCH(e, k_sr<true>, nb, PAIR_WARPS * 32, 0, e.n, e.cell, e.d_s, e.d_typ, e.d_pair, e.nt, e.d_nb,
-                    e.d_nbn, e.cap_nb, e.srcutsq, e.p.trunctype, 0, tt, e.d_f, e.d_part, (int)S_LJ_U,
+                    e.d_nbn, e.cap_nb, e.srcutsq, e.p.trunctype, 0, e.d_f, e.d_part, (int)S_LJ_U,
                     e.part_stride, fin);
-    else if (e.use32)
-        MDFF_LAUNCH(e, (k_sr<false, true>), nb, PAIR_WARPS * 32, 0, e.n, e.cell, e.d_s, e.d_typ, e.d_pair, e.nt,
-                    e.d_nb, e.d_nbn, e.cap_nb, e.srcutsq, e.p.trunctype, e.p.lbhmftd, tt, e.d_f, e.d_part,
-                    (int)S_BH_U, e.part_stride, fin);
     else
         MDFF_LAUNCH(e, k_sr<false>, nb, PAIR_WARPS * 32, 0, e.n, e.cell, e.d_s, e.d_typ, e.d_pair, e.nt, e.d_nb,
-                    e.d_nbn, e.cap_nb, e.srcutsq, e.p.trunctype, e.p.lbhmftd, tt, e.d_f, e.d_part, (int)S_BH_U,
+                    e.d_nbn, e.cap_nb, e.srcutsq, e.p.trunctype, e.p.lbhmftd, e.d_f, e.d_part, (int)S_BH_U,
                     e.part_stride, fin);
     if (!fin.ticket) MDFF_LAUNCH(e, k_sum_sr, 1, 896, 0, e.d_part, e.part_stride, nb, slot, fin);
 }
