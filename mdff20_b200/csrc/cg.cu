@@ -65,7 +65,30 @@ struct CgArgs {
     double2 *acc;
     const double3 *efs, *tx, *rhs;
     CgTest test;
+    CgComb comb;                 // A p to be formed (part set) in place of ap
 };
+
+// A p of the t-th ion i from the slice partials of the FP32 ion pass: alpha^-1 p - T p, k_combine32's
+// terms in its order.  A launch less per iteration than with k_combine32 between: the fit of
+// 48 configurations 10.18 -> 9.72 ms.
+__device__ __forceinline__ double3 comb_ap(const CgComb &b, int cnt, int t, int i, const double3 &p,
+                                           const double *__restrict__ I) {
+    double S[3] = {0, 0, 0};
+#pragma unroll 8
+    for (int s = 0; s < b.nslice; s++) {
+        const double *o = b.part + ((size_t)s * cnt + t) * 3;
+        for (int k = 0; k < 3; k++) S[k] += o[k];
+    }
+    const double3 d = b.ef_dir[i];
+    const double sp[3] = {b.self2 * p.x + d.x, b.self2 * p.y + d.y, b.self2 * p.z + d.z};
+    double T[3];
+    for (int k = 0; k < 3; k++) {
+        const double g = TPI_D * (b.c.B[k][0] * S[0] + b.c.B[k][1] * S[1] + b.c.B[k][2] * S[2]);
+        T[k] = sp[k] + (-b.tfpiV * g);
+    }
+    return make_double3(I[0] * p.x + I[1] * p.y + I[2] * p.z - T[0], I[3] * p.x + I[4] * p.y + I[5] * p.z - T[1],
+                        I[6] * p.x + I[7] * p.y + I[8] * p.z - T[2]);
+}
 
 // r, z = alpha r, p = z, r.z, r.r and the test before the first iteration; one ion per thread
 __global__ void __launch_bounds__(CGT) k_cg_begin(CgArgs a) {
@@ -121,7 +144,7 @@ __global__ void __launch_bounds__(CGT) k_cg_update(CgArgs a) {
     double P[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     if (on) {
         p = a.p[i];
-        q = a.ap[i];
+        q = a.comb.part ? comb_ap(a.comb, a.cnt, t, i, p, a.invpol + (size_t)i * 9) : a.ap[i];
         x = a.x[i];
         r = a.r[i];
 #pragma unroll
@@ -257,6 +280,8 @@ void launch_cg_update(Engine &e, double3 *x, const double2 *rho_p, double2 *acc,
     CgArgs a = cg_args(e, x, t);
     a.rho_p = rho_p;
     a.acc = acc;
+    a.comb = e.cg_comb;
+    e.cg_comb.part = nullptr;
     const int cs = cluster_of(a.cnt);
     MDFF_LAUNCH_C(e, cs, k_cg_update, cs, CGT, 0, a);
 }

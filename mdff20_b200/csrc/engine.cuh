@@ -170,6 +170,14 @@ struct CoulFin {
     const double *scal;
     double *u, *pvir, *tau;
 };
+// A p left as the slice partials of the FP32 ion pass: the cluster's update forms it (CgArgs)
+struct CgComb {
+    const double *part = nullptr;   // [slice][cnt][3]
+    int nslice = 0;
+    Cell c;
+    double tfpiV = 0.0, self2 = 0.0;
+    const double3 *ef_dir = nullptr;
+};
 struct RecOut {
     CoulFin fin;
     double3 *ef = nullptr;            // self2*mu + ef_dir + E_rec
@@ -371,6 +379,7 @@ struct Engine {
     float4 *d_qm_tc = nullptr;                          // per position of the order: (q, 2 pi B mu)
     float2 *d_rho_part32 = nullptr;                     // [rho32_chunks][nk]
     int ion32_slices = 0, nsm = 148;                    // most ion-pass slices; SMs
+    CgComb cg_comb;                                     // A p of the iteration being issued (part set)
     double *d_ion_part32 = nullptr;                     // [slices][n][6]
     int *d_pidx = nullptr;                              // polarisable ions, ascending
     bool rho_acc_ready = false;                         // d_rho_acc holds rho(k) of (q, mu_tot)

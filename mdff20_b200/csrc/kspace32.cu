@@ -787,13 +787,23 @@ void launch_combine32(Engine &e, const double *q, const double3 *mu, bool ld, co
     e.join_side(Engine::SIDE_PREP);
     e.join_side(Engine::SIDE_BODY);
     e.join_side(Engine::SIDE_FIELD);
+    const double tfpiV = 2.0 * 2.0 * TPI_D * e.cell.inveOmega;
+    if (o.cg.ap && !o.cg.part && !wf) {   // on one cluster: k_cg_update sums the slices
+        e.cg_comb.part = e.d_ion_part32;
+        e.cg_comb.nslice = slices;
+        e.cg_comb.c = e.cell;
+        e.cg_comb.tfpiV = tfpiV;
+        e.cg_comb.self2 = o.self2;
+        e.cg_comb.ef_dir = o.ef_dir;
+        return;
+    }
     Comb32Args b;
     b.cnt = cnt;
     b.nslice = slices;
     b.idx = idx;
     b.c = e.cell;
     b.part = e.d_ion_part32;
-    b.tfpiV = 2.0 * 2.0 * TPI_D * e.cell.inveOmega;
+    b.tfpiV = tfpiV;
     b.self2 = o.self2;
     b.coul = o.coul;
     b.ld = ld;
