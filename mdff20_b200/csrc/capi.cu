@@ -517,7 +517,7 @@ int mdffgpu_fit_plan_eval(mdffgpu_fit_plan *plan, const double *theta, double *r
             Engine &e = *P.ctx[c]->e;
             if (!e.fit_exec || e.fit_graph_gen != e.gen) {
                 try {
-                    e.capture_fit(P.d_theta, P.tSi, P.tO, P.scale, P.d_res + (size_t)c * NR);
+                    e.capture_fit(P.d_theta, P.tSi, P.tO, P.scale, P.d_res + (size_t)c * NR, nconf);
                 } catch (const Error &x) {
                     throw Error(x.code, "configuration " + std::to_string(c) + ": " + x.what());
                 }

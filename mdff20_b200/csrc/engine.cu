@@ -500,6 +500,7 @@ void Engine::setup_kspace() {
     MDFF_CK(cudaMemcpy(d_kcoe, kcoe.data(), sizeof(double) * nk, cudaMemcpyHostToDevice));
     MDFF_CK(cudaMemcpy(d_row, rows.data(), sizeof(KRow) * nrow, cudaMemcpyHostToDevice));
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+    split_sm = nsm;
     d_rho = dalloc<double2>(nk);
     d_rho_acc = dalloc<double2>(nk);
     d_rho_it = dalloc<double2>(nk);

@@ -379,6 +379,7 @@ struct Engine {
     float4 *d_qm_tc = nullptr;                          // per position of the order: (q, 2 pi B mu)
     float2 *d_rho_part32 = nullptr;                     // [rho32_chunks][nk]
     int ion32_slices = 0, nsm = 148;                    // most ion-pass slices; SMs
+    int split_sm = 148;                                 // SMs the FP64 k-space passes are split for
     CgComb cg_comb;                                     // A p of the iteration being issued (part set)
     double *d_ion_part32 = nullptr;                     // [slices][n][6]
     int *d_pidx = nullptr;                              // polarisable ions, ascending
@@ -564,7 +565,7 @@ struct Engine {
     void fit_alloc();
     void fit_apply_theta(const double *d_th, int tSi, int tO);
     void fit_issue(const double3 *d_ft, double scale, int tSi, int tO, const double *d_th, double *d_res);
-    void capture_fit(const double *d_th, int tSi, int tO, double scale, double *d_res);
+    void capture_fit(const double *d_th, int tSi, int tO, double scale, double *d_res, int nconf);
     void solve_pim(const double3 *d_b, double3 *d_x, double rtol, int maxit);
     void fit_reduce(int first, int cnt, int nparts);
     void coul_forces(const double *d_qv, const double3 *d_muv, bool lq, bool ld, double3 *out);

@@ -726,7 +726,13 @@ void Engine::force_match(const double3 *d_ft, double scale, double *h_res, int t
 
 // record one evaluation (theta from d_th, result into d_res) as a CUDA graph: the
 // parameter update, forces with the induced-dipole CG, adjoint CG and sensitivities
-void Engine::capture_fit(const double *d_th, int tSi, int tO, double scale, double *d_res) {
+// nconf: configurations that will be in flight together.  From a dozen on their FP64 k-space
+// passes are split for half of the SMs: pieces cut small for one system alone cost more (partial
+// sums, starts of the row loops) than the others leave idle.  Evaluations in FP64, ms, split for
+// 148 / 74 / 37 SMs: 48 configurations 13.60 / 12.62 / 12.66, 12: 3.74 / 3.56 / 3.80, 4: 2.10 /
+// 2.20 / 2.54.  (The FP32 passes stay as they are: a tenth of the SMs took 48 configurations from
+// 9.7 to 10.1 ms where the inputs come from memory, although 8.1 to 7.5 where they are in L2.)
+void Engine::capture_fit(const double *d_th, int tSi, int tO, double scale, double *d_res, int nconf) {
     if (fit_exec) cudaGraphExecDestroy(fit_exec);
     fit_exec = nullptr;
     if (p.lverletL && !list_ready) gen_verletlist();
@@ -742,10 +748,13 @@ void Engine::capture_fit(const double *d_th, int tSi, int tO, double scale, doub
         pdl = false;
         fit_apply_theta(d_th, tSi, tO);
         pdl = true;
+        if (!use32) split_sm = std::clamp(6 * nsm / nconf, nsm / 2, nsm);
         fit_issue(d_ft, scale, tSi, tO, d_th, d_res);
+        split_sm = nsm;
     } catch (...) {
         capturing = false;
         pdl = true;
+        split_sm = nsm;
         forget_sides();
         cudaStreamEndCapture(stream, &graph);
         if (graph) cudaGraphDestroy(graph);

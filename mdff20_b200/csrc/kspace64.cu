@@ -702,7 +702,7 @@ static void rho64(Engine &e, const double *q, const double3 *mu, bool lq, bool l
         int per = stages;
         for (int c = 1; c <= std::min(e.rho64_chunks_max, stages); c++) {
             const int p = ceil_div(stages, c), used = ceil_div(stages, p);
-            const double cost = ceil_div(rb * used, e.nsm) * (p + 1.0) + 0.02 * used;
+            const double cost = ceil_div(rb * used, e.split_sm) * (p + 1.0) + 0.02 * used;
             if (cost < best) {
                 best = cost;
                 per = p;
@@ -822,7 +822,7 @@ void launch_rec64(Engine &e, const double *q, const double3 *mu, bool lq, bool l
             const double unit = m * (m == 1 ? 1.3 : (m == 2 ? 1.1 : 1.0)) * (w == 8 ? 2.0 : 1.0);
             for (int s = 1; s <= e.ion64_slices_max && s * w <= std::max(a.units, 8); s++) {
                 const double cost =
-                    ceil_div(blocks * s, e.nsm) * ceil_div(a.units, s * w) * unit + 8.0 + (s > 1 ? 16.0 : 0.0);
+                    ceil_div(blocks * s, e.split_sm) * ceil_div(a.units, s * w) * unit + 8.0 + (s > 1 ? 16.0 : 0.0);
                 if (cost < best) {
                     best = cost;
                     mt = m;
