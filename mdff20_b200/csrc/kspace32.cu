@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(ION32_THREADS, ION32X2_MIN_BLOCKS) k_ion32x2(I
     }
 }
 
-// slices summed in a fixed order; field / force / self terms as k_rec_combine (kspace.cu)
+// slices summed in a fixed order; field / force / self terms as those of k_ion64 (kspace64.cu)
 struct Comb32Args {
     int cnt, nslice;
     const int *idx;
