@@ -705,9 +705,10 @@ static double self2_of(double alpha) {
 // electric field of (q, mu): self + direct + reciprocal, as multipole_ES with
 // do_ef only (src/ewald.c:75-348); no energy, no forces
 void Engine::field_of(const double *d_qv, const double3 *d_muv, bool lq, bool ld, bool damp, double3 *d_ef_out,
-                      double2 *rho_raw) {
-    if (!lq && ld && !damp && coef_ready) {
-        // induced dipoles: nonzero at polarisable ions only, field needed there only
+                      bool induced, double2 *rho_raw) {
+    if (induced && coef_ready) {
+        // nonzero at polarisable ions only, field needed there only: the records of those pairs
+        // (static dipoles may sit on any ion, so they never come here)
         if (use32 && real32) launch_pol_field32(*this, d_muv, d_tmp3);
         else launch_dir_field_cached(*this, d_muv, d_tmp3);
     } else if (use32 && real32) {
@@ -838,7 +839,7 @@ void Engine::tune_launch(int reps, int *choice, double *ms) {
 // momentpolaSCF (src/pim.c:177-306) with extrapolate_dipole_aspc (src/pim.c:314-424)
 void Engine::pim_reference() {
     int nb = ceil_div(n, 256);
-    field_of(d_q, d_mu_static, lqch != 0, ldip != 0, ldmp != 0, d_ef_stat);
+    field_of(d_q, d_mu_static, lqch != 0, ldip != 0, ldmp != 0, d_ef_stat, false);
     MDFF_CK(cudaMemcpyAsync(d_ef, d_ef_stat, sizeof(double3) * n, cudaMemcpyDeviceToDevice, stream));
     int ord = p.extrapolate_order;
     int e = (istep >= ord + 1) ? ord : (!istep ? 0 : istep - 1);
@@ -858,7 +859,7 @@ void Engine::pim_reference() {
             reduce(S_UPOL, 1, nb);
             MDFF_CK(cudaMemcpyAsync(&h_out->u_pol, d_scal + S_UPOL, sizeof(double), cudaMemcpyDeviceToHost, stream));
         }
-        field_of(d_qzero, d_mu_ind, false, true, false, d_ef_ind);
+        field_of(d_qzero, d_mu_ind, false, true, false, d_ef_ind, true);
         MDFF_LAUNCH(*this, k_add3, nb, 256, 0, n, d_ef_stat, d_ef_ind, d_ef);
         if (!iscf) MDFF_LAUNCH(*this, k_aspc_correct, nb, 256, 0, n, Wt[e], d_polar, d_pol, d_ef, d_mu_ind);
         MDFF_LAUNCH(*this, k_pim_sums, nb, 256, 0, n, d_polar, d_pol, d_invpol, d_mu_ind, d_ef, d_part, part_stride);
@@ -1016,9 +1017,9 @@ void Engine::pim_cg(bool fused) {
         join_side(SIDE_PREP);   // (joined by the ion pass already; the loop below reads the records)
     } else {
         join_side(SIDE_PREP);
-        field_of(d_q, d_mu_static, lqch != 0, ldip != 0, ldmp != 0, d_ef_stat);
+        field_of(d_q, d_mu_static, lqch != 0, ldip != 0, ldmp != 0, d_ef_stat, false);
         launch_pim_begin(*this, aspc_coef(e, cg_poly), es);
-        field_of(d_qzero, d_mu_ind, false, true, false, d_ef_ind);
+        field_of(d_qzero, d_mu_ind, false, true, false, d_ef_ind, true);
         efs = d_ef_stat;
     }
     if (!clustered) {
@@ -1044,7 +1045,7 @@ void Engine::pim_cg(bool fused) {
             // T p over the polarisable ions; Ap and p.Ap formed by the ion pass
             field_pol(d_cg_p, d_ef_ind, fused ? d_rho_it : nullptr, true);
         } else {
-            field_of(d_qzero, d_cg_p, false, true, false, d_ef_ind, fused ? d_rho_it : nullptr);
+            field_of(d_qzero, d_cg_p, false, true, false, d_ef_ind, true, fused ? d_rho_it : nullptr);
             MDFF_LAUNCH(*this, k_cg_ap, nb, 256, 0, n, d_polar, d_invpol, d_cg_p, d_ef_ind, d_cg_ap, d_part,
                         part_stride, d_scal, d_ticket);
         }
@@ -1135,7 +1136,7 @@ void Engine::ko_inner(double3 *d_dmu, const double3 *d_find) {
 // momentpolaSCFkO (src/pim.c:457-603)
 void Engine::pim_ko() {
     int nb = ceil_div(n, 256);
-    field_of(d_q, d_mu_static, lqch != 0, ldip != 0, ldmp != 0, d_ef_stat);
+    field_of(d_q, d_mu_static, lqch != 0, ldip != 0, ldmp != 0, d_ef_stat, false);
     MDFF_CK(cudaMemcpyAsync(d_ef, d_ef_stat, sizeof(double3) * n, cudaMemcpyDeviceToDevice, stream));
     MDFF_CK(cudaMemcpyAsync(d_cg_r, d_ef_stat, sizeof(double3) * n, cudaMemcpyDeviceToDevice, stream));  // f_ind
     MDFF_CK(cudaMemsetAsync(d_mu_ind, 0, sizeof(double3) * n, stream));
@@ -1155,7 +1156,7 @@ void Engine::pim_ko() {
             MDFF_LAUNCH(*this, k_scale_add3, nb, 256, 0, n, 1.0, d_cg_p, 1.0, d_mu_ind);
         }
         rmsd_of(d_mu_ind, d_ef, &upol);   // u_pol of these dipoles (src/pim.c:539)
-        field_of(d_qzero, d_mu_ind, false, true, false, d_ef_ind);
+        field_of(d_qzero, d_mu_ind, false, true, false, d_ef_ind, true);
         MDFF_LAUNCH(*this, k_add3, nb, 256, 0, n, d_ef_stat, d_ef_ind, d_ef);
         if (!iscf) MDFF_LAUNCH(*this, k_aspc_correct, nb, 256, 0, n, Wt[e], d_polar, d_pol, d_ef, d_mu_ind);
         rmsd = rmsd_of(d_mu_ind, d_ef, nullptr);

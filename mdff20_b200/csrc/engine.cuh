@@ -538,8 +538,10 @@ struct Engine {
     void engforce(bool check_finite = true, bool opened = false);
     void multipole_es_dev(const double *d_qv, const double3 *d_muv, double alpha, int flags, double3 *d_ef_out,
                           double *d_efg_out, double3 *d_f_out);
+    // induced: d_muv is zero at the ions that are not polarisable and only the dipoles act
+    // (no charges, no damping), so the pair records of the evaluation serve
     void field_of(const double *d_qv, const double3 *d_muv, bool lq, bool ld, bool damp, double3 *d_ef_out,
-                  double2 *rho_raw = nullptr);
+                  bool induced, double2 *rho_raw = nullptr);
     void field_pol(const double3 *d_p, double3 *d_out, double2 *rho_raw, bool cg_ap = false);
     void ensure_real32();
     void dfree32();

@@ -507,7 +507,7 @@ void Engine::solve_pim(const double3 *d_b, double3 *d_x, double rtol, int maxit)
     auto iteration = [&](CgTest t) {
         const bool sub = subset32 && npol > 0;
         if (sub) field_pol(d_cg_p, d_ef_ind, nullptr, true);
-        else field_of(d_qzero, d_cg_p, false, true, false, d_ef_ind);
+        else field_of(d_qzero, d_cg_p, false, true, false, d_ef_ind, true);
         if (!sub)
             MDFF_LAUNCH(*this, k_cg_ap, nb, 256, 0, n, d_polar, d_invpol, d_cg_p, d_ef_ind, d_cg_ap, d_part,
                         part_stride, d_scal, d_ticket);
@@ -699,7 +699,7 @@ void Engine::fit_issue(const double3 *d_ft, double scale, int tSi, int tO, const
     MDFF_LAUNCH(*this, k_dot3, nb, 256, 0, n, d_w, d_fa, nullptr, d_fpart, (int)F_WFALL, part_stride);
     MDFF_LAUNCH(*this, k_dot3, nb, 256, 0, n, d_w, d_fb, nullptr, d_fpart, (int)F_WFQ0, part_stride);
     MDFF_LAUNCH(*this, k_dot3, nb, 256, 0, n, d_w, d_fc, nullptr, d_fpart, (int)F_WF0M, part_stride);
-    field_of(q, d_muzero, true, false, ldmp != 0, d_fb);   // E(q, 0), the static field
+    field_of(q, d_muzero, true, false, ldmp != 0, d_fb, false);   // E(q, 0), the static field
     MDFF_LAUNCH(*this, k_dot3, nb, 256, 0, n, d_lam, d_fb, d_polar, d_fpart, (int)F_LESTAT, part_stride);
     MDFF_LAUNCH(*this, k_dot3, nb, 256, 0, n, d_lam, d_mu_ind, d_polar, d_fpart, (int)F_LMU, part_stride);
     fit_reduce(F_WFALL, 5, nb);
