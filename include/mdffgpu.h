@@ -311,7 +311,8 @@ int mdffgpu_fit_batch(mdffgpu_ctx **ctx, int nconf, int tSi, int tO, const doubl
  * summed in configuration order; the first eval (and the first after a context's
  * precision or solver changed) records the graphs.  The contexts must not be used by
  * other calls while an eval runs; after evals each context's tables hold the last
- * theta.  mdffgpu_fit_plan_last_error: message of the last failed call. */
+ * theta.  A context may belong to several plans, evaluated one after another (each plan
+ * holds its own targets, graphs and results).  mdffgpu_fit_plan_last_error: message of the last failed call. */
 typedef struct mdffgpu_fit_plan mdffgpu_fit_plan;
 int mdffgpu_fit_plan_create(mdffgpu_ctx **ctx, int nconf, int tSi, int tO, const double *const *targets,
                             double scale, mdffgpu_fit_plan **out);

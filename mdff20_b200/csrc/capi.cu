@@ -60,11 +60,20 @@ struct mdffgpu_fit_plan {
     double *d_theta = nullptr;   // shared by every recorded evaluation
     double *d_res = nullptr;     // [nconf][FIT_NRES]
     double *h_theta = nullptr, *h_res = nullptr;   // pinned staging
+    // per configuration: target forces, the recorded evaluation (its theta, targets and result
+    // buffers are this plan's, so it belongs here: contexts may be in several plans) and the
+    // generation of the context it was recorded at
+    std::vector<double3 *> d_ft;
+    std::vector<cudaGraphExec_t> exec;
+    std::vector<long long> gen;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_theta = nullptr;
     std::vector<cudaEvent_t> ev_done;
     std::string err;
     ~mdffgpu_fit_plan() {
+        for (cudaGraphExec_t x : exec)
+            if (x) cudaGraphExecDestroy(x);
+        for (double3 *x : d_ft) cudaFree(x);
         for (cudaEvent_t e : ev_done) cudaEventDestroy(e);
         if (ev_theta) cudaEventDestroy(ev_theta);
         if (stream) cudaStreamDestroy(stream);
@@ -489,10 +498,13 @@ int mdffgpu_fit_plan_create(mdffgpu_ctx **ctx, int nconf, int tSi, int tO, const
         P.d_res = mdffgpu::dalloc<double>((size_t)nconf * mdffgpu::FIT_NRES);
         MDFF_CK(cudaMallocHost((void **)&P.h_theta, sizeof(double) * MDFFGPU_FIT_NPARAM));
         MDFF_CK(cudaMallocHost((void **)&P.h_res, sizeof(double) * nconf * mdffgpu::FIT_NRES));
+        P.exec.assign(nconf, nullptr);
+        P.gen.assign(nconf, -1);
+        P.d_ft.assign(nconf, nullptr);
         for (int c = 0; c < nconf; c++) {
             Engine &e = *ctx[c]->e;
-            if (!e.d_ft) e.d_ft = mdffgpu::dalloc<double3>(e.n);
-            upload(e, e.d_ft, targets[c], sizeof(double3) * e.n);
+            P.d_ft[c] = mdffgpu::dalloc<double3>(e.n);
+            upload(e, P.d_ft[c], targets[c], sizeof(double3) * e.n);
             MDFF_CK(cudaStreamSynchronize(e.stream));
         }
     });
@@ -515,9 +527,13 @@ int mdffgpu_fit_plan_eval(mdffgpu_fit_plan *plan, const double *theta, double *r
         // record what is missing or stale before anything is in flight
         for (int c = 0; c < nconf; c++) {
             Engine &e = *P.ctx[c]->e;
-            if (!e.fit_exec || e.fit_graph_gen != e.gen) {
+            if (!P.exec[c] || P.gen[c] != e.gen) {
+                if (P.exec[c]) cudaGraphExecDestroy(P.exec[c]);
+                P.exec[c] = nullptr;
                 try {
-                    e.capture_fit(P.d_theta, P.tSi, P.tO, P.scale, P.d_res + (size_t)c * NR, nconf);
+                    P.exec[c] = e.capture_fit(P.d_ft[c], P.d_theta, P.tSi, P.tO, P.scale, P.d_res + (size_t)c * NR,
+                                              nconf);
+                    P.gen[c] = e.gen;
                 } catch (const Error &x) {
                     throw Error(x.code, "configuration " + std::to_string(c) + ": " + x.what());
                 }
@@ -530,7 +546,7 @@ int mdffgpu_fit_plan_eval(mdffgpu_fit_plan *plan, const double *theta, double *r
         for (int c = 0; c < nconf; c++) {
             Engine &e = *P.ctx[c]->e;
             MDFF_CK(cudaStreamWaitEvent(e.stream, P.ev_theta, 0));
-            MDFF_CK(cudaGraphLaunch(e.fit_exec, e.stream));
+            MDFF_CK(cudaGraphLaunch(P.exec[c], e.stream));
             MDFF_CK(cudaEventRecord(P.ev_done[c], e.stream));
             MDFF_CK(cudaStreamWaitEvent(P.stream, P.ev_done[c], 0));
         }

@@ -223,7 +223,6 @@ Engine::~Engine() {
     cudaFree(d_snap);
     cudaFree(d_soa);
     if (step_exec) cudaGraphExecDestroy(step_exec);
-    if (fit_exec) cudaGraphExecDestroy(fit_exec);
     if (body_stream) cudaStreamDestroy(body_stream);
     for (int k = 0; k < NSIDE; k++) {
         if (ev_fork[k]) cudaEventDestroy(ev_fork[k]);
@@ -1410,9 +1409,6 @@ void Engine::drop_graph() {
     if (step_exec) cudaGraphExecDestroy(step_exec);
     step_exec = nullptr;
     graph_gen = -1;
-    if (fit_exec) cudaGraphExecDestroy(fit_exec);
-    fit_exec = nullptr;
-    fit_graph_gen = -1;
 }
 
 // record prop_agate + check_verletlist of one step (src/md.c:237-241) as a graph

@@ -430,15 +430,10 @@ struct Engine {
     double *d_qw = nullptr, *d_efg_rec = nullptr;
     double3 *d_muw = nullptr;
     double2 *d_rw = nullptr;
-    double3 *d_ft = nullptr;         // target forces
+    double3 *d_ft = nullptr;         // target forces of a single evaluation
     double *d_theta = nullptr;       // theta on the device (read by the result assembly)
     double *d_fres = nullptr;        // [1 + NPARAM + 1]: the last evaluation's result and status
     int last_adj_iter = 0;
-    // one force-matching evaluation recorded as a CUDA graph (fit batches): both CG
-    // solves are while nodes, theta is read from a device buffer and the result is
-    // assembled on the device, so a replay needs no host round trip
-    cudaGraphExec_t fit_exec = nullptr;
-    long long fit_graph_gen = -1;
 
     // one MD step as a CUDA graph (md_steps): the induced-dipole CG loop is a while node
     // whose condition a device kernel sets, so a step needs no host round trip
@@ -567,7 +562,11 @@ struct Engine {
     void fit_alloc();
     void fit_apply_theta(const double *d_th, int tSi, int tO);
     void fit_issue(const double3 *d_ft, double scale, int tSi, int tO, const double *d_th, double *d_res);
-    void capture_fit(const double *d_th, int tSi, int tO, double scale, double *d_res, int nconf);
+    // one evaluation recorded as a CUDA graph (fit batches): both CG solves are while nodes,
+    // theta is read from a device buffer and the result is assembled on the device, so a replay
+    // needs no host round trip.  The caller owns the graph, valid while gen stays as it is
+    cudaGraphExec_t capture_fit(const double3 *d_ft, const double *d_th, int tSi, int tO, double scale, double *d_res,
+                                int nconf);
     void solve_pim(const double3 *d_b, double3 *d_x, double rtol, int maxit);
     void fit_reduce(int first, int cnt, int nparts);
     void coul_forces(const double *d_qv, const double3 *d_muv, bool lq, bool ld, double3 *out);

@@ -732,9 +732,8 @@ void Engine::force_match(const double3 *d_ft, double scale, double *h_res, int t
 // 148 / 74 / 37 SMs: 48 configurations 13.60 / 12.62 / 12.66, 12: 3.74 / 3.56 / 3.80, 4: 2.10 /
 // 2.20 / 2.54.  (The FP32 passes stay as they are: a tenth of the SMs took 48 configurations from
 // 9.7 to 10.1 ms where the inputs come from memory, although 8.1 to 7.5 where they are in L2.)
-void Engine::capture_fit(const double *d_th, int tSi, int tO, double scale, double *d_res, int nconf) {
-    if (fit_exec) cudaGraphExecDestroy(fit_exec);
-    fit_exec = nullptr;
+cudaGraphExec_t Engine::capture_fit(const double3 *d_ft, const double *d_th, int tSi, int tO, double scale,
+                                    double *d_res, int nconf) {
     if (p.lverletL && !list_ready) gen_verletlist();
     fit_alloc();
     if (use32 && real32 && p.lcoulombic) ensure_real32();   // no allocation while recording
@@ -763,14 +762,12 @@ void Engine::capture_fit(const double *d_th, int tSi, int tO, double scale, doub
     }
     capturing = false;
     MDFF_CK(cudaStreamEndCapture(stream, &graph));
-    cudaError_t err = cudaGraphInstantiate(&fit_exec, graph, cudaGraphInstantiateFlagUseNodePriority);
+    cudaGraphExec_t exec = nullptr;
+    cudaError_t err = cudaGraphInstantiate(&exec, graph, cudaGraphInstantiateFlagUseNodePriority);
     cudaGraphDestroy(graph);
-    if (err != cudaSuccess) {
-        fit_exec = nullptr;
-        MDFF_CK(err);
-    }
     launches = l0;
-    fit_graph_gen = gen;
+    MDFF_CK(err);
+    return exec;
 }
 
 }  // namespace mdffgpu
