@@ -209,9 +209,10 @@ int mdffgpu_md_steps(mdffgpu_ctx *ctx, int first, int nsteps, double *thermo);
  * globals).  in (may be NULL): 6 arrays rx ry rz vx vy vz of nion doubles copied in
  * before the steps (an entry NULL keeps that component's device values); out (may be
  * NULL): 9 arrays rx ry rz vx vy vz fx fy fz the state after the last step is copied to
- * (entries may be NULL).  The copies are queued with the steps: one call and, as in
- * mdffgpu_md_steps, one synchronisation per step, the outgoing copies riding on the last
- * one.  Equivalent to set_positions + set_velocities + md_steps + get_state. */
+ * (entries may be NULL).  A single step is one synchronisation, the outgoing copies
+ * riding on it; longer calls wait once per batch of up to 16 recorded steps, and copy out
+ * when the last batch is known to be sound: a call that fails before its last step leaves
+ * out as it was.  Equivalent to set_positions + set_velocities + md_steps + get_state. */
 int mdffgpu_md_steps_host(mdffgpu_ctx *ctx, int first, int nsteps, const double *const *in, double *thermo,
                           double *const *out);
 

@@ -1516,7 +1516,8 @@ void Engine::snapshot(bool restore) {
 // read back together (a step of a few hundred ions takes less than the synchronisation that
 // followed each one).  A step that needs the host (a list that outgrew its capacity) or fails
 // shows in its status word: the batch is then undone and its steps run one by one, so that the
-// error, the state it leaves and the records before it are those of single steps.
+// error, the state it leaves, the records before it and the caller's arrays are those of single
+// steps.
 void Engine::md_steps(int first, int nsteps, double *thermo, const double *const *in, double *const *out) {
     if (in) {
         // the caller's positions and velocities, packed on the device (no synchronisation:
@@ -1540,16 +1541,18 @@ void Engine::md_steps(int first, int nsteps, double *thermo, const double *const
             MDFF_LAUNCH(*this, k_pack_v, ceil_div(n, 256), 256, 0, n, d_soa, d_v);
         }
     }
-    auto queue_out = [&] {
-        if (!out) return;
-        MDFF_LAUNCH(*this, k_unpack_state, ceil_div(n, 256), 256, 0, n, d_r, d_v, d_f, d_soa);
+    auto unpack = [&] {
+        if (out) MDFF_LAUNCH(*this, k_unpack_state, ceil_div(n, 256), 256, 0, n, d_r, d_v, d_f, d_soa);
+    };
+    auto copy_out = [&] {
         for (int k = 0; k < 9; k++)
-            if (out[k])
+            if (out && out[k])
                 MDFF_CK(cudaMemcpyAsync(out[k], d_soa + (size_t)k * n, sizeof(double) * n, cudaMemcpyDeviceToHost,
                                         stream));
     };
     if (nsteps == 0) {
-        queue_out();
+        unpack();
+        copy_out();
         MDFF_CK(cudaStreamSynchronize(stream));
         return;
     }
@@ -1589,7 +1592,8 @@ void Engine::md_steps(int first, int nsteps, double *thermo, const double *const
             snapshot(false);
             for (int b = 0; b < batch; b++) MDFF_CK(cudaGraphLaunch(step_exec, stream));
             istep = step + batch - 1;
-            if (s + batch == nsteps) queue_out();
+            const bool end = s + batch == nsteps;
+            if (end) unpack();
             MDFF_CK(cudaMemcpyAsync(h_rec, d_rec, sizeof(DevScalars) * batch, cudaMemcpyDeviceToHost, stream));
             sync_scalars();
             unsigned st = (unsigned)h_out->status;
@@ -1599,6 +1603,10 @@ void Engine::md_steps(int first, int nsteps, double *thermo, const double *const
                 istep = istep0;
                 single_until = s + batch;
                 continue;
+            }
+            if (end && out) {   // the caller's arrays only once no step of the batch has failed
+                copy_out();
+                MDFF_CK(cudaStreamSynchronize(stream));
             }
             for (int b = 0; b < batch; b++) {
                 const DevScalars &o = b + 1 < batch ? h_rec[b + 1] : *h_out;
@@ -1616,7 +1624,10 @@ void Engine::md_steps(int first, int nsteps, double *thermo, const double *const
             prop_agate(step, StepCheck{p.lverletL != 0, nullptr});
             if (p.lverletL) rebuild_if_due();
         }
-        if (s == nsteps - 1) queue_out();   // on the last step's synchronisation
+        if (s == nsteps - 1) {   // on the last step's synchronisation
+            unpack();
+            copy_out();
+        }
         sync_scalars();
         const DevScalars o = *h_out;
         if (graphed) {
