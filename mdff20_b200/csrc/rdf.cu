@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "engine.cuh"
+#include "wrap32.h"
 
 namespace mdffgpu {
 
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(GR_THREADS) k_gr_pairs(const __grid_constant__
                 const int4 o = tile[jj];
 #pragma unroll
                 for (int m = 0; m < IPT; m++) {
-                    const int dx = me[m].x - o.x, dy = me[m].y - o.y, dz = me[m].z - o.z;
+                    const int dx = wrap_diff(me[m].x, o.x), dy = wrap_diff(me[m].y, o.y), dz = wrap_diff(me[m].z, o.z);
                     const float u = (float)dx, v = (float)dy, q = (float)dz;
                     float x, y, z;
                     bool edge = false;
