@@ -770,11 +770,25 @@ void Engine::tune_launch(int reps, int *choice, double *ms) {
         throw Error(MDFFGPU_ERR_STATE, "launch tuning applies to the mixed-precision polarisable k space");
     reps = std::max(reps, 1);
     const bool by64 = rec64;   // the default of few ions: one more candidate
-    rec64 = false;
-    engforce();
     struct Cand {
         int tc, chunks, slices, rtc, f64 = 0;
     };
+    // the shapes in force until the candidates are timed: an error on the way leaves them
+    struct Keep {
+        Engine &e;
+        Cand c;
+        bool on = true;
+        ~Keep() {
+            if (!on) return;
+            e.rec64 = c.f64 != 0;
+            e.ion_tc = c.tc != 0;
+            e.rho32_chunks = c.chunks;
+            e.ion_tc_slices_set = c.slices;
+            e.rho_tc = c.rtc != 0;
+        }
+    } keep{*this, {ion_tc ? 1 : 0, rho32_chunks, ion_tc_slices_set, rho_tc ? 1 : 0, by64 ? 1 : 0}};
+    rec64 = false;
+    engforce();
     std::vector<int> chunk_set;
     for (int c : {std::max(1, rho32_chunks / 2), rho32_chunks, std::min(rho32_chunks_max, 2 * rho32_chunks)})
         if (std::find(chunk_set.begin(), chunk_set.end(), c) == chunk_set.end()) chunk_set.push_back(c);
@@ -797,7 +811,7 @@ void Engine::tune_launch(int reps, int *choice, double *ms) {
         }
     } evs{t0, t1};
     if (by64) cands.push_back({0, rho32_chunks, 0, 0, 1});
-    Cand best{ion_tc ? 1 : 0, rho32_chunks, ion_tc_slices_set, rho_tc ? 1 : 0};
+    Cand best = keep.c;
     double best_ms = 1e300;
     auto apply = [&](const Cand &c) {
         rec64 = c.f64 != 0;
@@ -825,6 +839,7 @@ void Engine::tune_launch(int reps, int *choice, double *ms) {
     }
     apply(best);
     MDFF_CK(cudaStreamSynchronize(stream));
+    keep.on = false;
     gen++;   // recorded steps use the chosen shapes from now on
     if (choice) {
         choice[0] = best.tc;
