@@ -152,9 +152,11 @@ int mdffgpu_set_precision(mdffgpu_ctx *ctx, int precision) {
         if (const char *v = getenv("MDFFGPU_PIM_SUBSET")) e.subset32 = atoi(v) != 0;
         // the rho and ion passes on the tensor cores (kspace_tc.cu, kspace_ion_tc.cu) from
         // TC_MIN_IONS ions on, on CUDA cores below, in FP64 below REC64_IONS; MDFFGPU_RHO_TC /
-        // MDFFGPU_ION_TC = 1 or 0 select the tensor-core or the CUDA-core FP32 pass at any size
+        // MDFFGPU_ION_TC = 1 or 0 select the tensor-core or the CUDA-core FP32 pass at any size,
+        // and MDFFGPU_MIXED_PARTS says itself what is in FP32
         e.rho_tc = e.ion_tc = e.n >= TC_MIN_IONS;
-        e.rec64 = e.n < REC64_IONS && !getenv("MDFFGPU_RHO_TC") && !getenv("MDFFGPU_ION_TC");
+        e.rec64 = e.n < REC64_IONS && !getenv("MDFFGPU_RHO_TC") && !getenv("MDFFGPU_ION_TC") &&
+                  !getenv("MDFFGPU_MIXED_PARTS");
         if (const char *v = getenv("MDFFGPU_RHO_TC")) e.rho_tc = atoi(v) != 0;
         if (const char *v = getenv("MDFFGPU_ION_TC")) e.ion_tc = atoi(v) != 0;
     });

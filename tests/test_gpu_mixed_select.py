@@ -1,13 +1,32 @@
-"""Which k-space passes a mixed-precision context of few ions runs: a launch tuning that fails
-leaves the selection as it was.  The same passes give the same
+"""Which k-space passes a mixed-precision context of few ions runs: the selection by environment
+switches, and that a launch tuning which fails leaves it as it was.  The same passes give the same
 bits, so results are compared for equality."""
 import numpy as np
 import pytest
 
-from mdff20_b200.engine import MIXED, PIM_CG, PIM_CG_FUSED, Engine, MdffgpuError
+from mdff20_b200.engine import FP64, MIXED, PIM_CG, PIM_CG_FUSED, Engine, MdffgpuError
 from tests.golden import cases
 
 pytestmark = pytest.mark.gpu
+
+
+def _forces(monkeypatch, precision, **env):
+    with monkeypatch.context() as m:
+        for k, v in env.items():
+            m.setenv(k, v)
+        e = Engine(cases.crist192(True, extrapolate_order=0), precision=precision, pim_solver=PIM_CG)
+    e.gen_verletlist()
+    e.engforce()
+    f = e.forces()
+    e.close()
+    return f
+
+
+def test_only_the_k_space_in_fp32(monkeypatch):
+    f = _forces(monkeypatch, MIXED, MDFFGPU_MIXED_PARTS="rec")
+    g = _forces(monkeypatch, MIXED, MDFFGPU_MIXED_PARTS="rec", MDFFGPU_RHO_TC="0", MDFFGPU_ION_TC="0")
+    h = _forces(monkeypatch, FP64)
+    assert np.array_equal(f, g) and not np.array_equal(f, h)
 
 
 @pytest.mark.parametrize("solver", [PIM_CG, PIM_CG_FUSED])
