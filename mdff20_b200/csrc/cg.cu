@@ -20,6 +20,11 @@ namespace mdffgpu {
 constexpr int CGT = 512;                  // threads per block
 constexpr int CG_CLUSTER_MAX = 8 * CGT;   // one ion per thread of eight blocks; with four ions per
                                           // thread 16000 dipoles took 17.9 us, the grid kernels 12
+// carried rho(k) per thread from which a larger cluster shares them out: in one block they are a
+// serial chain of reads from L2.  FP64 force evaluations with the fused CG, one block / at most 4
+// per thread: 96 ions nk 12194 300 / 264 us, nk 137312 702 / 440 us, 300 ions 331 / 297 and 862 /
+// 609 us; below 4096 (kmax 10) no difference
+constexpr int CG_RHO = 4;
 
 // sums of NV values over the cluster, in warp order then rank order; sh: [NV][16 + 1] of this
 // phase alone (read by the other blocks until the next cluster barrier)
@@ -61,8 +66,8 @@ struct CgArgs {
     double3 *p;
     const double3 *ap;
     double3 *x, *r;
-    const double2 *rho_p;        // rho(k) of p, and of the iterate (null: not carried)
-    double2 *acc;
+    const double2 *__restrict__ rho_p;   // rho(k) of p, and of the iterate (null: not carried)
+    double2 *__restrict__ acc;
     const double3 *efs, *tx, *rhs;
     CgTest test;
     CgComb comb;                 // A p to be formed (part set) in place of ap
@@ -160,11 +165,13 @@ __global__ void __launch_bounds__(CGT) k_cg_update(CgArgs a) {
         a.x[i] = make_double3(x.x + al * p.x, x.y + al * p.y, x.z + al * p.z);
         a.r[i] = r;
     }
-    if (a.acc)
+    if (a.acc) {
+#pragma unroll 4
         for (int k = t; k < a.nk; k += T) {
             const double2 w = a.rho_p[k], s = a.acc[k];
             a.acc[k] = make_double2(s.x + al * w.x, s.y + al * w.y);
         }
+    }
     cluster_sum<2>(cl, v, sh2);
     const double beta = v[0] / rz;
     if (on) a.p[i] = make_double3(z.x + beta * p.x, z.y + beta * p.y, z.z + beta * p.z);
@@ -259,10 +266,11 @@ static CgArgs cg_args(Engine &e, double3 *x, const CgTest &t) {
     return a;
 }
 
-// the smallest cluster with one ion per thread, up to eight blocks (the portable limit)
-static int cluster_of(int cnt) {
+// the smallest cluster with one ion per thread and at most CG_RHO of the nk carried rho(k), up to
+// eight blocks (the portable limit).  (Blocks past the ions add zeros: the same bits.)
+static int cluster_of(int cnt, int nk = 0) {
     int cs = 1;
-    while (cs < 8 && cnt > CGT * cs) cs *= 2;
+    while (cs < 8 && (cnt > CGT * cs || nk > CG_RHO * CGT * cs)) cs *= 2;
     return cs;
 }
 
@@ -282,7 +290,7 @@ void launch_cg_update(Engine &e, double3 *x, const double2 *rho_p, double2 *acc,
     a.acc = acc;
     a.comb = e.cg_comb;
     e.cg_comb.part = nullptr;
-    const int cs = cluster_of(a.cnt);
+    const int cs = cluster_of(a.cnt, acc ? e.nk : 0);
     MDFF_LAUNCH_C(e, cs, k_cg_update, cs, CGT, 0, a);
 }
 
