@@ -47,11 +47,6 @@ void download(Engine &e, void *dst, const void *src, size_t bytes) {
 
 // ions from which the mixed k space runs on the tensor cores by default
 constexpr int TC_MIN_IONS = 4096;
-// ions below which it runs in FP64 (kspace64.cu: matrix instructions at half the FP32 rate, but
-// two launches fewer per pass and no table of its own): polarisable MD, 10 steps, FP32 on CUDA
-// cores against FP64: 192 ions 2885 / 2126 us, 648 ions 2187 / 1725, 1536 ions 2740 / 2580, 3000
-// ions 3396 / 3429
-constexpr int REC64_IONS = 2048;
 
 struct mdffgpu_fit_plan {
     std::vector<mdffgpu_ctx *> ctx;
@@ -151,11 +146,11 @@ int mdffgpu_set_precision(mdffgpu_ctx *ctx, int precision) {
         }
         if (const char *v = getenv("MDFFGPU_PIM_SUBSET")) e.subset32 = atoi(v) != 0;
         // the rho and ion passes on the tensor cores (kspace_tc.cu, kspace_ion_tc.cu) from
-        // TC_MIN_IONS ions on, on CUDA cores below, in FP64 below REC64_IONS; MDFFGPU_RHO_TC /
+        // TC_MIN_IONS ions on, on CUDA cores below, in FP64 where few_for_rec32 says; MDFFGPU_RHO_TC /
         // MDFFGPU_ION_TC = 1 or 0 select the tensor-core or the CUDA-core FP32 pass at any size,
         // and MDFFGPU_MIXED_PARTS says itself what is in FP32
         e.rho_tc = e.ion_tc = e.n >= TC_MIN_IONS;
-        e.rec64 = e.n < REC64_IONS && !getenv("MDFFGPU_RHO_TC") && !getenv("MDFFGPU_ION_TC") &&
+        e.rec64 = mdffgpu::few_for_rec32(e) && !getenv("MDFFGPU_RHO_TC") && !getenv("MDFFGPU_ION_TC") &&
                   !getenv("MDFFGPU_MIXED_PARTS");
         if (const char *v = getenv("MDFFGPU_RHO_TC")) e.rho_tc = atoi(v) != 0;
         if (const char *v = getenv("MDFFGPU_ION_TC")) e.ion_tc = atoi(v) != 0;

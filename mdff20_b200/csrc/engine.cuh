@@ -203,6 +203,8 @@ void launch_rec(Engine &e, const double *q, const double3 *mu, bool lq, bool ld,
 // kspace64.cu: the FP64 passes
 void setup_kspace64(Engine &e, const std::vector<KRow> &rows);
 void launch_rec64(Engine &e, const double *q, const double3 *mu, bool lq, bool ld, const RecOut &o);
+// whether a mixed-precision context of this size runs its k space in FP64 by default
+bool few_for_rec32(const Engine &e);
 // fit.cu: the status bits of a force-matching evaluation as an Error (none: returns)
 void fit_status(unsigned status);
 constexpr int FIT_NRES = 1 + MDFFGPU_FIT_NPARAM + 1;   // loss, gradient, status bits per evaluation
@@ -239,6 +241,8 @@ void launch_dir32(Engine &e, const double *q, const double3 *mu, double alpha, b
 // pair.cu: whether a pair kernel of that many blocks sums its energy slots in its last block
 bool sum_in_last(const Engine &e, int blocks);
 void launch_pol_field32(Engine &e, const double3 *p, double3 *out_ef);
+// kspace32.cu: the |nz| values a row of its ion pass is padded to
+int kz_of(int K2);
 // kspace32.cu: per force evaluation, the phase tables of the current positions
 void launch_coords32(Engine &e);
 // kspace32.cu: FP32 phase tables and k-space passes (idx: optional ion subset of cnt ions)

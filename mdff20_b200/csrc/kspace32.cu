@@ -616,7 +616,7 @@ static TabLayout layout_of(const Engine &e) {
     return L;
 }
 
-static int kz_of(int K2) { return K2 <= 8 ? 8 : (K2 <= 14 ? 14 : (K2 <= 16 ? 16 : 32)); }
+int kz_of(int K2) { return K2 <= 8 ? 8 : (K2 <= 14 ? 14 : (K2 <= 16 ? 16 : 32)); }
 
 void setup_kspace32(Engine &e, const std::vector<KRow> &rows) {
     TabLayout L = layout_of(e);

@@ -622,6 +622,25 @@ static int ksteps64(const Engine &e) {
     return cols <= 8 ? 2 : std::max(4, ceil_div(cols, 4));
 }
 
+// Mixed precision of few ions: the matrix instructions run at half the FP32 rate, but with two
+// launches fewer per pass and no table of their own.  Up to REC64_IONS ions, unless padding or the
+// size of the passes takes that back: both precisions pad |nz| (here to whole groups of ZG, there
+// to kz_of), counted below in (ion, row, padded |nz|).  Measured, FP32 on CUDA cores against FP64.
+// Polarisable MD, 10 steps, kmax 14: 192 ions 2885 / 2126 us, 648 ions 2187 / 1725, 1536 ions 2740 /
+// 2580, 3000 ions 3396 / 3429.  Force evaluations, rigid and with dipoles: 1920 ions kmax 12 97 / 84
+// and 417 / 409 us, kmax 15 109 / 97 and 484 / 457.  One |nz| past a group: kmax 16 999 ions (0.87e7
+// more here) 99 / 101 and 462 / 447, 1296 ions (1.1e7) 101 / 122 and 478 / 530, 1920 ions 110 / 146 and
+// 489 / 629; kmax 32 300 ions (1.0e7) 203 / 138 and 770 / 623, 648 ions (2.2e7) 212 / 198 and 849 /
+// 932.  Large passes: 1296 ions kmax 24 (5.0e7 here) 197 / 171 and 812 / 704, 1920 ions kmax 20 (5.2e7)
+// 195 / 232 and 762 / 820, 1536 ions kmax 31 (9.8e7) 309 / 270 and 1099 / 1282.
+bool few_for_rec32(const Engine &e) {
+    constexpr int REC64_IONS = 2048;
+    constexpr double MORE = 1e7, MOST = 5e7;
+    const double rows = (double)e.n * e.nrow;
+    const double w64 = rows * ZG * ceil_div(e.kmax[2] + 1, ZG), w32 = rows * kz_of(e.kmax[2]);
+    return e.n < REC64_IONS && w64 - w32 <= MORE && w64 <= MOST;
+}
+
 void setup_kspace64(Engine &e, const std::vector<KRow> &rows) {
     const Tab64 t = layout64(e);
     const int nrg = ceil_div(rows.size(), 4);
