@@ -9,7 +9,7 @@
 // operations, each rounded once (no contraction), so every pair lands in the
 // reference's bin and the integer counts are identical.  A pair's distance is the same
 // both ways round (negation is exact through every step), so each unordered pair is
-// evaluated once and counted for both orders.
+// evaluated and counted once; mdffgpu_rdf_counts adds the two orders up.
 //
 // What bounds it: instructions per pair (n^2 / 2 of them; half the pairs lie inside half the
 // box width).  The exact distance, square root and division in FP64 are about 100 issue slots;
@@ -115,9 +115,7 @@ __global__ void __launch_bounds__(GR_THREADS) k_gr_pairs(const __grid_constant__
         for (int k = threadIdx.x; k < nh; k += GR_THREADS) {
             const unsigned c = h_sh[k];
             if (!c) continue;
-            const int b = k / np, q = k - b * np, ti = q / a.nt, tj = q - ti * a.nt;
             atomicAdd(&a.hist[k], (unsigned long long)c);
-            atomicAdd(&a.hist[b * np + tj * a.nt + ti], (unsigned long long)c);
             h_sh[k] = 0u;
         }
         __syncthreads();
@@ -176,12 +174,8 @@ __global__ void __launch_bounds__(GR_THREADS) k_gr_pairs(const __grid_constant__
                     }
                     const int k = b * np + me[m].w + o.w;
                     if (in) {
-                        if (PRIV) {
-                            atomicAdd(&h_sh[k], 1u);
-                        } else {
-                            atomicAdd(&a.hist[k], 1ull);
-                            atomicAdd(&a.hist[b * np + o.w * a.nt + me[m].w / a.nt], 1ull);
-                        }
+                        if (PRIV) atomicAdd(&h_sh[k], 1u);
+                        else atomicAdd(&a.hist[k], 1ull);
                     }
                 }
             }
@@ -427,6 +421,13 @@ int mdffgpu_rdf_counts(mdffgpu_rdf *r, long long *pairs, int *nconf) {
         size_t nh = (size_t)x.nbins * x.nt * x.nt;
         MDFF_CK(cudaMemcpyAsync(pairs, x.d_hist, sizeof(unsigned long long) * nh, cudaMemcpyDeviceToHost, x.stream));
         MDFF_CK(cudaStreamSynchronize(x.stream));
+        // both orders of every pair: (ti, tj) and (tj, ti) hold their sum, like pairs count twice
+        for (size_t b = 0; b < (size_t)x.nbins; b++) {
+            long long *h = pairs + b * x.nt * x.nt;
+            for (int ti = 0; ti < x.nt; ti++)
+                for (int tj = ti; tj < x.nt; tj++)
+                    h[ti * x.nt + tj] = h[tj * x.nt + ti] = h[ti * x.nt + tj] + h[tj * x.nt + ti];
+        }
         if (nconf) *nconf = x.nconf;
     });
 }
