@@ -80,19 +80,31 @@ struct GrArgs {
 };
 
 // the reference's bin of a pair, or -1 (outside)
-__device__ __noinline__ int gr_exact(const GrArgs &a, int i, int j) {
-    const double4 si = a.s[i], sj = a.s[j];
+__device__ __forceinline__ int gr_bin(const GrArgs &a, const double4 &si, const double4 &sj) {
     const double3 d = pbc_frac(a.c, dsub(si.x, sj.x), dsub(si.y, sj.y), dsub(si.z, sj.z));
     const double r2 = norm2_exact(d);
     if (!(r2 < a.cut2)) return -1;
     const int b = (int)__ddiv_rn(sqrt(r2), a.resg);
     return b < 0 || b >= a.nbins ? -1 : b;   // never past the end for nbins > cutgr / resg
 }
+__device__ __noinline__ int gr_exact(const GrArgs &a, int i, int j) { return gr_bin(a, a.s[i], a.s[j]); }
 
 __device__ __forceinline__ float rsqrt_approx(float x) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+// the block's counters added to the histogram and cleared
+__device__ __forceinline__ void gr_flush(const GrArgs &a, unsigned *h, int nh) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < nh; k += GR_THREADS) {
+        const unsigned c = h[k];
+        if (!c) continue;
+        atomicAdd(&a.hist[k], (unsigned long long)c);
+        h[k] = 0u;
+    }
+    __syncthreads();
 }
 
 template <int IPT, bool ORTHO, bool PRIV>
@@ -110,16 +122,6 @@ __global__ void __launch_bounds__(GR_THREADS) k_gr_pairs(const __grid_constant__
     // the certain counts of one block stay below 2^31 up to about 10^6 ions; past that they are
     // added to the global histogram on the way
     long long seen = 0;
-    auto flush = [&] {
-        __syncthreads();
-        for (int k = threadIdx.x; k < nh; k += GR_THREADS) {
-            const unsigned c = h_sh[k];
-            if (!c) continue;
-            atomicAdd(&a.hist[k], (unsigned long long)c);
-            h_sh[k] = 0u;
-        }
-        __syncthreads();
-    };
     for (long long t = blockIdx.x; t < (long long)nbi * nbj; t += gridDim.x) {
         const int bi = (int)(t / nbj), bj = (int)(t - (long long)bi * nbj);
         const int i0 = bi * GR_THREADS * IPT, j0 = bj * a.jt, jn = min(a.jt, a.n - j0);
@@ -184,11 +186,65 @@ __global__ void __launch_bounds__(GR_THREADS) k_gr_pairs(const __grid_constant__
         else scan(std::false_type());
         seen += (long long)GR_THREADS * IPT * jn;
         if (PRIV && seen > (1ll << 30)) {
-            flush();
+            gr_flush(a, h_sh, nh);
             seen = 0;
         }
     }
-    if (PRIV) flush();
+    if (PRIV) gr_flush(a, h_sh, nh);
+}
+
+// Every pair by the FP64 operations, for bins so fine that FP32 would leave most warps an open pair
+// (gr_fine): the same loop over tiles with one i per thread, the exact fractions in shared memory.
+template <bool PRIV>
+__global__ void __launch_bounds__(GR_THREADS) k_gr_fine(const __grid_constant__ GrArgs a) {
+    grid_dep();
+    extern __shared__ unsigned h_sh[];
+    __shared__ double4 tile[GR_JT];
+    __shared__ int ttile[GR_JT];
+    const int np = a.nt * a.nt, nh = a.nbins * np;
+    if (PRIV)
+        for (int k = threadIdx.x; k < nh; k += GR_THREADS) h_sh[k] = 0u;
+    const int nbi = (a.n + GR_THREADS - 1) / GR_THREADS, nbj = (a.n + a.jt - 1) / a.jt;
+    long long seen = 0;
+    for (long long t = blockIdx.x; t < (long long)nbi * nbj; t += gridDim.x) {
+        const int bi = (int)(t / nbj), bj = (int)(t - (long long)bi * nbj);
+        const int i0 = bi * GR_THREADS, j0 = bj * a.jt, jn = min(a.jt, a.n - j0);
+        if (j0 + jn - 1 <= i0) continue;   // no j > i here
+        __syncthreads();
+        for (int k = threadIdx.x; k < jn; k += GR_THREADS) {
+            tile[k] = a.s[j0 + k];
+            ttile[k] = a.fx[j0 + k].w;
+        }
+        __syncthreads();
+        const int i = i0 + threadIdx.x;
+        if (i < a.n) {
+            const double4 si = a.s[i];
+            const int ti = a.fx[i].w * a.nt;
+#pragma unroll 2
+            for (int jj = max(0, i + 1 - j0); jj < jn; jj++) {
+                const int b = gr_bin(a, si, tile[jj]);
+                if (b < 0) continue;
+                const int k = b * np + ti + ttile[jj];
+                if (PRIV) atomicAdd(&h_sh[k], 1u);
+                else atomicAdd(&a.hist[k], 1ull);
+            }
+        }
+        seen += (long long)GR_THREADS * jn;
+        if (PRIV && seen > (1ll << 30)) {
+            gr_flush(a, h_sh, nh);
+            seen = 0;
+        }
+    }
+    if (PRIV) gr_flush(a, h_sh, nh);
+}
+
+// Whether to take k_gr_fine: a pair is open in FP32 with a chance of about 2 (e0 + 3/4 e1 nbins) (most
+// pairs lie in the outer bins), and a warp is done by FP32 only where none of its 32 is.  Measured, in
+// us, FP32 decision / all in FP64, triclinic cell, bins to 0.45 of the box: 24000 ions, 1 type, chance
+// 0.040 1326 / 1374, 0.048 1413 / 1371, 0.129 1960 / 1382; 6000 ions, 2 types, 0.016 142 / 160, 0.040
+// 172 / 162, 0.129 218 / 158; orthorhombic, 24000 ions, 0.037 1621 / 1691, 0.073 1604 / 1413.
+static bool gr_fine(const GrErr &w, int nbins) {
+    return 2.0 * ((double)w.e0 + 0.75 * (double)w.e1 * nbins) > 0.045;
 }
 
 // lattice (src/cell.c:13-91) as far as kardir and pbc need it: A, B = (A_j x A_k) / omega
@@ -298,7 +354,8 @@ void launch_gr(mdffgpu_rdf &r, const mdffgpu::Cell &c, const double *soa, const 
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, r.device);
     // two i per thread once that leaves several tile pairs per block; j tiles short enough for
     // the same (a block's start and its flush cost about as much as 20000 pairs)
-    const int ipt = r.n >= 12288 ? 2 : 1, blocks = 4 * nsm;
+    const bool fine = gr_fine(a.w, r.nbins);
+    const int ipt = r.n >= 12288 && !fine ? 2 : 1, blocks = 4 * nsm;
     a.jt = GR_JT;
     while (a.jt > 32 && (long long)ceil_div(r.n, GR_THREADS * ipt) * ceil_div(r.n, a.jt) < 8ll * blocks) a.jt /= 2;
     const long long tiles = (long long)ceil_div(r.n, GR_THREADS * ipt) * ceil_div(r.n, a.jt);
@@ -309,7 +366,11 @@ void launch_gr(mdffgpu_rdf &r, const mdffgpu::Cell &c, const double *soa, const 
         if (ortho) go(k_gr_pairs<I, true, decltype(priv)::value>);
         else go(k_gr_pairs<I, false, decltype(priv)::value>);
     };
-    if (ipt == 2 && a.priv) by_cell(std::true_type(), std::true_type());
+    if (fine && a.priv) {   // (with its tile of fractions past the default limit)
+        MDFF_CK(cudaFuncSetAttribute(k_gr_fine<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        go(k_gr_fine<true>);
+    } else if (fine) go(k_gr_fine<false>);
+    else if (ipt == 2 && a.priv) by_cell(std::true_type(), std::true_type());
     else if (ipt == 2) by_cell(std::true_type(), std::false_type());
     else if (a.priv) by_cell(std::false_type(), std::true_type());
     else by_cell(std::false_type(), std::false_type());

@@ -1,6 +1,7 @@
 """Counts of both orders of a pair from a histogram that holds each pair once: one to four types, bins
-that just fit the block's shared counters (10240) and that do not, two configurations added up.
-Whole numbers: equality with the oracle."""
+that just fit the block's shared counters (10240) and that do not, two configurations added up.  Bins
+so fine that every pair is decided in FP64 (triclinic cells: 0.004 A), at ion counts around the tiles
+of 256.  Whole numbers: equality with the oracle."""
 import numpy as np
 import pytest
 
@@ -26,3 +27,18 @@ def test_both_orders(nionit, past):
     assert nconf == 2
     np.testing.assert_array_equal(got, oracle.gr_counts(frames, nionit, cut, resg, nbins))
     np.testing.assert_array_equal(got, again)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 255, 256, 257, 513, 1300])
+@pytest.mark.parametrize("nbins", [2000, 2500, 2600])   # either side of the chance of an open pair, of 10240 counters
+def test_fine_bins(n, nbins):
+    rng = np.random.default_rng(n)
+    cell = np.array([[21.0, 0.0, 0.0], [4.0, 26.0, 0.0], [-3.0, 6.0, 33.0]])
+    pos = (rng.random((n, 3)) * 5.0 - 2.0) @ cell
+    nionit = [n // 3, n - n // 3]
+    cut = 9.7
+    resg = cut / nbins * 1.0001
+    with RDF(nionit, cut, resg=resg, nbins=nbins) as acc:
+        acc.add(cell, pos)
+        got = acc.counts()[0]
+    np.testing.assert_array_equal(got, oracle.gr_counts([(cell, pos)], nionit, cut, resg, nbins))
