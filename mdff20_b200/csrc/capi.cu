@@ -331,33 +331,24 @@ int mdffgpu_multipole_es(mdffgpu_ctx *ctx, const double *q, const double *mu, in
     if (!q || !mu) return MDFFGPU_ERR_ARG;
     return guarded(ctx, [&](Engine &e) {
         if (!e.p.lcoulombic) throw Error(MDFFGPU_ERR_STATE, "lcoulombic is not set");
-        size_t n = e.n;
-        double *dq = nullptr, *defg = nullptr;
-        double3 *dmu = nullptr, *def = nullptr, *df = nullptr;
-        MDFF_CK(cudaMalloc(&dq, sizeof(double) * n));
-        MDFF_CK(cudaMalloc(&dmu, sizeof(double3) * n));
-        MDFF_CK(cudaMalloc(&def, sizeof(double3) * n));
-        MDFF_CK(cudaMalloc(&df, sizeof(double3) * n));
-        MDFF_CK(cudaMalloc(&defg, sizeof(double) * 9 * n));
-        try {
-            upload(e, dq, q, sizeof(double) * n);
-            upload(e, dmu, mu, sizeof(double3) * n);
-            MDFF_CK(cudaMemsetAsync(df, 0, sizeof(double3) * n, e.stream));
-            double a = alpha > 0.0 ? alpha : e.p.alphaES;
-            e.multipole_es_dev(dq, dmu, a, flags, def, efg ? defg : nullptr, df);
-            e.sync_scalars();
-            if (ef) download(e, ef, def, sizeof(double3) * n);
-            if (efg) download(e, efg, defg, sizeof(double) * 9 * n);
-            if (f) download(e, f, df, sizeof(double3) * n);
-            MDFF_CK(cudaStreamSynchronize(e.stream));
-            if (u) *u = e.h_out->u_coul;
-            if (pvir) *pvir = e.h_out->pvir_coul;
-            if (tau) memcpy(tau, e.h_out->tau_coul, sizeof(double) * 9);
-        } catch (...) {
-            cudaFree(dq); cudaFree(dmu); cudaFree(def); cudaFree(df); cudaFree(defg);
-            throw;
-        }
-        cudaFree(dq); cudaFree(dmu); cudaFree(def); cudaFree(df); cudaFree(defg);
+        const size_t n = e.n;
+        // the arrays of a call, kept by the context
+        if (!e.d_es) e.d_es = mdffgpu::dalloc<double>(19 * n);
+        double *dq = e.d_es, *defg = dq + 10 * n;
+        double3 *dmu = (double3 *)(dq + n), *def = dmu + n, *df = def + n;
+        upload(e, dq, q, sizeof(double) * n);
+        upload(e, dmu, mu, sizeof(double3) * n);
+        MDFF_CK(cudaMemsetAsync(df, 0, sizeof(double3) * n, e.stream));
+        double a = alpha > 0.0 ? alpha : e.p.alphaES;
+        e.multipole_es_dev(dq, dmu, a, flags, def, efg ? defg : nullptr, df);
+        e.sync_scalars();
+        if (ef) download(e, ef, def, sizeof(double3) * n);
+        if (efg) download(e, efg, defg, sizeof(double) * 9 * n);
+        if (f) download(e, f, df, sizeof(double3) * n);
+        MDFF_CK(cudaStreamSynchronize(e.stream));
+        if (u) *u = e.h_out->u_coul;
+        if (pvir) *pvir = e.h_out->pvir_coul;
+        if (tau) memcpy(tau, e.h_out->tau_coul, sizeof(double) * 9);
     });
 }
 

@@ -222,6 +222,7 @@ Engine::~Engine() {
     cudaFree(d_rec_count);
     cudaFree(d_snap);
     cudaFree(d_soa);
+    cudaFree(d_es);
     if (step_exec) cudaGraphExecDestroy(step_exec);
     if (body_stream) cudaStreamDestroy(body_stream);
     for (int k = 0; k < NSIDE; k++) {

@@ -316,6 +316,7 @@ struct Engine {
     double3 *d_rs = nullptr;     // leap-frog r(t-dt)
     double *d_hist = nullptr;    // ASPC history [n][6][3]
     double *d_efg = nullptr;     // [n][9]
+    double *d_es = nullptr;      // q, mu, field, force, EFG of multipole_es on caller data (first call on)
     double3 *d_tmp3 = nullptr;   // scratch field / force
     double *d_qzero = nullptr;
     double3 *d_muzero = nullptr;
