@@ -158,7 +158,9 @@ __global__ void k_fill_cells(int n, const int *__restrict__ cell_of, const int *
 // sort each cell's ion indices ascending (bitonic in shared memory) so that the list
 // order, hence every pair sum, is the same from run to run; pk receives, in that order, the
 // fractional coordinates wrapped to [-1/2, 1/2] in FP32 with the index in w (the candidates
-// of k_build's first test, read there without a gather)
+// of k_build's first test, read there without a gather).  An ion 2^20 boxes away or more gets NaN:
+// its differences to other ions round by more than k_build's shells allow for, so FP64 decides
+// all its pairs.
 __global__ void k_sort_cells(int ncell, int cell_cap, const int *__restrict__ start, const int *__restrict__ cnt,
                              int *__restrict__ ions, const double4 *__restrict__ s, float4 *__restrict__ pk,
                              const int *__restrict__ rebuild) {
@@ -171,8 +173,9 @@ __global__ void k_sort_cells(int ncell, int cell_cap, const int *__restrict__ st
     int b = start[c];
     auto pack = [&](int k, int j) {
         const double4 p = s[j];
-        pk[b + k] = make_float4((float)(p.x - rint(p.x)), (float)(p.y - rint(p.y)), (float)(p.z - rint(p.z)),
-                                __int_as_float(j));
+        const bool far = !(fmax(fabs(p.x), fmax(fabs(p.y), fabs(p.z))) < 1048576.0);
+        pk[b + k] = make_float4(far ? __int_as_float(0x7fffffff) : (float)(p.x - rint(p.x)),
+                                (float)(p.y - rint(p.y)), (float)(p.z - rint(p.z)), __int_as_float(j));
     };
     if (m <= 1 || m > cell_cap) {
         for (int k = threadIdx.x; k < m; k += blockDim.x) pack(k, ions[b + k]);
