@@ -216,7 +216,9 @@ __global__ void k_sort_cells(int ncell, int cell_cap, const int *__restrict__ st
 // per ion), so the pair sets stay exact; a candidate is loaded and placed once for the G ions.
 // Measured against testing every candidate in FP64 (B200, cuts 8 and 11 A): 24000 ions 367 ->
 // 275 us (G = 4), 6000 ions 120 -> 79 us (G = 2), 3000 ions 62 -> 60 us (G = 1: few warps, so
-// ions per warp would cost more occupancy than they save).
+// ions per warp would cost more occupancy than they save).  All ions in one cell (whole call): 4000
+// ions 234 -> 223 us (G = 2; 237 with G = 1), 6000 ions 505 -> 399, 2048 ions 137 -> 125 (G = 1; 128
+// with G = 2), 8000 ions 604 -> 571.
 // NEAR (at least three cells in each dimension, orthorhombic): candidates are placed relative
 // to the cell's centre, which fixes the periodic image of every pair within the cut.
 struct BuildCut {
@@ -254,6 +256,12 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) k_build(BuildArgs a) {
     for (int k = 0; k < 9; k++) A[k] = (float)a.c.A[k / 3][k % 3];
     const BuildCut q = a.cut;
     const float hi = fmaxf(q.hi_nb, q.hi_co);
+    // the shells as |r^2 - mid| <= half (4e-7 for the roundings of that form): three instructions
+    // fewer per candidate.  One ion per warp over its cells keeps the comparisons of r^2 itself
+    // (2048 ions 67 us, 75 with this form)
+    constexpr bool MID = !NEAR || G > 1;
+    const float mid_nb = 0.5f * (q.lo_nb + q.hi_nb), half_nb = 0.5f * (q.hi_nb - q.lo_nb) + 4e-7f * q.hi_nb;
+    const float mid_co = 0.5f * (q.lo_co + q.hi_co), half_co = 0.5f * (q.hi_co - q.lo_co) + 4e-7f * q.hi_co;
     const unsigned lt = (1u << lane) - 1u;
     int knb[G], kco[G];
 #pragma unroll
@@ -309,9 +317,17 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) k_build(BuildArgs a) {
                         z = u * A[2] + v * A[5] + w * A[8];
                     }
                     const float r2 = x * x + y * y + z * z;
-                    const bool cand = in && j != ig[g] && (edge || !(r2 > hi));
-                    bool in_nb = cand && !edge && r2 < q.lo_nb, in_co = cand && !edge && r2 < q.lo_co;
-                    const bool open = cand && (edge || (!in_nb && !(r2 > q.hi_nb)) || (!in_co && !(r2 > q.hi_co)));
+                    bool in_nb, in_co, open;
+                    if (MID) {
+                        const bool cand = in && j != ig[g];
+                        const float d = fminf(fabsf(r2 - mid_nb) - half_nb, fabsf(r2 - mid_co) - half_co);
+                        open = cand && (edge || !(d > 0.0f));
+                        in_nb = cand && r2 < mid_nb, in_co = cand && r2 < mid_co;
+                    } else {
+                        const bool cand = in && j != ig[g] && (edge || !(r2 > hi));
+                        in_nb = cand && !edge && r2 < q.lo_nb, in_co = cand && !edge && r2 < q.lo_co;
+                        open = cand && (edge || (!in_nb && !(r2 > q.hi_nb)) || (!in_co && !(r2 > q.hi_co)));
+                    }
                     if (__any_sync(0xffffffffu, open)) {
                         if (open) {
                             const double4 si = a.s[ig[g]], sj = a.s[j];
@@ -415,7 +431,8 @@ void run_build(cudaStream_t st, bool pdl, int n, const Cell &c, const int nc[3],
         cfg.gridDim = dim3(ceil_div(n, g * BUILD_WARPS));
         MDFF_CK(cudaLaunchKernelEx(&cfg, kernel, a));
     };
-    if (!near) go(k_build<1, false>, 1);
+    if (!near && n >= 3000) go(k_build<2, false>, 2);
+    else if (!near) go(k_build<1, false>, 1);
     else if (n >= 16384) go(k_build<4, true>, 4);
     else if (n >= 4096) go(k_build<2, true>, 2);
     else go(k_build<1, true>, 1);
