@@ -635,7 +635,7 @@ static int ksteps64(const Engine &e) {
 // 195 / 232 and 762 / 820, 1536 ions kmax 31 (9.8e7) 309 / 270 and 1099 / 1282.
 bool few_for_rec32(const Engine &e) {
     constexpr int REC64_IONS = 2048;
-    constexpr double MORE = 1e7, MOST = 5e7;
+    constexpr double MORE = 1.05e7, MOST = 5e7;
     const double rows = (double)e.n * e.nrow;
     const double w64 = rows * ZG * ceil_div(e.kmax[2] + 1, ZG), w32 = rows * kz_of(e.kmax[2]);
     return e.n < REC64_IONS && w64 - w32 <= MORE && w64 <= MOST;

@@ -48,10 +48,10 @@ def test_failing_tune_keeps_the_selection(solver):
     e.close()
 
 
-# |nz| padded to 16, 32, 48 and 8, 14, 16, 32 in FP64 and FP32: few ions run in FP64 unless that is 1e7
+# |nz| padded to 16, 32, 48 and 8, 14, 16, 32 in FP64 and FP32: few ions run in FP64 unless that is 1.05e7
 # (ion, row, |nz|) more, or 5e7 in all
 @pytest.mark.parametrize("n_si,kmax,fp64", [(32, 16, True), (333, 16, True), (432, 16, False), (640, 15, True),
-                                            (432, 24, True), (640, 20, False), (32, 32, True), (333, 32, False),
+                                            (432, 24, True), (640, 20, False), (32, 32, True), (100, 32, True), (333, 32, False),
                                             (682, 8, True), (683, 8, False)])
 def test_default_by_size(n_si, kmax, fp64, monkeypatch):
     s = synth.silica(n_si, seed=3, kmax=kmax, rc_sr=4.0, rc_lr=4.0, skin=0.5, alpha=0.6, dmin=synth.PIM_DMIN)
