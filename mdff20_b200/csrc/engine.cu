@@ -1508,10 +1508,8 @@ void Engine::snapshot(bool restore) {
     }
     add(d_nhc, 48);
     add(d_out, sizeof(DevScalars) / sizeof(double));
-    if (!d_snap) {
-        d_snap = dalloc<double>(total);
-        MDFF_CK(cudaMallocHost((void **)&h_rec, sizeof(DevScalars) * (STEP_BATCH + 1)));
-    }
+    if (!d_snap) d_snap = dalloc<double>(total);
+    if (!h_rec) MDFF_CK(cudaMallocHost((void **)&h_rec, sizeof(DevScalars) * (STEP_BATCH + 1)));
     s.restore = restore;
     s.snap = d_snap;
     s.rec_count = d_rec_count;
