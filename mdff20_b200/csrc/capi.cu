@@ -28,9 +28,11 @@ int guarded(mdffgpu_ctx *ctx, F &&f) {
         f(*ctx->e);
         return MDFFGPU_OK;
     } catch (const Error &x) {
+        ctx->e->join_failed();
         ctx->err = x.what();
         return x.code;
     } catch (const std::exception &x) {
+        ctx->e->join_failed();
         ctx->err = x.what();
         return MDFFGPU_ERR_CUDA;
     }

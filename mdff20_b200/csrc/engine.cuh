@@ -502,6 +502,16 @@ struct Engine {
         side_open[k] = false;
         MDFF_CK(cudaStreamWaitEvent(stream, ev_join[k], 0));
     }
+    // after a call that failed part way: what its side branches still write is waited for by all that
+    // comes next on `stream`
+    void join_failed() noexcept {
+        for (int k = 0; k < NSIDE; k++)
+            if (side_open[k]) {
+                side_open[k] = false;
+                cudaStreamWaitEvent(stream, ev_join[k], 0);
+            }
+        prep_issued = false;
+    }
     // after a recording that failed part way: its forks belong to the abandoned capture
     void forget_sides() {
         for (bool &o : side_open) o = false;
