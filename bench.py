@@ -22,7 +22,9 @@ ours      : state resident on the GPU; each timed step is bracketed by CUDA even
             uploaded, one step, positions, velocities and forces downloaded, every step,
             in one mdffgpu_md_steps_host call per step (one synchronisation).
 reference : the reference's own CPU code (oracle/_ref, -O3 -Ofast -fopenmp) on all host
-            cores, on a bounded sample of steps of the same system.
+            cores, on a bounded sample of steps of the same system; where it is not compiled
+            the arm prints an `unavailable` line (and `cpu_baseline` of the other arm times
+            the C restatement of oracle/, marked "port").
 N > 1 GPUs: one process per GPU (torchrun).  MD: an independent replica per rank (the
 path has no collective; weak scaling).  Fit: configurations sharded over the ranks,
 one all-reduce of (loss, gradient) per evaluation.  Times = max over ranks.
@@ -144,7 +146,7 @@ def cpu_baseline(system, nsteps: int = 20, warm: int = 5) -> dict:
         r = ref.run(system, "md", warm + nsteps, 0, 6, variant="tim", threads=threads, timeout=3600)
         wall = float(r["step_wall"][warm:warm + nsteps].sum())
         return {"value": system.nion * nsteps / wall, "unit": "ion-steps/s", "cores": threads,
-                "kind": "reference",
+                "kind": "reference", "steps": nsteps, "warmup": warm,
                 "sample": f"{nsteps} MD steps after {warm} untimed ones of the same {system.nion}-ion system, "
                           f"mdff20 C code -O3 -Ofast -fopenmp, OMP_NUM_THREADS={threads}, {wall:.2f} s timed"}
     from oracle.oracle import Oracle
@@ -164,7 +166,7 @@ def cpu_baseline(system, nsteps: int = 20, warm: int = 5) -> dict:
         done += 1
     nsteps, wall = done, time.perf_counter() - t0
     return {"value": system.nion * nsteps / wall, "unit": "ion-steps/s", "cores": os.cpu_count() or 1,
-            "kind": "port",
+            "kind": "port", "steps": nsteps, "warmup": warm,
             "sample": f"{nsteps} MD steps after {warm} untimed ones with the C restatement (OpenMP), {wall:.2f} s"}
 
 
@@ -289,6 +291,13 @@ def run_fit(args, world, rank, dev, pg) -> Optional[dict]:
 
 
 def run_reference(args):
+    from oracle import ref
+    if not ref.available("tim"):   # another program's time would not be the reference's
+        if int(os.environ.get("RANK", "0")) == 0:
+            print(json.dumps({"impl": "reference", "unavailable": "the compiled reference (oracle/_ref) is not here: "
+                                                                  "it is built by oracle/Makefile from the "
+                                                                  "reference's sources"}), flush=True)
+        return
     world, rank, local, pg = dist_setup(args)
     from mdff20_b200 import synth
     if rank == 0:
@@ -297,7 +306,7 @@ def run_reference(args):
         warm = max(0, min(args.warmup, args.cpu_warmup))
         cb = cpu_baseline(s, nsteps, warm)
         line = {"impl": "reference", "metric": METRIC, "value": cb["value"], "unit": "ion-steps/s",
-                "n_gpus": args.gpus, "steps": nsteps, "warmup": warm, "ms_per_step": 1000.0 * s.nion / cb["value"],
+                "n_gpus": args.gpus, "steps": cb["steps"], "warmup": cb["warmup"], "ms_per_step": 1000.0 * s.nion / cb["value"],
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64",
                 "data": "synthetic: seeded beta-cristobalite silica, MB velocities",
                 "config": {"workload": WORKLOAD, "nion": s.nion, "parallelism": "host OpenMP"},
