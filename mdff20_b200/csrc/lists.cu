@@ -563,12 +563,15 @@ void Engine::half_list(int which, int *point, int *list, int cap, int *count) {
     const int tot = point[n];
     if (count) *count = tot;
     if (list && tot > 0) {
-        if ((size_t)tot > csr_room) {   // kept between calls, grown with the list
+        if ((size_t)tot > csr_room) {
+            // kept between calls, for either list at the present capacities (a pair is in two rows of
+            // the full list): one allocation for the first calls of a context
+            const size_t room = std::max((size_t)n * std::max(cap_nb, cap_co) / 2, (size_t)tot);
             if (d_csr_list) MDFF_CK(cudaFree(d_csr_list));
             d_csr_list = nullptr;
             csr_room = 0;
-            d_csr_list = dalloc<int>((size_t)tot + tot / 8);
-            csr_room = (size_t)tot + tot / 8;
+            d_csr_list = dalloc<int>(room);
+            csr_room = room;
         }
         const size_t smem = sizeof(unsigned) * ((std::min(n, HALF_WIN) + 31) / 32);
         MDFF_LAUNCH(*this, k_half_fill, n, 128, smem, n, c, L, m, d_csr_point, d_csr_list);
