@@ -730,7 +730,8 @@ void Engine::force_match(const double3 *d_ft, double scale, double *h_res, int t
 // passes are split for half of the SMs: pieces cut small for one system alone cost more (partial
 // sums, starts of the row loops) than the others leave idle.  Evaluations in FP64, ms, split for
 // 148 / 74 / 37 SMs: 48 configurations 13.60 / 12.62 / 12.66, 12: 3.74 / 3.56 / 3.80, 4: 2.10 /
-// 2.20 / 2.54.  (The FP32 passes stay as they are: a tenth of the SMs took 48 configurations from
+// 2.20 / 2.54.  Sizes alike, 148 / 74 SMs: 12 of 96 ions 1.36 / 1.36, 24 of 480 3.07 / 3.04, 24 of 960 5.27 /
+// 5.27, 12 of 1536 (each of which fills the GPU at times) 4.98 / 4.72.  (The FP32 passes stay as they are: a tenth of the SMs took 48 configurations from
 // 9.7 to 10.1 ms where the inputs come from memory, although 8.1 to 7.5 where they are in L2.)
 cudaGraphExec_t Engine::capture_fit(const double3 *d_ft, const double *d_th, int tSi, int tO, double scale,
                                     double *d_res, int nconf) {
