@@ -165,7 +165,9 @@ Engine::Engine(const mdffgpu_params &prm, int dev) : p(prm) {
     for (int i = 0; i < p.nhc_n && i < 16; i++) nhc[32 + i] = timesca * timesca * temp;
     nhc[32] *= L;
     MDFF_CK(cudaMemcpy(d_nhc, nhc.data(), sizeof(double) * 48, cudaMemcpyHostToDevice));
-    MDFF_CK(cudaDeviceSynchronize());
+    // the copies above ran on the legacy stream (not the whole device: a stream another thread records
+    // on must not be waited for)
+    MDFF_CK(cudaStreamSynchronize(0));
 }
 
 Engine::~Engine() {

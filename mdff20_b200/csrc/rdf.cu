@@ -414,8 +414,9 @@ int mdffgpu_rdf_create(int nion, int ntype, const int *nionit, double cutgr, dou
         for (int t = 0, ia = 0; t < ntype; t++)
             for (int k = 0; k < nionit[t]; k++) typ[ia++] = t;
         MDFF_CK(cudaMemcpy(x.d_typ, typ.data(), sizeof(int) * nion, cudaMemcpyHostToDevice));
-        // (from pageable memory it may return before the device has it; the kernels run on their own stream)
-        MDFF_CK(cudaDeviceSynchronize());
+        // (from pageable memory it may return before the device has it; the kernels run on their own
+        // stream.  Not the whole device: a stream another thread records on must not be waited for)
+        MDFF_CK(cudaStreamSynchronize(0));
     });
     if (rc != MDFFGPU_OK) {
         mdffgpu_rdf_destroy(r);
