@@ -187,12 +187,8 @@ Engine::~Engine() {
     cudaFree(d_pair);
     cudaFree(d_damp);
     cudaFree(d_cell_pk);
-    cudaFree(d_tab64);
-    cudaFree(d_rowxy);
-    cudaFree(d_w64);
-    cudaFree(d_btick);
+    cudaFree(d_k64);
     cudaFree(d_row);
-    cudaFree(d_rho_part);
     cudaFree(d_rho);
     cudaFree(d_rho_acc);
     cudaFree(d_rho_it);
@@ -207,10 +203,7 @@ Engine::~Engine() {
     cudaFree(d_ion_order);
     cudaFree(d_ion_atab);
     cudaFree(d_ion_wtab);
-    cudaFree(d_ion_part);
     cudaFree(d_coef);
-    cudaFree(d_pcol);
-    cudaFree(d_pcon);
     dfree32();
     for (void *x : {(void *)d_fpart, (void *)d_fscal, (void *)d_w, (void *)d_lam, (void *)d_sv, (void *)d_fa,
                     (void *)d_fb, (void *)d_fc, (void *)d_qw, (void *)d_efg_rec, (void *)d_muw, (void *)d_rw,
@@ -551,12 +544,13 @@ void Engine::alloc_lists(int cnb, int cco) {
     d_co = dalloc<int>((size_t)n * cap_co);
     d_con = dalloc<int>(n);
     dfree(d_coef);
-    dfree(d_pcol);
-    dfree(d_pcon);
+    d_pcol = d_pcon = nullptr;
     if (p.lcoulombic && lpol) {
-        d_coef = dalloc<double2>((size_t)n * cap_co);
-        d_pcol = dalloc<int>((size_t)n * cap_co);
-        d_pcon = dalloc<int>(n);
+        // records of 20 bytes and the counts in one allocation (setup_kspace64 says why)
+        const size_t rec = (size_t)n * cap_co;
+        d_coef = dalloc<double2>(rec + (rec + n + 3) / 4);
+        d_pcol = (int *)(d_coef + rec);
+        d_pcon = d_pcol + rec;
     }
     list_ready = false;
     coef_ready = false;

@@ -330,7 +330,8 @@ struct Engine {
     int cap_nb = 0, cap_co = 0;
     int *d_nb = nullptr, *d_nbn = nullptr, *d_co = nullptr, *d_con = nullptr;
     double2 *d_coef = nullptr;   // [n][cap_co] cached dipole-field pair factors (k_dir_prep) ...
-    int *d_pcol = nullptr;       // ... of the polarisable pairs inside the cut-off, d_pcon[i] per ion
+    int *d_pcol = nullptr;       // ... of the polarisable pairs inside the cut-off, d_pcon[i] per ion (both
+                                 // in d_coef's allocation)
     int *d_pcon = nullptr;
     bool use32 = false;          // mixed precision: FP32 Ewald kernels
     // parts of the mixed path (all on by default; MDFFGPU_MIXED_PARTS=real|rec keeps
@@ -391,6 +392,7 @@ struct Engine {
     bool rho_acc_ready = false;                         // d_rho_acc holds rho(k) of (q, mu_tot)
     // FP64 k space (kspace64.cu): phase table rows [n][tab64_w], ion-pass weights, (nx, ny) of
     // the rows, slice partials [slice][n][9] and the arrival counter per block of ions
+    char *d_k64 = nullptr;                              // the arrays of this group and d_rho_part
     double2 *d_tab64 = nullptr, *d_rowxy = nullptr;
     double *d_w64 = nullptr, *d_ion_part = nullptr;
     unsigned *d_btick = nullptr;

@@ -645,17 +645,30 @@ void setup_kspace64(Engine &e, const std::vector<KRow> &rows) {
     const Tab64 t = layout64(e);
     const int nrg = ceil_div(rows.size(), 4);
     e.tab64_w = t.w;
-    e.d_tab64 = dalloc<double2>((size_t)e.n * t.w);
-    e.d_w64 = dalloc<double>((size_t)t.nzg * nrg * 3 * ksteps64(e) * 32);   // zero: padding rows and columns stay so
+    e.rho64_chunks_max = std::max(1, std::min(64, ceil_div(e.n, R64_TI)));
+    e.ion64_slices_max = std::max(1, std::min({t.nzg * nrg, 32, std::max(4, 65536 / e.n)}));
+    // one allocation (each of more than half a megabyte costs 0.35 ms here and 0.27 ms when it is
+    // freed), zeroed: padding rows and columns of the weights stay so
+    size_t bytes = 0;
+    auto take = [&](size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255) / 256 * 256;
+        return at;
+    };
+    const size_t tab = take(sizeof(double2) * e.n * t.w), w = take(sizeof(double) * t.nzg * nrg * 3 * ksteps64(e) * 32),
+                 rowxy = take(sizeof(double2) * nrg * 4), part = take(sizeof(double2) * e.rho64_chunks_max * e.nk),
+                 btick = take(sizeof(unsigned) * (ceil_div(e.n, 8) + 1)),
+                 ion_part = take(sizeof(double) * e.ion64_slices_max * e.n * 9);
+    e.d_k64 = dalloc<char>(bytes);
+    e.d_tab64 = (double2 *)(e.d_k64 + tab);
+    e.d_w64 = (double *)(e.d_k64 + w);
+    e.d_rowxy = (double2 *)(e.d_k64 + rowxy);
+    e.d_rho_part = (double2 *)(e.d_k64 + part);
+    e.d_btick = (unsigned *)(e.d_k64 + btick);
+    e.d_ion_part = (double *)(e.d_k64 + ion_part);
     std::vector<double2> xy((size_t)nrg * 4, make_double2(0.0, 0.0));
     for (size_t r = 0; r < rows.size(); r++) xy[r] = make_double2(rows[r].nx, rows[r].ny);
-    e.d_rowxy = dalloc<double2>(xy.size());
     MDFF_CK(cudaMemcpy(e.d_rowxy, xy.data(), sizeof(double2) * xy.size(), cudaMemcpyHostToDevice));
-    e.rho64_chunks_max = std::max(1, std::min(64, ceil_div(e.n, R64_TI)));
-    e.d_rho_part = dalloc<double2>((size_t)e.rho64_chunks_max * e.nk);
-    e.d_btick = dalloc<unsigned>(ceil_div(e.n, 8) + 1);
-    e.ion64_slices_max = std::max(1, std::min({t.nzg * nrg, 32, std::max(4, 65536 / e.n)}));
-    e.d_ion_part = dalloc<double>((size_t)e.ion64_slices_max * e.n * 9);
 }
 
 static void launch_phase64(Engine &e) {
