@@ -513,11 +513,11 @@ __global__ void __launch_bounds__(1024) k_half_scan(int n, int *__restrict__ poi
 }
 
 // one block per row: the kept j as bits of a window of HALF_WIN ions in shared memory, read
-// back in ascending order (no sort)
+// back in ascending order (no sort); the first `room` entries of the list
 constexpr int HALF_WIN = 65536;
 __global__ void __launch_bounds__(128) k_half_fill(int n, int cap, const int *__restrict__ list,
                                                    const int *__restrict__ cnt, const int *__restrict__ point,
-                                                   int *__restrict__ out) {
+                                                   int *__restrict__ out, size_t room) {
     grid_dep();
     extern __shared__ unsigned bits[];
     __shared__ int w[32];
@@ -541,7 +541,8 @@ __global__ void __launch_bounds__(128) k_half_fill(int n, int cap, const int *__
         const int incl = block_scan(c, w);
         int pos = at + incl - c;
         for (int k = b; k < e; k++)
-            for (unsigned u = bits[k]; u; u &= u - 1) out[pos++] = w0 + 32 * k + __ffs(u) - 1;
+            for (unsigned u = bits[k]; u; u &= u - 1, pos++)
+                if ((size_t)pos < room) out[pos] = w0 + 32 * k + __ffs(u) - 1;
         __syncthreads();
         if (threadIdx.x == blockDim.x - 1) w[0] = incl;
         __syncthreads();
@@ -558,23 +559,28 @@ void Engine::half_list(int which, int *point, int *list, int cap, int *count) {
     if (!d_csr_point) d_csr_point = dalloc<int>((size_t)n + 1);
     MDFF_LAUNCH(*this, k_half_count, ceil_div((long long)n * 32, 256), 256, 0, n, c, L, m, d_csr_point + 1);
     MDFF_LAUNCH(*this, k_half_scan, 1, 1024, 0, n, d_csr_point);
-    MDFF_CK(cudaMemcpyAsync(point, d_csr_point, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, stream));
-    MDFF_CK(cudaStreamSynchronize(stream));
-    const int tot = point[n];
-    if (count) *count = tot;
-    if (list && tot > 0) {
-        if ((size_t)tot > csr_room) {
+    const size_t smem = sizeof(unsigned) * ((std::min(n, HALF_WIN) + 31) / 32);
+    auto fill = [&](size_t room) {
+        if (room > csr_room) {
             // kept between calls, for either list at the present capacities (a pair is in two rows of
             // the full list): one allocation for the first calls of a context
-            const size_t room = std::max((size_t)n * std::max(cap_nb, cap_co) / 2, (size_t)tot);
             if (d_csr_list) MDFF_CK(cudaFree(d_csr_list));
             d_csr_list = nullptr;
             csr_room = 0;
             d_csr_list = dalloc<int>(room);
             csr_room = room;
         }
-        const size_t smem = sizeof(unsigned) * ((std::min(n, HALF_WIN) + 31) / 32);
-        MDFF_LAUNCH(*this, k_half_fill, n, 128, smem, n, c, L, m, d_csr_point, d_csr_list);
+        MDFF_LAUNCH(*this, k_half_fill, n, 128, smem, n, c, L, m, d_csr_point, d_csr_list, csr_room);
+    };
+    // filled while the row starts are on their way (launched after their wait: 32 ions 65 us for both
+    // calls of a list, so 62; 256 ions 78 and 76)
+    if (list) fill((size_t)n * std::max(cap_nb, cap_co) / 2);
+    MDFF_CK(cudaMemcpyAsync(point, d_csr_point, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, stream));
+    MDFF_CK(cudaStreamSynchronize(stream));
+    const int tot = point[n];
+    if (count) *count = tot;
+    if (list && tot > 0) {
+        if ((size_t)tot > csr_room) fill(tot);
         MDFF_CK(cudaMemcpyAsync(list, d_csr_list, sizeof(int) * std::min(tot, std::max(cap, 0)), cudaMemcpyDeviceToHost,
                                 stream));
         MDFF_CK(cudaStreamSynchronize(stream));
