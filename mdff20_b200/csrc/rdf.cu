@@ -240,11 +240,11 @@ __global__ void __launch_bounds__(GR_THREADS) k_gr_fine(const __grid_constant__ 
 
 // Whether to take k_gr_fine: a pair is open in FP32 with a chance of about 2 (e0 + 3/4 e1 nbins) (most
 // pairs lie in the outer bins), and a warp is done by FP32 only where none of its 32 is.  Measured, in
-// us, FP32 decision / all in FP64, triclinic cell, bins to 0.45 of the box: 24000 ions, 1 type, chance
-// 0.040 1326 / 1374, 0.048 1413 / 1371, 0.129 1960 / 1382; 6000 ions, 2 types, 0.016 142 / 160, 0.040
-// 172 / 162, 0.129 218 / 158; orthorhombic, 24000 ions, 0.037 1621 / 1691, 0.073 1604 / 1413.
+// us, FP32 decision / all in FP64, bins to 0.45 of the box: triclinic cell, 1 type, 9000 ions, chance
+// 0.020 211 / 216, 0.030 234 / 216; 20000 ions 0.030 859 / 880, 0.040 955 / 879; 40000 ions 0.030 3026 /
+// 3184, 0.040 3358 / 3187; orthorhombic, 2 types, 20000 ions, 0.030 826 / 818, 0.040 909 / 822.
 static bool gr_fine(const GrErr &w, int nbins) {
-    return 2.0 * ((double)w.e0 + 0.75 * (double)w.e1 * nbins) > 0.045;
+    return 2.0 * ((double)w.e0 + 0.75 * (double)w.e1 * nbins) > 0.033;
 }
 
 // lattice (src/cell.c:13-91) as far as kardir and pbc need it: A, B = (A_j x A_k) / omega
@@ -355,11 +355,15 @@ void launch_gr(mdffgpu_rdf &r, const mdffgpu::Cell &c, const double *soa, const 
     // two i per thread once that leaves several tile pairs per block; j tiles short enough for
     // the same (a block's start and its flush cost about as much as 20000 pairs)
     const bool fine = gr_fine(a.w, r.nbins);
-    const int ipt = r.n >= 12288 && !fine ? 2 : 1, blocks = 4 * nsm;
-    a.jt = GR_JT;
-    while (a.jt > 32 && (long long)ceil_div(r.n, GR_THREADS * ipt) * ceil_div(r.n, a.jt) < 8ll * blocks) a.jt /= 2;
+    const int ipt = r.n >= 12288 && !fine ? 2 : 1, few = 4 * nsm;
+    a.jt = fine ? GR_JT / 4 : GR_JT;
+    while (a.jt > 32 && (long long)ceil_div(r.n, GR_THREADS * ipt) * ceil_div(r.n, a.jt) < 8ll * few) a.jt /= 2;
     const long long tiles = (long long)ceil_div(r.n, GR_THREADS * ipt) * ceil_div(r.n, a.jt);
-    const int grid = (int)std::min<long long>(blocks, tiles);
+    // in FP64 a tile is long, so blocks are handed out as others end: 16 per SM where each has counters
+    // to add up, one per tile otherwise (us, tiles of 256 j at 4 blocks per SM / so, triclinic cell: 20000
+    // ions, 5000 bins 1093 / 882, 30000 bins of 2 types 1126 / 822; 9000 ions 254 / 218 and 259 / 217)
+    const long long most = !fine ? few : a.priv ? 4 * few : 1ll << 30;
+    const int grid = (int)std::min(most, tiles);
     auto go = [&](auto kernel) { kernel<<<grid, GR_THREADS, smem, st>>>(a); };
     auto by_cell = [&](auto two, auto priv) {
         constexpr int I = decltype(two)::value ? 2 : 1;

@@ -42,3 +42,18 @@ def test_fine_bins(n, nbins):
         acc.add(cell, pos)
         got = acc.counts()[0]
     np.testing.assert_array_equal(got, oracle.gr_counts([(cell, pos)], nionit, cut, resg, nbins))
+
+
+@pytest.mark.parametrize("n", [8897, 9025])   # tiles of 64, more of them than blocks per SM
+@pytest.mark.parametrize("nbins", [2500, 2600])   # either side of 10240 counters
+def test_fine_bins_many_tiles(n, nbins):
+    rng = np.random.default_rng(n)
+    cell = np.array([[51.0, 0.0, 0.0], [4.0, 56.0, 0.0], [-3.0, 6.0, 53.0]])
+    pos = (rng.random((n, 3)) * 5.0 - 2.0) @ cell
+    nionit = [n // 3, n - n // 3]
+    cut = 9.7
+    resg = cut / nbins * 1.0001
+    with RDF(nionit, cut, resg=resg, nbins=nbins) as acc:
+        acc.add(cell, pos)
+        got = acc.counts()[0]
+    np.testing.assert_array_equal(got, oracle.gr_counts([(cell, pos)], nionit, cut, resg, nbins))
