@@ -1213,9 +1213,7 @@ void Engine::get_dipoles() {
         if (!cont) {
             int nb = ceil_div(n, 256);
             MDFF_LAUNCH(*this, k_add3, nb, 256, 0, n, d_mu_static, d_mu_ind, d_mu_tot);
-            MDFF_LAUNCH(*this, k_self_sums, nb, 256, 0, n, d_q, d_mu_tot, d_part, part_stride);
-            reduce(S_Q2, 2, nb);
-            return;
+            return;   // (the self sums: engforce)
         }
     }
     // total dipoles, the self sums and, after a CG, u_pol and the history
@@ -1262,6 +1260,11 @@ void Engine::engforce(bool check_finite, bool opened) {
     if (p.lcoulombic) {
         rho_acc_ready = false;
         get_dipoles();
+        if (lpol && pim_solver == MDFFGPU_PIM_REFERENCE) {
+            const int nb = ceil_div(n, 256);
+            MDFF_LAUNCH(*this, k_self_sums, nb, 256, 0, n, d_q, d_mu_tot, d_part, part_stride);
+            reduce(S_Q2, 2, nb);
+        }
         bool ld = (ldip || lpol);
         // direct space: forces, energy, virial (do_forces, do_stress; src/field.c:381-383);
         // beside the k-space force pass (the ion pass or its combine joins it)
